@@ -196,13 +196,19 @@ __global__ void __launch_bounds__(kFrontierBS) k_write_all(const QueryDev* __res
 template <int M, int BS>
 constexpr int kExpandAllMinBlocks = BS == 256 ? (M == KPAX_MODEL_QUADROTOR ? 4 : 5) : (512 / BS > 0 ? 512 / BS : 1);
 
+// Steps per collision query: the kept states of four quadrotor or five 6-state CTAs of 256 threads
+// must fit in an SM beside the queries' offsets.
+template <int M, int BS>
+constexpr int kGroupAll = BS == 256 && M == KPAX_MODEL_QUADROTOR ? 3 : kGroup;
+
 template <int M, int BS>
 __global__ void __launch_bounds__(BS, (kExpandAllMinBlocks<M, BS>)) k_expand_all(const QueryDev* __restrict__ qs,
                                                                                 const Ctl* __restrict__ ctls,
                                                                                 const uint32_t* __restrict__ qidx,
                                                                                 uint32_t nq, uint32_t* __restrict__ active)
 {
-    extern __shared__ uint32_t s_off[];
+    extern __shared__ float s_save[];  // kept states, then the offsets
+    uint32_t* s_off = reinterpret_cast<uint32_t*>(s_save + kSaveBytes<M, BS, kGroupAll<M, BS>> / sizeof(float));
     __shared__ QueryDev sq;
     __shared__ ExpandSmem<BS / 32> sm;
     __shared__ uint32_t s_warp[BS / 32];
@@ -219,7 +225,7 @@ __global__ void __launch_bounds__(BS, (kExpandAllMinBlocks<M, BS>)) k_expand_all
             n = sq.ctl->n, k = sq.ctl->k;
             cur = i;
         }
-        if(!expand_tiles<M, BS>(sq, n, k, g - s_off[i], 0x80000000u, active, sm, true)) return;
+        if(!expand_tiles<M, BS, kGroupAll<M, BS>>(sq, n, k, g - s_off[i], 0x80000000u, active, sm, s_save, true)) return;
     }
 }
 
@@ -233,7 +239,8 @@ __global__ void __launch_bounds__(BS, (512 / BS > 0 ? 512 / BS : 1)) k_expand_mi
                                                                                   const uint32_t* __restrict__ qidx,
                                                                                   uint32_t nq, uint32_t* __restrict__ active)
 {
-    extern __shared__ uint32_t s_off[];
+    extern __shared__ float s_save[];  // kept states, then the offsets
+    uint32_t* s_off = reinterpret_cast<uint32_t*>(s_save + kSaveBytes<KPAX_MODEL_QUADROTOR, BS> / sizeof(float));
     __shared__ QueryDev sq;
     __shared__ ExpandSmem<BS / 32> sm;
     __shared__ uint32_t s_warp[BS / 32];
@@ -253,10 +260,11 @@ __global__ void __launch_bounds__(BS, (512 / BS > 0 ? 512 / BS : 1)) k_expand_mi
         }
         const uint32_t t = g - s_off[i];
         bool ok;
-        if(model == KPAX_MODEL_QUADROTOR) ok = expand_tiles<KPAX_MODEL_QUADROTOR, BS>(sq, n, k, t, 0x80000000u, active, sm, true);
+        if(model == KPAX_MODEL_QUADROTOR)
+            ok = expand_tiles<KPAX_MODEL_QUADROTOR, BS>(sq, n, k, t, 0x80000000u, active, sm, s_save, true);
         else if(model == KPAX_MODEL_DUBINS_AIRPLANE)
-            ok = expand_tiles<KPAX_MODEL_DUBINS_AIRPLANE, BS>(sq, n, k, t, 0x80000000u, active, sm, true);
-        else ok = expand_tiles<KPAX_MODEL_DOUBLE_INTEGRATOR, BS>(sq, n, k, t, 0x80000000u, active, sm, true);
+            ok = expand_tiles<KPAX_MODEL_DUBINS_AIRPLANE, BS>(sq, n, k, t, 0x80000000u, active, sm, s_save, true);
+        else ok = expand_tiles<KPAX_MODEL_DOUBLE_INTEGRATOR, BS>(sq, n, k, t, 0x80000000u, active, sm, s_save, true);
         if(!ok) return;
     }
 }

@@ -136,6 +136,11 @@ inline uint32_t warp_blocks(uint32_t n) { return (uint32_t)(((uint64_t)n * 32 + 
 
 // ---------------------------------------------------------------- batch kernels
 
+// Steps per collision query of the batch kernels (run_steps): 256-thread CTAs, four per SM, so the
+// kept states of a CTA must stay below the 48 KB of static shared memory.
+template <int M>
+constexpr int kBatchGroup = M == KPAX_MODEL_QUADROTOR ? 3 : 5;
+
 template <int M>
 __global__ void __launch_bounds__(256, 4) k_propagate_batch(KParams p, Grid g, const float* __restrict__ parents,
                                                          const float* __restrict__ draws, uint32_t stream_id, uint32_t n,
@@ -143,6 +148,7 @@ __global__ void __launch_bounds__(256, 4) k_propagate_batch(KParams p, Grid g, c
                                                          int32_t* __restrict__ steps_out)
 {
     constexpr int SD = ModelDims<M>::SD, CD = ModelDims<M>::CD, S = SD + CD + 1;
+    __shared__ float s_save[kBatchGroup<M> * SD * 256];
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if(i >= n) return;
     float s[SD], u[6], c[4], rc[4];
@@ -157,7 +163,7 @@ __global__ void __launch_bounds__(256, 4) k_propagate_batch(KParams p, Grid g, c
     }
     const int steps = draw_controls(p, u, c);
     int done = 0;
-    const bool ok = propagate<M>(p, g, s, c, steps, done);
+    const bool ok = propagate<M, kBatchGroup<M>>(p, g, s, c, steps, done, s_save + threadIdx.x, 256);
     row_controls<M>(c, rc);
     float* dst = rows + (size_t)i * S;
 #pragma unroll
@@ -244,6 +250,7 @@ __global__ void __launch_bounds__(256, 4) k_propagate_head(KParams p, Grid g, co
                                                         int32_t* __restrict__ steps_out, LiveList live)
 {
     constexpr int SD = ModelDims<M>::SD, CD = ModelDims<M>::CD;
+    __shared__ float s_save[kHeadSteps * SD * 256];
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     const int lane = threadIdx.x & 31;
     bool alive = false;
@@ -263,13 +270,8 @@ __global__ void __launch_bounds__(256, 4) k_propagate_head(KParams p, Grid g, co
         steps = draw_controls(p, u, c);
         const auto k = segment_consts<M>(p, c);
         const StepParams sp = step_params(p);
-        bool ok = true;
         int done = 0;
-        while(done < steps && done < kHeadSteps) {
-            ok = model_step<M>(sp, g, s, c, k);
-            ++done;
-            if(!ok) break;
-        }
+        const bool ok = run_steps<M, kHeadSteps>(sp, g, s, c, k, min(steps, kHeadSteps), done, s_save + threadIdx.x, 256);
         alive = ok && done < steps;
         if(!alive) write_segment<M>(p, i, s, c, steps, ok, done, rows, valid, steps_out);
     }
@@ -282,6 +284,7 @@ __global__ void __launch_bounds__(256, 4) k_propagate_tail(KParams p, Grid g, fl
                                                         LiveList live, int from, int until, LiveList next)
 {
     constexpr int SD = ModelDims<M>::SD, CD = ModelDims<M>::CD;
+    __shared__ float s_save[kBatchGroup<M> * SD * 256];
     const uint32_t count = *live.count;
     if(blockIdx.x * blockDim.x >= count) return;  // whole block past the list: the ballot below needs full warps
     const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
@@ -299,13 +302,8 @@ __global__ void __launch_bounds__(256, 4) k_propagate_tail(KParams p, Grid g, fl
         for(int k = 0; k < SD; ++k) s[k] = live.state[(size_t)j * SD + k];
         const auto kc = segment_consts<M>(p, c);
         const StepParams sp = step_params(p);
-        bool ok = true;
         int done = from;
-        while(done < steps && done < until) {
-            ok = model_step<M>(sp, g, s, c, kc);
-            ++done;
-            if(!ok) break;
-        }
+        const bool ok = run_steps<M, kBatchGroup<M>>(sp, g, s, c, kc, min(steps, until), done, s_save + threadIdx.x, 256);
         alive = next.count && ok && done < steps;
         if(!alive) write_segment<M>(p, i, s, c, steps, ok, done, rows, valid, steps_out);
     }

@@ -516,15 +516,24 @@ struct ExpandSmem {
     uint32_t wn[NW], wv[NW], ws[NW];
 };
 
+// Steps per collision query (run_steps) of the single-query expansions: 5 divides the presets' 10, 20
+// and 25 steps, and the kept states (120 KB of shared memory at 512 quadrotor children per SM) leave
+// the grid over 100 KB of L1.
+constexpr int kGroup = 5;
+template <int M, int BS, int K = kGroup>
+constexpr size_t kSaveBytes = sizeof(float) * K * ModelDims<M>::SD * BS;
+
 // Expansion of a query's children (KPAX.cu:358-439 with 445-502).  Children form look-back tiles
 // of BS consecutive children; this block processes tiles b = first, first + stride, ... (grid-stride
 // rounds), so every tile only waits on tiles of its own round or earlier.  Per child: draws, RK4 with
 // per-step checks and grid queries, R1/R2 ids, counters, frontier mark; accepted children are
 // appended in child order.  Returns false when a look-back wait gave up (the query is then finished
 // with an error).
-template <int M, int BS>
+// save: kSaveBytes<M, BS, K> bytes of shared memory.
+template <int M, int BS, int K = kGroup>
 __device__ __forceinline__ bool expand_tiles(QueryDev& sq, uint32_t n, uint32_t k, uint32_t first, uint32_t stride,
-                                             uint32_t* __restrict__ active, ExpandSmem<BS / 32>& sm, bool defer_finish = false)
+                                             uint32_t* __restrict__ active, ExpandSmem<BS / 32>& sm, float* save,
+                                             bool defer_finish = false)
 {
     constexpr int SD = ModelDims<M>::SD, CD = ModelDims<M>::CD, S = SD + CD + 1;
     constexpr int NW = BS / 32;
@@ -553,7 +562,7 @@ __device__ __forceinline__ bool expand_tiles(QueryDev& sq, uint32_t n, uint32_t 
                 if(sq.mix) mlp::mixture_draws(p, sq.mix + (size_t)(c / k) * mlp::kMixFloats, sq.prop_eps, plan, iter, c, u);
             }
             steps = draw_controls(p, u, cc);
-            valid = propagate<M>(p, sq.g, s, cc, steps, steps_done);
+            valid = propagate<M, K>(p, sq.g, s, cc, steps, steps_done, save + threadIdx.x, BS);
             r1v = region_r1<SD>(p, s);
             r2v = region_r2<SD>(p, s, r1v);
             atomicAdd(rg.counter + r1v, 1);
@@ -640,13 +649,14 @@ template <int M, int BS>
 __global__ void __launch_bounds__(BS, (512 / BS > 0 ? 512 / BS : 1)) k_expand(const QueryDev* __restrict__ qs, const uint32_t* __restrict__ qidx,
                                                uint32_t* __restrict__ active)
 {
+    extern __shared__ float s_save[];
     __shared__ QueryDev sq;
     __shared__ ExpandSmem<BS / 32> sm;
     load_query(qs, qidx, sq);
     wait_predecessor();
     release_successor();
     if(__syncthreads_or(sq.ctl->done != 0u)) return;  // one decision for the whole block: barriers follow
-    expand_tiles<M, BS>(sq, sq.ctl->n, sq.ctl->k, blockIdx.x, gridDim.x, active, sm);
+    expand_tiles<M, BS>(sq, sq.ctl->n, sq.ctl->k, blockIdx.x, gridDim.x, active, sm, s_save);
 }
 
 // Region scores (Graph.cu:233-358): one warp per partial sum j; the warp scores groups of 32
@@ -850,6 +860,7 @@ __global__ void __launch_bounds__(BS, (512 / BS > 0 ? 512 / BS : 1)) k_iterate(c
                                                                              uint32_t* __restrict__ active)
 {
     constexpr int NW = BS / 32;
+    extern __shared__ float s_save[];  // not used by kIterFront
     __shared__ QueryDev sq;
     __shared__ ExpandSmem<NW> sm;
     __shared__ uint32_t s_flag, s_last;
@@ -985,7 +996,7 @@ __global__ void __launch_bounds__(BS, (512 / BS > 0 ? 512 / BS : 1)) k_iterate(c
 
     // ---- expansion (k_expand); a CTA whose look-back wait gave up has finished the query with an
     // error and still takes part in the barrier
-    expand_tiles<M, BS>(sq, n, k, cb, G, active, sm);
+    expand_tiles<M, BS>(sq, n, k, cb, G, active, sm, s_save);
     if(!grid_barrier(sq.bar, G, &s_flag)) {
         if(tid == 0) atomicOr(&ctl->error, kErrTimeout), finish_query(ctl, active);
         return;

@@ -62,11 +62,36 @@ template <int M>
 void launch_expand(int bs, dim3 grid, cudaStream_t s, const QueryDev* dq, const uint32_t* qidx, uint32_t* active)
 {
     switch(bs) {
-        case 128: launch_chained(k_expand<M, 128>, grid, 128, 0, s, dq, qidx, active); break;
-        case 256: launch_chained(k_expand<M, 256>, grid, 256, 0, s, dq, qidx, active); break;
-        case 512: launch_chained(k_expand<M, 512>, grid, 512, 0, s, dq, qidx, active); break;
-        default: launch_chained(k_expand<M, kExpandBS>, grid, kExpandBS, 0, s, dq, qidx, active); break;
+        case 128: launch_chained(k_expand<M, 128>, grid, 128, kSaveBytes<M, 128>, s, dq, qidx, active); break;
+        case 256: launch_chained(k_expand<M, 256>, grid, 256, kSaveBytes<M, 256>, s, dq, qidx, active); break;
+        case 512: launch_chained(k_expand<M, 512>, grid, 512, kSaveBytes<M, 512>, s, dq, qidx, active); break;
+        default: launch_chained(k_expand<M, kExpandBS>, grid, kExpandBS, kSaveBytes<M, kExpandBS>, s, dq, qidx, active); break;
     }
+}
+
+template <int M>
+void* expand_kernel(int bs)
+{
+    switch(bs) {
+        case 128: return (void*)k_expand<M, 128>;
+        case 256: return (void*)k_expand<M, 256>;
+        case 512: return (void*)k_expand<M, 512>;
+        default: return (void*)k_expand<M, kExpandBS>;
+    }
+}
+
+// Shared memory of the kept states of a block of bs children (run_steps), by model 1..3.
+size_t save_bytes(int model, int bs, int group = kGroup)
+{
+    const size_t sd = model == KPAX_MODEL_QUADROTOR ? 12 : 6;
+    return sizeof(float) * (size_t)group * sd * (size_t)bs;
+}
+
+// Allows a kernel its dynamic shared memory (more than the 48 KB a launch may ask for by default).
+kpax_status allow_smem(const void* fn, size_t bytes)
+{
+    KPAX_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    return KPAX_OK;
 }
 
 // The fused iteration kernel (or one of its two parts around the proposal pass) at one of its
@@ -85,11 +110,12 @@ void* iterate_kernel(int bs)
 template <int M, int PART = kIterWhole>
 void launch_iterate(int bs, uint32_t gx, cudaStream_t s, const QueryDev* dq, const Ctl* ctl, uint32_t* active)
 {
+    const size_t smem = PART == kIterFront ? 0 : save_bytes(M, bs);
     switch(bs) {
-        case 128: launch_chained(k_iterate<M, 128, PART>, dim3(gx), 128, 0, s, dq, ctl, active); break;
-        case 256: launch_chained(k_iterate<M, 256, PART>, dim3(gx), 256, 0, s, dq, ctl, active); break;
-        case 512: launch_chained(k_iterate<M, 512, PART>, dim3(gx), 512, 0, s, dq, ctl, active); break;
-        default: launch_chained(k_iterate<M, kExpandBS, PART>, dim3(gx), kExpandBS, 0, s, dq, ctl, active); break;
+        case 128: launch_chained(k_iterate<M, 128, PART>, dim3(gx), 128, smem, s, dq, ctl, active); break;
+        case 256: launch_chained(k_iterate<M, 256, PART>, dim3(gx), 256, smem, s, dq, ctl, active); break;
+        case 512: launch_chained(k_iterate<M, 512, PART>, dim3(gx), 512, smem, s, dq, ctl, active); break;
+        default: launch_chained(k_iterate<M, kExpandBS, PART>, dim3(gx), kExpandBS, smem, s, dq, ctl, active); break;
     }
 }
 
@@ -310,6 +336,14 @@ struct PlanBatch {
         const uint32_t groups0 = ((uint32_t)prm[0].num_r1 + 31) / 32;
         gx_score = n == 1 ? std::min<uint32_t>(kScoreCTAs, std::max<uint32_t>(1, (groups0 + 7) / 8))
                           : std::max<uint32_t>(1, 1024 / n);
+        for(int m = 0; m < 3; ++m) {
+            if(groups[m].empty()) continue;
+            const void* fn = m == 0 ? expand_kernel<KPAX_MODEL_DOUBLE_INTEGRATOR>(expand_bs[m])
+                                    : m == 1 ? expand_kernel<KPAX_MODEL_DUBINS_AIRPLANE>(expand_bs[m])
+                                             : expand_kernel<KPAX_MODEL_QUADROTOR>(expand_bs[m]);
+            kpax_status st = allow_smem(fn, save_bytes(m + 1, expand_bs[m]));
+            if(st != KPAX_OK) return st;
+        }
         if(n == 1) {  // the fused iteration: as many CTAs as the expansion wants and can stay resident
             int dev = 0, sms = 148, per_sm = 0;
             KPAX_CUDA(cudaGetDevice(&dev));
@@ -317,7 +351,9 @@ struct PlanBatch {
             const int m = prm[0].model - 1, bs = expand_bs[m];
             void* fn = m == 0 ? iterate_kernel<KPAX_MODEL_DOUBLE_INTEGRATOR>(bs)
                               : m == 1 ? iterate_kernel<KPAX_MODEL_DUBINS_AIRPLANE>(bs) : iterate_kernel<KPAX_MODEL_QUADROTOR>(bs);
-            KPAX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, bs, 0));
+            kpax_status st = allow_smem(fn, save_bytes(m + 1, bs));
+            if(st != KPAX_OK) return st;
+            KPAX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, bs, save_bytes(m + 1, bs)));
             const uint32_t resident = (uint32_t)std::max(per_sm, 0) * (uint32_t)sms;
             // every resident CTA: the frontier and score phases use them all, the expansion as many as
             // it has tiles (a small budget's iteration leaves the rest idle in that phase)
@@ -326,8 +362,9 @@ struct PlanBatch {
                 int front = 0, back = 0;
                 KPAX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
                     &front, iterate_kernel<KPAX_MODEL_QUADROTOR, kIterFront>(bs), bs, 0));
+                if((st = allow_smem(iterate_kernel<KPAX_MODEL_QUADROTOR, kIterBack>(bs), save_bytes(m + 1, bs))) != KPAX_OK) return st;
                 KPAX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-                    &back, iterate_kernel<KPAX_MODEL_QUADROTOR, kIterBack>(bs), bs, 0));
+                    &back, iterate_kernel<KPAX_MODEL_QUADROTOR, kIterBack>(bs), bs, save_bytes(m + 1, bs)));
                 gx_split = std::min<uint32_t>((uint32_t)std::max(std::min(front, back), 0) * (uint32_t)sms,
                                               (uint32_t)kIterMaxCTAs);
             }
@@ -338,6 +375,8 @@ struct PlanBatch {
             KPAX_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
             auto resident = [&](const void* fn, int bs, size_t smem, uint32_t& gx) -> kpax_status {
                 int per_sm = 0;
+                kpax_status sst = allow_smem(fn, smem);
+                if(sst != KPAX_OK) return sst;
                 KPAX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, bs, smem));
                 gx = (uint32_t)std::max(per_sm, 0) * (uint32_t)sms;
                 return KPAX_OK;
@@ -348,7 +387,7 @@ struct PlanBatch {
             if(st == KPAX_OK) st = resident((const void*)k_scores_all, kScoreBS, sq, gx_scores_all);
             for(int m = 0; m < 3 && st == KPAX_OK; ++m) {
                 if(groups[m].empty()) continue;
-                const size_t sg = 4 * (groups[m].size() + 1);
+                const size_t sg = expand_all_smem(m, groups[m].size());
                 const void* fn = m == 0 ? expand_all_kernel<KPAX_MODEL_DOUBLE_INTEGRATOR>(expand_bs[m])
                                         : m == 1 ? expand_all_kernel<KPAX_MODEL_DUBINS_AIRPLANE>(expand_bs[m])
                                                  : expand_all_kernel<KPAX_MODEL_QUADROTOR>(expand_bs[m]);
@@ -373,7 +412,7 @@ struct PlanBatch {
                 KPAX_CUDA(cudaMemcpyAsync(d_mixed, order.data(), sizeof(uint32_t) * order.size(), cudaMemcpyHostToDevice,
                                           stream));
                 uint32_t gx = 0;
-                if((st = resident(expand_mixed_kernel(bs0), bs0, 4 * ((size_t)n + 1), gx)) != KPAX_OK) return st;
+                if((st = resident(expand_mixed_kernel(bs0), bs0, save_bytes(KPAX_MODEL_QUADROTOR, bs0) + 4 * ((size_t)n + 1), gx)) != KPAX_OK) return st;
                 if(gx) mixed_bs = bs0, gx_mixed = gx;
             }
         }
@@ -383,6 +422,14 @@ struct PlanBatch {
         KPAX_CUDA(cudaMemsetAsync(d_ctl, 0, sizeof(Ctl) * n, stream));
         KPAX_CUDA(cudaStreamSynchronize(stream));
         return KPAX_OK;
+    }
+
+    // Dynamic shared memory of the persistent expansion of model group m with g queries.
+    size_t expand_all_smem(int m, size_t g) const
+    {
+        const int bs = expand_bs[m];
+        const int group = m == 2 && bs == 256 ? kGroupAll<KPAX_MODEL_QUADROTOR, 256> : kGroup;
+        return save_bytes(m + 1, bs, group) + 4 * (g + 1);
     }
 
     void update_fused()
@@ -499,12 +546,12 @@ struct PlanBatch {
                 }
                 for(int u = 0; u + 1 < nused; ++u) cudaStreamWaitEvent(stream, ev_join[u], 0);
             } else if(expand_mode == 2 && mixed_bs) {
-                launch_expand_mixed(mixed_bs, gx_mixed, sq, stream, dq, d_ctl, d_mixed, nq, d_active);
+                launch_expand_mixed(mixed_bs, gx_mixed, save_bytes(KPAX_MODEL_QUADROTOR, mixed_bs) + sq, stream, dq, d_ctl, d_mixed, nq, d_active);
             } else {
                 for(int m = 0; m < 3; ++m) {
                     if(groups[m].empty()) continue;
                     const uint32_t g = (uint32_t)groups[m].size();
-                    const size_t sg = 4 * ((size_t)g + 1);
+                    const size_t sg = expand_all_smem(m, g);
                     if(m == 0)
                         launch_expand_all<KPAX_MODEL_DOUBLE_INTEGRATOR>(expand_bs[m], gx_expand_all[m], sg, stream, dq, d_ctl,
                                                                         d_groups[m], g, d_active);
