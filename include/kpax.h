@@ -91,7 +91,8 @@ typedef struct kpax_config {
     int32_t sparse_valid_threshold; /* region is sparse if valid count < this (10, KPAX.cu:476) */
     uint64_t seed;                  /* Philox4x32-10 key (the reference seeds cuRAND from the clock) */
     int32_t block_size;             /* threads per CTA of the expansion kernel: 0 (= 448), 128, 256, 448, 512 */
-    int32_t unroll_iters;           /* planner iterations per captured CUDA graph (0 = default) */
+    int32_t unroll_iters;           /* planner iterations between two looks at the done flag: of a captured
+                                       CUDA graph, or of one fused launch (0 = default) */
     int32_t samples_per_thread;     /* children per expansion thread, 0 (= 1) .. 8 (grid-stride rounds) */
     /* PruneKPAX goal-progress pruning (PruneKPAX.cu:466-498): an accepted child is kept with
      * probability clamp(exploration_bias + goal_bias * clamp(progress / progress_scale + 1/2, 0, 1),

@@ -225,7 +225,7 @@ __global__ void __launch_bounds__(BS, (kExpandAllMinBlocks<M, BS>)) k_expand_all
             n = sq.ctl->n, k = sq.ctl->k;
             cur = i;
         }
-        if(!expand_tiles<M, BS, kGroupAll<M, BS>>(sq, n, k, g - s_off[i], 0x80000000u, active, sm, s_save, true)) return;
+        if(!expand_query_tiles<M, BS, kGroupAll<M, BS>, true>(sq, n, k, g - s_off[i], 0x80000000u, active, sm, s_save, true)) return;
     }
 }
 
@@ -261,10 +261,10 @@ __global__ void __launch_bounds__(BS, (512 / BS > 0 ? 512 / BS : 1)) k_expand_mi
         const uint32_t t = g - s_off[i];
         bool ok;
         if(model == KPAX_MODEL_QUADROTOR)
-            ok = expand_tiles<KPAX_MODEL_QUADROTOR, BS>(sq, n, k, t, 0x80000000u, active, sm, s_save, true);
+            ok = expand_query_tiles<KPAX_MODEL_QUADROTOR, BS, kGroup, true>(sq, n, k, t, 0x80000000u, active, sm, s_save, true);
         else if(model == KPAX_MODEL_DUBINS_AIRPLANE)
-            ok = expand_tiles<KPAX_MODEL_DUBINS_AIRPLANE, BS>(sq, n, k, t, 0x80000000u, active, sm, s_save, true);
-        else ok = expand_tiles<KPAX_MODEL_DOUBLE_INTEGRATOR, BS>(sq, n, k, t, 0x80000000u, active, sm, s_save, true);
+            ok = expand_query_tiles<KPAX_MODEL_DUBINS_AIRPLANE, BS, kGroup, true>(sq, n, k, t, 0x80000000u, active, sm, s_save, true);
+        else ok = expand_query_tiles<KPAX_MODEL_DOUBLE_INTEGRATOR, BS, kGroup, true>(sq, n, k, t, 0x80000000u, active, sm, s_save, true);
         if(!ok) return;
     }
 }

@@ -73,8 +73,8 @@ struct alignas(16) Ctl {
     unsigned long long n_exp, n_valid, n_steps;
     unsigned long long t_begin_ns, t_done_ns;
     float path_cost, pad2;
-    // k_iterate: device-clock nanoseconds spent in its phases (frontier, expansion, scores), summed
-    // over launches
+    // k_iterate: device-clock nanoseconds CTA 0 spent in its phases (frontier: count and entry list;
+    // expansion, up to the gather that ends it; appends and scores), summed over iterations
     unsigned long long t_front_ns, t_expand_ns, t_score_ns, pad3;
 };
 
@@ -92,8 +92,8 @@ struct alignas(16) QueryDev {
     unsigned long long* lb;  // look-back status of k_expand, one per block
     float* partials;      // kPartials partial score sums
     uint32_t* sarr;       // arrival counter of k_scores
-    uint32_t* bar;        // grid barrier of k_iterate: arrivals (one word used)
-    uint32_t* ctas;       // per-CTA repeat sums of k_iterate's frontier phase
+    unsigned long long* words;  // gather words of k_iterate
+    unsigned long long* entry_words;  // its entry list: (iteration's tag, node) per entry
     float* path;
     const float* init_goal;  // init row then goal row, S floats each
     // learned proposal (quadrotor queries that enabled it; null otherwise)
@@ -101,7 +101,7 @@ struct alignas(16) QueryDev {
     float* mix;              // one mixture record per frontier entry
     const uint32_t* occ;     // occupancy bits of the R1 workspace cells
     float prop_eps;          // fraction of draws kept uniform
-    uint32_t path_rows, pad[2];
+    uint32_t path_rows, pad;
 };
 
 __device__ __forceinline__ unsigned long long globaltimer()
@@ -279,7 +279,6 @@ __global__ void k_begin(const QueryDev* __restrict__ qs, uint32_t plan_base, uin
     z.goal[0] = ig[p.S], z.goal[1] = ig[p.S + 1], z.goal[2] = ig[p.S + 2];
     z.t_begin_ns = globaltimer();
     *ctl = z;
-    sq.bar[0] = 0u;  // arrivals of k_iterate's grid barrier (a plan ended by a timeout may leave some)
     *sq.sarr = 0u, *sq.farr = 0u;
 }
 
@@ -509,11 +508,101 @@ __global__ void __launch_bounds__(kFrontierBS) k_frontier_write(const QueryDev* 
     for(uint32_t b = blockIdx.x; b < ntiles; b += gridDim.x) write_tile(sq, b, tree, R, E, s_warp);
 }
 
+// ---------------------------------------------------------------- gathers over a launch's CTAs
+// In the fused iteration every CTA is resident, and its phases exchange one 32-bit value per CTA: a
+// CTA publishes (flag, tag, value) as one 64-bit word and every CTA polls all words until they carry
+// the phase's tag.  The word is both the barrier arrival and the datum, so a phase costs one store
+// and one read that sees it.  A CTA's first warp stores its word to kReplicas copies of the array, a
+// lane each, and CTA c polls copy c % kReplicas: with one copy the polls of all CTAs hit the same ten
+// lines and a gather took over 4 us.  Tags are the query's epoch, which grows by one per iteration
+// and never returns; each of an iteration's gathers has its own array, and a CTA rewrites a word only
+// after a later gather of the same iteration, which every CTA enters after it has read the earlier one.
+constexpr int kIterMaxCTAs = 1024;  // CTAs of a k_iterate launch
+constexpr uint32_t kTagMask = 0x3FFFFFFFu;
+enum GatherId { kGatherFrontier = 0, kGatherChildren, kGatherScores, kGathers };
+constexpr uint32_t kReplicas = 32;
+// Words of one gather of G CTAs.
+__host__ __device__ constexpr size_t gather_words(uint32_t G) { return (size_t)kReplicas * G; }
+
+__device__ __forceinline__ void fence_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
+
+__device__ __forceinline__ unsigned long long ld_relaxed(const unsigned long long* p)
+{
+    unsigned long long v;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
+}
+
+__device__ __forceinline__ void st_relaxed(unsigned long long* p, unsigned long long v)
+{
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+
+// Called by the first warp.
+__device__ __forceinline__ void gather_publish(unsigned long long* words, uint32_t G, uint32_t cb, uint32_t tag, uint32_t value,
+                                               bool flag, bool release)
+{
+    if(release) fence_gpu();  // the CTA's writes (ordered before by its barrier) become visible first
+    st_relaxed(words + threadIdx.x * G + cb,
+               ((unsigned long long)flag << 63) | ((unsigned long long)(tag & kTagMask) << 32) | value);
+}
+
+// One CTA's word; false when it never carried the tag (bounded wait).
+__device__ __forceinline__ bool gather_poll(const unsigned long long* word, uint32_t tag, uint32_t& value, bool& flag,
+                                            uint32_t spin_limit = kSpinLimit)
+{
+    tag &= kTagMask;
+    for(uint32_t spins = 0;; ++spins) {
+        const unsigned long long w = ld_relaxed(word);
+        if(((uint32_t)(w >> 32) & kTagMask) == tag) {
+            value = (uint32_t)w, flag = (w >> 63) != 0ull;
+            return true;
+        }
+        if(spins > spin_limit) return false;
+        if(spins > 16) __nanosleep(32);
+    }
+}
+
+template <int NW>
+struct GatherSmem {
+    uint32_t tot[NW], pre[NW];
+};
+
+// Sum of the CTAs' values and of those below cb.  All threads call it after a __syncthreads() that
+// follows the writes to be released; with `release` the other CTAs' writes before their arrival are
+// visible afterwards.  Returns the same answer in every thread: false when a wait gave up.
+template <int NW>
+__device__ __forceinline__ bool gather_sum(unsigned long long* words, uint32_t tag, uint32_t G, uint32_t cb, uint32_t value,
+                                           bool release, GatherSmem<NW>& gs, uint32_t& below, uint32_t& total)
+{
+    const uint32_t tid = threadIdx.x;
+    if(tid < kReplicas) gather_publish(words, G, cb, tag, value, false, release);
+    words += (cb % kReplicas) * G;
+    uint32_t t = 0, b = 0;
+    bool ok = true;
+    for(uint32_t j = tid; j < G && ok; j += 32 * NW) {
+        uint32_t v = 0;
+        bool f = false;
+        ok = gather_poll(words + j, tag, v, f);
+        t += v;
+        b += j < cb ? v : 0u;
+    }
+    if(release && tid < G) fence_gpu();
+    t = __reduce_add_sync(0xffffffffu, t);
+    b = __reduce_add_sync(0xffffffffu, b);
+    if((tid & 31u) == 0u) gs.tot[tid >> 5] = t, gs.pre[tid >> 5] = b;
+    ok = __syncthreads_and(ok) != 0;
+    total = below = 0;
+    for(uint32_t w = 0; w < min((uint32_t)NW, (G + 31u) / 32u); ++w) total += gs.tot[w], below += gs.pre[w];
+    return ok;
+}
+
 // Shared-memory scratch of the expansion tiles of one block.
 template <int NW>
 struct ExpandSmem {
     uint32_t excl, ok;
     uint32_t wn[NW], wv[NW], ws[NW];
+    GatherSmem<NW> gs;
 };
 
 // Steps per collision query (run_steps) of the single-query expansions: 5 divides the presets' 10, 20
@@ -523,43 +612,69 @@ constexpr int kGroup = 5;
 template <int M, int BS, int K = kGroup>
 constexpr size_t kSaveBytes = sizeof(float) * K * ModelDims<M>::SD * BS;
 
-// Expansion of a query's children (KPAX.cu:358-439 with 445-502).  Children form look-back tiles
-// of BS consecutive children; this block processes tiles b = first, first + stride, ... (grid-stride
-// rounds), so every tile only waits on tiles of its own round or earlier.  Per child: draws, RK4 with
-// per-step checks and grid queries, R1/R2 ids, counters, frontier mark; accepted children are
-// appended in child order.  Returns false when a look-back wait gave up (the query is then finished
-// with an error).
-// save: kSaveBytes<M, BS, K> bytes of shared memory.
-template <int M, int BS, int K = kGroup>
-__device__ __forceinline__ bool expand_tiles(QueryDev& sq, uint32_t n, uint32_t k, uint32_t first, uint32_t stride,
-                                             uint32_t* __restrict__ active, ExpandSmem<BS / 32>& sm, float* save,
-                                             bool defer_finish = false)
+// The control-block values an expansion reads, and what a block's tiles add up to (thread 0).
+struct ExpandState {
+    uint32_t tree, iter, plan, epoch, ready;
+    float total;
+};
+struct ExpandTotals {
+    uint32_t accepted = 0;  // children appended by this block's tiles (every thread of the first warp)
+    bool goal = false;      // this thread appended a node in the goal ball
+    unsigned long long valid = 0, steps = 0;  // (thread 0)
+};
+
+// Expansion of a query's children (KPAX.cu:358-439 with 445-502).  Children form tiles of BS
+// consecutive children; this block processes tiles b = first, first + stride, ...  Per child: draws,
+// RK4 with grouped collision queries, R1/R2 ids, counters, frontier mark; accepted children are
+// appended in child order, at the tile's exclusive prefix of accepted children.
+// entry_words (the fused iteration): an entry's node is polled from the tagged word that its CTA writes
+// without a barrier in between; null: plain entries, complete before the kernel's launch or barrier.
+// gather == null: the prefix comes from a decoupled look-back over the tiles (grid-stride rounds, so
+// every tile only waits on tiles of its own round or earlier).
+// gather != null (the fused iteration with at most one tile per CTA): every CTA passes once, with or
+// without children, and tiles are only as wide as spreads the children over all CTAs; the prefix is a
+// gather over the CTAs, which is also the barrier behind which all counters are complete; n_total
+// receives the children appended by all CTAs.
+// kOne: the caller takes exactly one tile per call.  Returns false when a wait gave up.  save:
+// kSaveBytes<M, BS, K> bytes of shared memory.
+template <int M, int BS, int K = kGroup, bool kOne = false>
+__device__ __forceinline__ bool expand_tiles(QueryDev& sq, const ExpandState st, uint32_t n, uint32_t k, uint32_t first,
+                                             uint32_t stride, ExpandSmem<BS / 32>& sm, float* save, ExpandTotals& tot,
+                                             const unsigned long long* entry_words = nullptr,
+                                             unsigned long long* gather = nullptr, uint32_t* n_total = nullptr)
 {
     constexpr int SD = ModelDims<M>::SD, CD = ModelDims<M>::CD, S = SD + CD + 1;
     constexpr int NW = BS / 32;
     const KParams& p = sq.p;
     Ctl* ctl = sq.ctl;
-    const uint32_t tree = ctl->tree, iter = ctl->iter, plan = ctl->plan_idx, epoch = ctl->epoch;
-    const uint32_t ready = ctl->scores_ready;
-    const float total = ctl->score_total;
     const uint32_t ntile = n ? (n + BS - 1) / BS : 1u;
+    const uint32_t width = gather ? min((uint32_t)BS, ((n + gridDim.x - 1) / gridDim.x + 31u) & ~31u) : (uint32_t)BS;
     const TreeDev& t = sq.t;
     const RegDev& rg = sq.rg;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for(uint32_t b = first; b < ntile; b += stride) {
-        const uint32_t c = b * BS + threadIdx.x;
-        const bool active_child = c < n;
-        bool valid = false, next = false;
+    for(uint32_t b = first; gather ? b == first : b < ntile; b += stride) {
+        const uint32_t c = b * width + threadIdx.x;
+        const bool active_child = threadIdx.x < width && c < n;
+        bool valid = false, next = false, waited = true;
         float s[SD], cc[4], rc[4], u[6];
         uint32_t parent = 0;
         int r1v = 0, r2v = 0, steps = 0, steps_done = 0;
         if(active_child) {
-            parent = __ldcg(sq.entries + c / k);  // written by other CTAs of a fused launch: through L2
+            if(entry_words) {
+                bool f = false;
+                waited = gather_poll(entry_words + c / k, st.epoch, parent, f);
+            } else {
+                parent = sq.entries[c / k];
+            }
+        }
+        // the warps start their segments together: in step they share their instruction fetches
+        if(entry_words && !__syncthreads_and(waited)) return false;
+        if(active_child) {
             load_state<SD>(t, parent, s);
             const float d_parent = p.prune ? goal_distance(s, ctl->goal) : 0.0f;
-            child_draws(p, plan, iter, c, u);
+            child_draws(p, st.plan, st.iter, c, u);
             if constexpr(M == KPAX_MODEL_QUADROTOR) {
-                if(sq.mix) mlp::mixture_draws(p, sq.mix + (size_t)(c / k) * mlp::kMixFloats, sq.prop_eps, plan, iter, c, u);
+                if(sq.mix) mlp::mixture_draws(p, sq.mix + (size_t)(c / k) * mlp::kMixFloats, sq.prop_eps, st.plan, st.iter, c, u);
             }
             steps = draw_controls(p, u, cc);
             valid = propagate<M, K>(p, sq.g, s, cc, steps, steps_done, save + threadIdx.x, BS);
@@ -569,10 +684,11 @@ __device__ __forceinline__ bool expand_tiles(QueryDev& sq, uint32_t n, uint32_t 
             if(valid) {
                 atomicAdd(rg.valid + r1v, 1);
                 const uint32_t word = (uint32_t)r2v >> 5, bit = 1u << (r2v & 31);
-                const bool seen = (__ldg(rg.cur + word) & bit) != 0u;
-                next = (u[5] < region_score(__ldg(rg.score + r1v), total, ready, p.eps)) || !seen;
+                // snapshot and scores change between the iterations of one launch: through L2
+                const bool seen = (__ldcg(rg.cur + word) & bit) != 0u;
+                next = (u[5] < region_score(__ldcg(rg.score + r1v), st.total, st.ready, p.eps)) || !seen;
                 atomicOr(rg.nxt + word, bit);
-                if(next && p.prune) next = prune_keep(p, d_parent, goal_distance(s, ctl->goal), plan, iter, c);
+                if(next && p.prune) next = prune_keep(p, d_parent, goal_distance(s, ctl->goal), st.plan, st.iter, c);
             }
             row_controls<M>(cc, rc);
             if(sq.cap.rows) {
@@ -586,43 +702,48 @@ __device__ __forceinline__ bool expand_tiles(QueryDev& sq, uint32_t n, uint32_t 
         }
         const uint32_t mn = __ballot_sync(0xffffffffu, next), mv = __ballot_sync(0xffffffffu, valid);
         const uint32_t rank = __popc(mn & ((1u << lane) - 1u));
-        uint32_t wsteps = active_child ? (uint32_t)steps_done : 0u;  // RK4 steps executed (algorithmic work)
-#pragma unroll
-        for(int d = 16; d > 0; d >>= 1) wsteps += __shfl_xor_sync(0xffffffffu, wsteps, d);
+        // RK4 steps executed (algorithmic work)
+        const uint32_t wsteps = __reduce_add_sync(0xffffffffu, active_child ? (uint32_t)steps_done : 0u);
         if(lane == 0) sm.wn[warp] = __popc(mn), sm.wv[warp] = __popc(mv), sm.ws[warp] = wsteps;
         __syncthreads();
-        if(warp == 0) {
-            uint32_t acc = 0, nv = 0;
-            unsigned long long ns = 0;
-            for(int w = 0; w < NW; ++w) acc += sm.wn[w], nv += sm.wv[w], ns += sm.ws[w];
-            uint32_t excl = 0;
-            bool ok = true;
-            if(b == 0) {
-                if(lane == 0) lb_publish(sq.lb, epoch, 2u, acc);
-            } else {
-                if(lane == 0) lb_publish(sq.lb + b, epoch, 1u, acc);
-                ok = lb_exclusive(sq.lb, b, epoch, excl);
-                if(ok && lane == 0) lb_publish(sq.lb + b, epoch, 2u, excl + acc);
-            }
-            if(lane == 0) {
-                if(nv) atomicAdd(&ctl->n_valid, (unsigned long long)nv);
-                if(ns) atomicAdd(&ctl->n_steps, ns);
-                if(!ok) {
-                    atomicOr(&ctl->error, kErrTimeout);
-                    if(defer_finish) request_finish(ctl);
-                    else finish_query(ctl, active);
+        uint32_t excl = 0;
+        bool block_ok;
+        if(gather) {
+            uint32_t acc = 0;
+            for(int w = 0; w < NW; ++w) acc += sm.wn[w];
+            block_ok = gather_sum<NW>(gather, st.epoch, gridDim.x, first, acc, true, sm.gs, excl, *n_total);
+            tot.accepted += acc;
+            if(threadIdx.x == 0)
+                for(int w = 0; w < NW; ++w) tot.valid += sm.wv[w], tot.steps += sm.ws[w];
+        } else {
+            if(warp == 0) {
+                uint32_t acc = 0;
+                for(int w = 0; w < NW; ++w) {
+                    acc += sm.wn[w];
+                    if(lane == 0) tot.valid += sm.wv[w], tot.steps += sm.ws[w];
                 }
-                if(ok && b == ntile - 1) ctl->appended = excl + acc;
-                sm.excl = excl;
-                sm.ok = ok;
+                bool ok = true;
+                if(b == 0) {
+                    if(lane == 0) lb_publish(sq.lb, st.epoch, 2u, acc);
+                } else {
+                    if(lane == 0) lb_publish(sq.lb + b, st.epoch, 1u, acc);
+                    ok = lb_exclusive(sq.lb, b, st.epoch, excl);
+                    if(ok && lane == 0) lb_publish(sq.lb + b, st.epoch, 2u, excl + acc);
+                }
+                tot.accepted += acc;
+                if(lane == 0) {
+                    if(ok && b == ntile - 1) ctl->appended = excl + acc;
+                    sm.excl = excl;
+                    sm.ok = ok;
+                }
             }
+            __syncthreads();
+            excl = sm.excl, block_ok = sm.ok != 0u;
         }
-        __syncthreads();
-        const bool block_ok = sm.ok != 0u;
         if(next && block_ok) {
             uint32_t wex = 0;  // accepted children of the lower warps of this tile
             for(int w = 0; w < warp; ++w) wex += sm.wn[w];
-            const uint32_t slot = tree + sm.excl + wex + rank;
+            const uint32_t slot = st.tree + excl + wex + rank;
             if(slot >= p.cap) {
                 atomicOr(&ctl->error, kErrCapacity);
             } else {
@@ -634,13 +755,37 @@ __device__ __forceinline__ bool expand_tiles(QueryDev& sq, uint32_t n, uint32_t 
                 t.cost[slot] = d;
                 t.r1[slot] = r1v;
                 t.rep[slot] = kPending;
-                if(d < p.goal_thresh) atomicMin(&ctl->goal_idx, slot);
+                if(d < p.goal_thresh) atomicMin(&ctl->goal_idx, slot), tot.goal = true;
             }
         }
         if(!block_ok) return false;
         __syncthreads();  // the shared words are rewritten by the next round
+        if constexpr(kOne) break;
     }
     return true;
+}
+
+// The per-stage and batch expansions: state from the control block, counters added to it, a wait
+// that gave up finishes the query with an error.
+template <int M, int BS, int K = kGroup, bool kOne = false>
+__device__ __forceinline__ bool expand_query_tiles(QueryDev& sq, uint32_t n, uint32_t k, uint32_t first, uint32_t stride,
+                                                   uint32_t* __restrict__ active, ExpandSmem<BS / 32>& sm, float* save,
+                                                   bool defer_finish = false)
+{
+    Ctl* ctl = sq.ctl;
+    const ExpandState st{ctl->tree, ctl->iter, ctl->plan_idx, ctl->epoch, ctl->scores_ready, ctl->score_total};
+    ExpandTotals tot;
+    const bool ok = expand_tiles<M, BS, K, kOne>(sq, st, n, k, first, stride, sm, save, tot);
+    if(threadIdx.x == 0) {
+        if(tot.valid) atomicAdd(&ctl->n_valid, tot.valid);
+        if(tot.steps) atomicAdd(&ctl->n_steps, tot.steps);
+        if(!ok) {
+            atomicOr(&ctl->error, kErrTimeout);
+            if(defer_finish) request_finish(ctl);
+            else finish_query(ctl, active);
+        }
+    }
+    return ok;
 }
 
 // Expansion kernel of a batch: the children of query blockIdx.y (through qidx), tiles in grid-stride
@@ -656,7 +801,7 @@ __global__ void __launch_bounds__(BS, (512 / BS > 0 ? 512 / BS : 1)) k_expand(co
     wait_predecessor();
     release_successor();
     if(__syncthreads_or(sq.ctl->done != 0u)) return;  // one decision for the whole block: barriers follow
-    expand_tiles<M, BS>(sq, sq.ctl->n, sq.ctl->k, blockIdx.x, gridDim.x, active, sm, s_save);
+    expand_query_tiles<M, BS>(sq, sq.ctl->n, sq.ctl->k, blockIdx.x, gridDim.x, active, sm, s_save);
 }
 
 // Region scores (Graph.cu:233-358): one warp per partial sum j; the warp scores groups of 32
@@ -666,41 +811,61 @@ __global__ void __launch_bounds__(BS, (512 / BS > 0 ? 512 / BS : 1)) k_expand(co
 // partials.  Raw scores are stored (negative = no valid sample) and normalised where they are read
 // (region_score).  Threads gtid of gsize also copy the iteration's R2 bits into the snapshot;
 // warps wg of nwarps compute partials.
-__device__ __forceinline__ void score_partials(const QueryDev& sq, uint32_t gtid, uint32_t gsize, int wg, int nwarps)
+__device__ __forceinline__ float score_partial(const QueryDev& sq, int j)
 {
     const KParams& p = sq.p;
     const RegDev& rg = sq.rg;
     const int lane = threadIdx.x & 31;
-    for(uint32_t w = gtid; w < p.r2_words; w += gsize) rg.cur[w] = __ldcg(rg.nxt + w);
     const uint32_t ngroups = (p.num_r1 + 31) / 32;  // 32 consecutive regions per group
-    const int used = (int)min(ngroups, (uint32_t)kPartials);  // partials at and above `used` stay 0
-    for(int j = wg; j < used; j += nwarps) {
-        float part = 0.0f;
-        for(uint32_t grp = j; grp < ngroups; grp += kPartials) {
-            const int r = 32 * grp + lane;
-            float contrib = 0.0f;
-            if(r < p.num_r1) {
-                // counters and R2 bits were updated by atomics of other CTAs (of the same launch in
-                // k_iterate): read through L2
-                const int nv = __ldcg(rg.valid + r);
-                float stored = -1.0f;  // region without valid samples: score 1
-                if(nv > 0) {           // Graph.cu:241-256, coverage from an exact R2 popcount
-                    const int cnt = __ldcg(rg.counter + r);
-                    const uint32_t pc = popcount_range(rg.nxt, (uint64_t)r * p.P, (uint64_t)(r + 1) * p.P);
-                    const float cov = __fdiv_rn((float)pc, (float)p.P);
-                    const float fnv = __fadd_rn(p.eps, (float)nv);
-                    const float fv = __fmul_rn(__fdiv_rn(fnv, __fadd_rn(fnv, (float)(cnt - nv))), p.vol);
-                    const float fv2 = __fmul_rn(fv, fv), fv4 = __fmul_rn(fv2, fv2), cf = (float)cnt;
-                    stored = contrib = __fdiv_rn(fv4, __fmul_rn(__fadd_rn(1.0f, cov), __fadd_rn(1.0f, __fmul_rn(cf, cf))));
-                }
-                rg.score[r] = stored;
+    float part = 0.0f;
+    for(uint32_t grp = j; grp < ngroups; grp += kPartials) {
+        const int r = 32 * grp + lane;
+        float contrib = 0.0f;
+        if(r < p.num_r1) {
+            // counters and R2 bits were updated by atomics of other CTAs (of the same launch in
+            // k_iterate): read through L2
+            const int nv = __ldcg(rg.valid + r);
+            float stored = -1.0f;  // region without valid samples: score 1
+            if(nv > 0) {           // Graph.cu:241-256, coverage from an exact R2 popcount
+                const int cnt = __ldcg(rg.counter + r);
+                const uint32_t pc = popcount_range(rg.nxt, (uint64_t)r * p.P, (uint64_t)(r + 1) * p.P);
+                const float cov = __fdiv_rn((float)pc, (float)p.P);
+                const float fnv = __fadd_rn(p.eps, (float)nv);
+                const float fv = __fmul_rn(__fdiv_rn(fnv, __fadd_rn(fnv, (float)(cnt - nv))), p.vol);
+                const float fv2 = __fmul_rn(fv, fv), fv4 = __fmul_rn(fv2, fv2), cf = (float)cnt;
+                stored = contrib = __fdiv_rn(fv4, __fmul_rn(__fadd_rn(1.0f, cov), __fadd_rn(1.0f, __fmul_rn(cf, cf))));
             }
-#pragma unroll
-            for(int d = 16; d > 0; d >>= 1) contrib = __fadd_rn(contrib, __shfl_xor_sync(0xffffffffu, contrib, d));
-            part = __fadd_rn(part, contrib);
+            rg.score[r] = stored;
         }
-        if(lane == 0) sq.partials[j] = part;
+#pragma unroll
+        for(int d = 16; d > 0; d >>= 1) contrib = __fadd_rn(contrib, __shfl_xor_sync(0xffffffffu, contrib, d));
+        part = __fadd_rn(part, contrib);
     }
+    return part;
+}
+
+__device__ __forceinline__ void copy_snapshot(const QueryDev& sq, uint32_t gtid, uint32_t gsize)
+{
+    const RegDev& rg = sq.rg;
+    for(uint32_t w = gtid; w < sq.p.r2_words; w += gsize) rg.cur[w] = __ldcg(rg.nxt + w);
+}
+
+__device__ __forceinline__ void score_partials(const QueryDev& sq, uint32_t gtid, uint32_t gsize, int wg, int nwarps)
+{
+    copy_snapshot(sq, gtid, gsize);
+    const int used = (int)min((sq.p.num_r1 + 31u) / 32u, (uint32_t)kPartials);  // partials at and above `used` stay 0
+    for(int j = wg; j < used; j += nwarps) {
+        const float part = score_partial(sq, j);
+        if((threadIdx.x & 31) == 0) sq.partials[j] = part;
+    }
+}
+
+// KPAX.cu:527-528
+__device__ __forceinline__ float accept_rate(const KParams& p, uint32_t iter, uint32_t tree)
+{
+    const float a = __fsub_rn(1.0f, __fdiv_rn((float)tree, (float)p.cap));
+    const float a2 = __fmul_rn(a, a), a4 = __fmul_rn(a2, a2), a5 = __fmul_rn(a4, a);
+    return __fmul_rn(__fmul_rn((float)iter, p.eps), a5);
 }
 
 // Total of the partials by the block's first warp, then the iteration's bookkeeping by thread 0:
@@ -747,9 +912,7 @@ __device__ __forceinline__ void score_finish(const QueryDev& sq, uint32_t* __res
         const uint32_t iter = vc->iter, tree_old = vc->tree, tree_new = tree_old + vc->appended;
         ctl->tree_old = tree_old;
         ctl->tree = tree_new;
-        const float a = __fsub_rn(1.0f, __fdiv_rn((float)tree_new, (float)p.cap));  // KPAX.cu:527-528
-        const float a2 = __fmul_rn(a, a), a4 = __fmul_rn(a2, a2), a5 = __fmul_rn(a4, a);
-        ctl->faccept = __fmul_rn(__fmul_rn((float)iter, p.eps), a5);
+        ctl->faccept = accept_rate(p, iter, tree_new);
         ctl->n_exp = vc->n_exp + vc->n;
         ctl->iters_done = iter;
         ctl->iter = iter + 1u;
@@ -785,87 +948,55 @@ __global__ void __launch_bounds__(kScoreBS) k_scores(const QueryDev* __restrict_
     score_finish(sq, active);
 }
 
-// ---------------------------------------------------------------- fused iteration (single query)
-// k_iterate runs one whole iteration in one launch: frontier count, entry list, expansion and
-// region scores, separated by grid-wide barriers.  Every CTA must be resident (the host sizes the
-// grid by the occupancy of the kernel), every barrier is bounded, and each phase computes exactly
-// what the corresponding per-stage kernel computes (same per-node, per-child and per-region
-// arithmetic, same partial sums), so plans are bit-identical to the per-stage path.
+// ---------------------------------------------------------------- fused iterations (single query)
+// k_iterate runs up to max_inner whole iterations in one launch: frontier count, entry list,
+// expansion and region scores, separated by gathers over the CTAs.  Every CTA must be resident (the
+// host sizes the grid by the occupancy of the kernel), every wait is bounded, and each phase computes
+// exactly what the corresponding per-stage kernel computes (same per-node, per-child and per-region
+// arithmetic, same partial sums), so plans are bit-identical to the per-stage path.  The control
+// block is read once at the launch's start and written back by CTA 0 at its end; in between every
+// CTA keeps the same copy, since every value in it follows from the gathers.
+//
+// What bounds it besides the expansion is round trips through L2, so there are few: three gathers per
+// iteration (frontier sums; accepted children, which also gives each tile its slots; score values)
+// of 1.9-2.3 us each, and entries handed over word by word.  B200, whole plans, against one launch
+// per iteration with counter barriers and a look-back: Dubins 11.9 -> 10.0 ms (300 iterations, 39.5 ->
+// 33 us each), double integrator 10.1 -> 8.0 ms, quadrotor near plans of 2^14 children 1.35 -> 0.83 ms
+// (with the expansion's tiles spread over all CTAs: 57 -> 41 us), quadrotor 24.7 -> 23.6 ms.
 
-constexpr int kIterMaxCTAs = 1024;  // CTAs of a k_iterate launch
-constexpr int kIterBatch = 8;       // nodes per thread whose loads are issued together
-
-__device__ __forceinline__ uint32_t ld_acquire(const uint32_t* p)
-{
-    uint32_t v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-
-// Grid-wide barrier of a launch whose CTAs are all resident.  bar[0] counts arrivals over the
-// launch's barriers without being reset in between: the CTA whose arrival returns `old` waits
-// until the count reaches the next multiple of nblocks above it, so the last CTA to arrive passes
-// at once and the others need one poll that sees its arrival (the last CTA of the launch resets
-// the count once every CTA is past the last barrier).  Bounded: returns false after spin_limit
-// polls.
-__device__ __forceinline__ bool grid_barrier(uint32_t* bar, uint32_t nblocks, uint32_t* s_flag,
-                                             uint32_t spin_limit = kSpinLimit)
-{
-    __syncthreads();
-    if(threadIdx.x == 0) {
-        __threadfence();  // the block's writes before its arrival
-        const uint32_t target = (atomicAdd(bar, 1u) / nblocks + 1u) * nblocks;
-        bool ok = true;
-        uint32_t spins = 0;
-        while(ld_acquire(bar) < target) {
-            if(++spins > spin_limit) {
-                ok = false;
-                break;
-            }
-            if(spins > 16) __nanosleep(32);
-        }
-        __threadfence();
-        *s_flag = ok ? 1u : 0u;
-    }
-    __syncthreads();
-    return *s_flag != 0u;
-}
-
-// Sum of v over the block (all threads call it; s_warp holds one word per warp).
-template <int NW>
-__device__ __forceinline__ uint32_t block_sum(uint32_t v, uint32_t* s_warp)
-{
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for(int d = 16; d > 0; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
-    __syncthreads();
-    if(lane == 0) s_warp[warp] = v;
-    __syncthreads();
-    uint32_t t = 0;
-    for(int w = 0; w < NW; ++w) t += s_warp[w];
-    return t;
-}
+constexpr int kIterBatch = 8;      // nodes per thread whose loads are issued together
+constexpr uint32_t kScoreCTAs = 128;  // CTAs that add score partials (a power of two)
 
 // ctl_line: the query's control block, whose line thread 0 prefetches into L2 while the block
 // copies its descriptor (L2 is where the predecessor's writes land, so the prefetch cannot serve a
 // stale copy; the fields are read after the predecessor completes).
 // The whole iteration in one launch (kIterWhole), or split around the learned proposal pass:
-// kIterFront (frontier count, budget, entry list) and kIterBack (expansion, scores), with
-// k_propose launched between them.
+// kIterFront (frontier count, budget, entry list) and kIterBack (expansion, scores), one iteration
+// each, with k_propose launched between them.
 constexpr int kIterWhole = 0, kIterFront = 1, kIterBack = 2;
+
+// A launch's copy of the control block's iteration values.
+struct IterState {
+    uint32_t tree, tree_old, iter, plan, epoch, ready, goal, appended;
+    uint32_t R, k, E, n, full, stop;
+    float faccept, total;
+    unsigned long long n_exp;
+};
 
 template <int M, int BS, int PART = kIterWhole>
 __global__ void __launch_bounds__(BS, (512 / BS > 0 ? 512 / BS : 1)) k_iterate(const QueryDev* __restrict__ qs,
                                                                              const Ctl* ctl_line,
-                                                                             uint32_t* __restrict__ active)
+                                                                             uint32_t* __restrict__ active,
+                                                                             uint32_t max_inner)
 {
     constexpr int NW = BS / 32;
     extern __shared__ float s_save[];  // not used by kIterFront
     __shared__ QueryDev sq;
     __shared__ ExpandSmem<NW> sm;
-    __shared__ uint32_t s_flag, s_last;
-    __shared__ uint32_t s_warp[NW], s_warp2[NW];
-    __shared__ unsigned long long s_t[3];  // phase start times (thread 0)
+    __shared__ uint32_t s_warp[NW];
+    __shared__ IterState it;
+    __shared__ float s_part[kPartials], s_val[kScoreCTAs];
+    __shared__ unsigned long long s_t[3], s_ns[3];  // phase start times and sums (thread 0)
     if(threadIdx.x == 0) asm volatile("prefetch.global.L2 [%0];" ::"l"(ctl_line));
     load_query(qs, nullptr, sq);
     const KParams& p = sq.p;
@@ -875,150 +1006,231 @@ __global__ void __launch_bounds__(BS, (512 / BS > 0 ? 512 / BS : 1)) k_iterate(c
     const uint32_t G = gridDim.x, cb = blockIdx.x;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     wait_predecessor();
-    if(__syncthreads_or(ctl->done != 0u)) return;  // one decision for the whole grid: barriers follow
-    if(tid == 0) s_t[0] = globaltimer();
-    uint32_t k = 0, n = 0;  // children per entry and children of this iteration
-    if constexpr(PART != kIterBack) {
-        const uint32_t tree = ctl->tree, tree_old = ctl->tree_old, iter = ctl->iter, plan = ctl->plan_idx;
-        const uint32_t ready = ctl->scores_ready;
-        const float fa = ctl->faccept, total = ctl->score_total;
-
-        // ---- frontier count (k_frontier_count): re-activation of the previous iteration
-        // (KPAX.cu:505-517) and repeats of its new nodes (476-479) over this thread's contiguous nodes
-        const uint32_t per_cta = (tree + G - 1) / G, per_thr = (per_cta + BS - 1) / BS;
-        const uint32_t c_lo = min(tree, cb * per_cta), c_hi = min(tree, c_lo + per_cta);
-        const uint32_t lo = min(c_hi, c_lo + (uint32_t)tid * per_thr), hi = min(c_hi, lo + per_thr);
-        uint32_t sum = 0;
-        for(uint32_t i0 = lo; i0 < hi; i0 += kIterBatch) {
-            uint32_t r0[kIterBatch];
-            int32_t reg[kIterBatch], nv[kIterBatch];
-            float raw[kIterBatch];
-    #pragma unroll
-            for(int j = 0; j < kIterBatch; ++j) {  // each node's byte and region id, then its region's
-                const uint32_t i = i0 + j;         // score and valid count: two rounds of loads per batch
-                r0[j] = i < hi ? (uint32_t)t.rep[i] : 0u;
-                reg[j] = i < hi ? t.r1[i] : 0;
-            }
-    #pragma unroll
-            for(int j = 0; j < kIterBatch; ++j) raw[j] = rg.score[reg[j]], nv[j] = rg.valid[reg[j]];
-    #pragma unroll
-            for(int j = 0; j < kIterBatch; ++j) {
-                const uint32_t i = i0 + j;
-                if(i >= hi) continue;
-                uint32_t r = r0[j];
-                if(r == 0u) {
-                    if(i < tree_old) {
-                        const float sc = region_score(raw[j], total, ready, p.eps);
-                        if(reactivate_draw(p, plan, iter - 1u, i) <= __fadd_rn(sc, fa)) r = 1u;
-                    }
-                } else if(r == kPending) {
-                    r = nv[j] < p.sparse_thr ? p.sparse_repeat : 1u;
-                }
-                if(r != r0[j]) t.rep[i] = (uint8_t)r;
-                sum += r;
-            }
-        }
-        // this thread's exclusive prefix inside the CTA, and the CTA's sum
-        uint32_t x = sum;
-    #pragma unroll
-        for(int d = 1; d < 32; d <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, x, d);
-            if(lane >= d) x += y;
-        }
-        if(lane == 31) s_warp[warp] = x;
-        __syncthreads();
-        uint32_t wex = 0, cta_sum = 0;
-        for(int w = 0; w < NW; ++w) {
-            wex += w < warp ? s_warp[w] : 0u;
-            cta_sum += s_warp[w];
-        }
-        const uint32_t thr_excl = wex + x - sum;
-        if(tid == 0) sq.ctas[cb] = cta_sum;
-        if(!grid_barrier(sq.bar, G, &s_flag)) {
-            if(tid == 0) atomicOr(&ctl->error, kErrTimeout), finish_query(ctl, active);
-            return;
-        }
-        release_successor();  // every CTA is resident now
-
-        // ---- budget (KPAX.cu:323-350) from the CTA sums, then the entry list (k_frontier_write)
-        uint32_t tot = 0, pre = 0;
-        for(uint32_t j = tid; j < G; j += BS) {
-            const uint32_t v = __ldcg(sq.ctas + j);
-            tot += v;
-            pre += j < cb ? v : 0u;
-        }
-        const uint64_t R = block_sum<NW>(tot, s_warp);
-        const uint32_t a_cta = block_sum<NW>(pre, s_warp2);
-        const uint32_t B = min(p.budget, p.cap - tree);
-        k = p.per_entry;
-        uint32_t E = 0;
-        if(B != 0 && R) {
-            if(R * k > B) {
-                k = (uint32_t)(B / R);
-                if(k == 0) k = 1;
-            }
-            E = (uint32_t)(R < (uint64_t)(B / k) ? R : (uint64_t)(B / k));
-            n = E * k;
-        }
-        if(cb == 0 && tid == 0) {
-            ctl->R = (uint32_t)R;
-            ctl->k = k, ctl->E = E, ctl->n = n;
-            if(B == 0) {
-                ctl->full = 1u;
-                finish_query(ctl, active);
-            }
-        }
-        if(B == 0) return;  // every CTA decides alike
-        if(E) {
-            uint64_t a = (uint64_t)a_cta + thr_excl;  // node i owns virtual entries [a, a + rep)
-            uint64_t elo = sum ? entry_ceil(a, E, R) : 0;
-            for(uint32_t i = lo; i < hi; ++i) {
-                const uint32_t cnt = t.rep[i];
-                if(!cnt) continue;
-                const uint64_t bnd = a + cnt, ehi = entry_ceil(bnd, E, R);
-                for(uint64_t e = elo; e < ehi; ++e) sq.entries[e] = i;
-                if(elo < ehi) t.rep[i] = 0;
-                a = bnd, elo = ehi;
-            }
-        }
-        if constexpr(PART == kIterFront) {  // the proposal pass and kIterBack follow
-            if(cb == 0 && tid == 0) ctl->t_front_ns += globaltimer() - s_t[0];
-            return;
-        }
-        if(!grid_barrier(sq.bar, G, &s_flag)) {
-            if(tid == 0) atomicOr(&ctl->error, kErrTimeout), finish_query(ctl, active);
-            return;
-        }
-    } else {
-        k = ctl->k, n = ctl->n;  // the budget and entry list of the front launch
-    }
-    if(tid == 0) s_t[1] = globaltimer();
-
-    // ---- expansion (k_expand); a CTA whose look-back wait gave up has finished the query with an
-    // error and still takes part in the barrier
-    expand_tiles<M, BS>(sq, n, k, cb, G, active, sm, s_save);
-    if(!grid_barrier(sq.bar, G, &s_flag)) {
-        if(tid == 0) atomicOr(&ctl->error, kErrTimeout), finish_query(ctl, active);
-        return;
-    }
-    if constexpr(PART == kIterBack) release_successor();  // every CTA is resident now
-    if(tid == 0) s_t[2] = globaltimer();
-
-    // ---- region scores (k_scores); the last CTA to finish adds the partials and closes the iteration
-    score_partials(sq, cb * BS + tid, G * BS, (int)(cb * NW) + warp, (int)(G * NW));
-    __threadfence();
-    __syncthreads();
-    if(tid == 0) s_last = atomicAdd(sq.sarr, 1u) == G - 1u;
-    __syncthreads();
-    if(!s_last) return;
-    __threadfence();
-    if(tid == 0) *sq.sarr = 0u, sq.bar[0] = 0u;  // every CTA is past the last grid barrier
-    score_finish(sq, active);
+    if(__syncthreads_or(ctl->done != 0u)) return;  // one decision for the whole grid: waits follow
+    const uint32_t max_iters = ctl->max_iters, stop_at_goal = ctl->stop_at_goal;
+    ExpandTotals tot;
     if(tid == 0) {
-        const unsigned long long t4 = globaltimer();
-        if constexpr(PART == kIterWhole) ctl->t_front_ns += s_t[1] - s_t[0];
-        ctl->t_expand_ns += s_t[2] - s_t[1];
-        ctl->t_score_ns += t4 - s_t[2];
+        it.tree = ctl->tree, it.tree_old = ctl->tree_old, it.iter = ctl->iter, it.plan = ctl->plan_idx;
+        it.epoch = ctl->epoch, it.ready = ctl->scores_ready, it.faccept = ctl->faccept, it.total = ctl->score_total;
+        it.goal = ctl->goal_idx != kNone, it.appended = 0, it.full = 0, it.stop = 0, it.n_exp = ctl->n_exp;
+        it.R = 0, it.k = ctl->k, it.E = ctl->E, it.n = ctl->n;  // kIterBack: the front launch's budget
+        s_ns[0] = s_ns[1] = s_ns[2] = 0, s_t[0] = globaltimer();
+    }
+    unsigned long long* const words = sq.words;
+    auto give_up = [&]() {  // no tag published so far may be taken for one of a later plan's
+        if(tid == 0) atomicMax(&ctl->epoch, it.epoch + 1u), atomicOr(&ctl->error, kErrTimeout), finish_query(ctl, active);
+    };
+    auto stamp = [&](int phase, int next) {  // closes a phase's time and starts the next one's
+        if(cb == 0 && tid == 0) {
+            const unsigned long long now = globaltimer();
+            s_ns[phase] += now - s_t[phase];
+            s_t[next] = now;
+        }
+    };
+    __syncthreads();
+    for(uint32_t inner = 0; inner < max_inner; ++inner) {
+        uint32_t k = it.k, n = it.n;  // children per entry and children of this iteration
+        if constexpr(PART != kIterBack) {
+            const uint32_t tree = it.tree, tree_old = it.tree_old, iter = it.iter;
+            const float fa = it.faccept, total = it.total;
+            const uint32_t ready = it.ready;
+
+            // ---- frontier count (k_frontier_count): re-activation of the previous iteration
+            // (KPAX.cu:505-517) and repeats of its new nodes (476-479) over this thread's contiguous
+            // nodes.  Other CTAs' appends, scores and counters of the previous iteration lie behind
+            // its last gather (whose fence drops stale L1 lines).
+            const uint32_t per_cta = (tree + G - 1) / G, per_thr = (per_cta + BS - 1) / BS;
+            const uint32_t c_lo = min(tree, cb * per_cta), c_hi = min(tree, c_lo + per_cta);
+            const uint32_t lo = min(c_hi, c_lo + (uint32_t)tid * per_thr), hi = min(c_hi, lo + per_thr);
+            uint32_t sum = 0;
+            for(uint32_t i0 = lo; i0 < hi; i0 += kIterBatch) {
+                uint32_t r0[kIterBatch];
+                int32_t reg[kIterBatch], nv[kIterBatch];
+                float raw[kIterBatch];
+#pragma unroll
+                for(int j = 0; j < kIterBatch; ++j) {  // each node's byte and region id, then its region's
+                    const uint32_t i = i0 + j;         // score and valid count: two rounds of loads per batch
+                    r0[j] = i < hi ? (uint32_t)t.rep[i] : 0u;
+                    reg[j] = i < hi ? t.r1[i] : 0;
+                }
+#pragma unroll
+                for(int j = 0; j < kIterBatch; ++j) raw[j] = rg.score[reg[j]], nv[j] = rg.valid[reg[j]];
+#pragma unroll
+                for(int j = 0; j < kIterBatch; ++j) {
+                    const uint32_t i = i0 + j;
+                    if(i >= hi) continue;
+                    uint32_t r = r0[j];
+                    if(r == 0u) {
+                        if(i < tree_old) {
+                            const float sc = region_score(raw[j], total, ready, p.eps);
+                            if(reactivate_draw(p, it.plan, iter - 1u, i) <= __fadd_rn(sc, fa)) r = 1u;
+                        }
+                    } else if(r == kPending) {
+                        r = nv[j] < p.sparse_thr ? p.sparse_repeat : 1u;
+                    }
+                    if(r != r0[j]) t.rep[i] = (uint8_t)r;
+                    sum += r;
+                }
+            }
+            // this thread's exclusive prefix inside the CTA, and the CTA's sum
+            uint32_t x = sum;
+#pragma unroll
+            for(int d = 1; d < 32; d <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, x, d);
+                if(lane >= d) x += y;
+            }
+            if(lane == 31) s_warp[warp] = x;
+            __syncthreads();
+            uint32_t wex = 0, cta_sum = 0;
+            for(int w = 0; w < NW; ++w) {
+                wex += w < warp ? s_warp[w] : 0u;
+                cta_sum += s_warp[w];
+            }
+            const uint32_t thr_excl = wex + x - sum;
+            // only the sums themselves cross CTAs here: no fence
+            uint32_t R32 = 0, a_cta = 0;
+            if(!gather_sum<NW>(words + kGatherFrontier * gather_words(G), it.epoch, G, cb, cta_sum, false, sm.gs, a_cta, R32))
+                return give_up();
+            if(inner == 0) release_successor();  // every CTA is resident now
+
+            // ---- budget (KPAX.cu:323-350), then the entry list (k_frontier_write)
+            const uint64_t R = R32;
+            const uint32_t B = min(p.budget, p.cap - tree);
+            uint32_t E = 0;
+            k = p.per_entry, n = 0;
+            if(B != 0 && R) {
+                if(R * k > B) {
+                    k = (uint32_t)(B / R);
+                    if(k == 0) k = 1;
+                }
+                E = (uint32_t)(R < (uint64_t)(B / k) ? R : (uint64_t)(B / k));
+                n = E * k;
+            }
+            if(tid == 0) it.R = R32, it.k = k, it.E = E, it.n = n, it.full = B == 0;
+            if(B == 0) break;  // every CTA decides alike
+            if(E) {
+                uint64_t a = (uint64_t)a_cta + thr_excl;  // node i owns virtual entries [a, a + rep)
+                uint64_t elo = sum ? entry_ceil(a, E, R) : 0;
+                for(uint32_t i = lo; i < hi; ++i) {
+                    const uint32_t cnt = t.rep[i];
+                    if(!cnt) continue;
+                    const uint64_t bnd = a + cnt, ehi = entry_ceil(bnd, E, R);
+                    for(uint64_t e = elo; e < ehi; ++e) {
+                        if constexpr(PART == kIterFront) sq.entries[e] = i;
+                        else st_relaxed(sq.entry_words + e, ((unsigned long long)(it.epoch & kTagMask) << 32) | i);
+                    }
+                    if(elo < ehi) t.rep[i] = 0;
+                    a = bnd, elo = ehi;
+                }
+            }
+            if constexpr(PART == kIterFront) {  // the proposal pass and kIterBack follow
+                stamp(0, 0);
+                break;
+            }
+            // no barrier: the expansion polls the entries it needs (a gather here, whose fence waits
+            // for the entries' stores, took 3.4-4.4 us)
+            stamp(0, 1);
+        } else {
+            stamp(0, 1);
+        }
+
+        // ---- expansion (k_expand): with at most one tile per CTA the tiles' prefixes come from the
+        // gather that ends the phase; more tiles resolve them by look-back, and the gather follows
+        const ExpandState st{it.tree, it.iter, it.plan, it.epoch, it.ready, it.total};
+        const unsigned long long* const w_entries = PART == kIterWhole ? sq.entry_words : nullptr;
+        unsigned long long* const w_children = words + kGatherChildren * gather_words(G);
+        uint32_t appended = 0;
+        bool ok;
+        if((uint64_t)n <= (uint64_t)G * BS) {
+            ok = expand_tiles<M, BS>(sq, st, n, k, cb, G, sm, s_save, tot, w_entries, w_children, &appended);
+        } else {
+            const uint32_t before = tot.accepted;
+            ok = expand_tiles<M, BS>(sq, st, n, k, cb, G, sm, s_save, tot, w_entries);
+            uint32_t below = 0;
+            if(ok) ok = gather_sum<NW>(w_children, it.epoch, G, cb, tot.accepted - before, true, sm.gs, below, appended);
+        }
+        if(!ok) return give_up();
+        if constexpr(PART == kIterBack) release_successor();  // every CTA is resident now
+        stamp(1, 2);
+
+        // ---- region scores (k_scores).  The total's halving tree over the 1024 partials pairs
+        // partial j with j + 512, j + 256, ...: CTA c of the first Q (a power of two) holds the
+        // partials c, c + Q, c + 2Q, ..., so the tree's upper levels are its own and each CTA publishes
+        // one value; the lower levels are added by every warp after the gather.
+        uint32_t Q = kScoreCTAs;
+        while(Q > G) Q >>= 1;
+        const uint32_t per = kPartials / Q, used = min((p.num_r1 + 31u) / 32u, (uint32_t)kPartials);
+        copy_snapshot(sq, cb * BS + tid, G * BS);
+        if(cb < Q)
+            for(uint32_t m = warp; m < per; m += NW) {
+                const uint32_t j = cb + Q * m;
+                const float part = j < used ? score_partial(sq, (int)j) : 0.0f;
+                if(lane == 0) s_part[m] = part;
+            }
+        if(tid < (int)kScoreCTAs) s_val[tid] = 0.0f;
+        const bool goal_here = __syncthreads_or(tot.goal) != 0;
+        unsigned long long* const w_scores = words + kGatherScores * gather_words(G);
+        if(warp == 0) {
+            if(cb < Q) {
+                for(uint32_t h = per >> 1; h > 0; h >>= 1) {
+                    for(uint32_t m = lane; m < h; m += 32) s_part[m] = __fadd_rn(s_part[m], s_part[m + h]);
+                    __syncwarp();
+                }
+            }
+            gather_publish(w_scores, G, cb, it.epoch, cb < Q ? __float_as_uint(s_part[0]) : 0u, goal_here, true);
+        }
+        bool seen = true, goal_any = false;
+        for(uint32_t j = tid; j < G && seen; j += BS) {
+            uint32_t v = 0;
+            bool f = false;
+            seen = gather_poll(w_scores + (cb % kReplicas) * G + j, it.epoch, v, f);
+            goal_any = goal_any || f;
+            if(j < Q) s_val[j] = __uint_as_float(v);
+        }
+        if((uint32_t)tid < G) fence_gpu();
+        if(!__syncthreads_and(seen)) return give_up();
+        goal_any = __syncthreads_or(goal_any) != 0;
+        if(warp == 0) {
+            float v[kScoreCTAs / 32];
+#pragma unroll
+            for(int m = 0; m < (int)kScoreCTAs / 32; ++m) v[m] = s_val[lane + 32 * m];
+#pragma unroll
+            for(int h = (int)kScoreCTAs / 64; h >= 1; h >>= 1)
+#pragma unroll
+                for(int m = 0; m < h; ++m) v[m] = __fadd_rn(v[m], v[m + h]);
+            for(int sh = 16; sh > 0; sh >>= 1) {
+                const float o = __shfl_down_sync(0xffffffffu, v[0], sh);
+                if(lane < sh) v[0] = __fadd_rn(v[0], o);
+            }
+            if(lane == 0) {  // the iteration's bookkeeping (score_finish)
+                const uint32_t iter = it.iter;
+                it.total = v[0], it.ready = 1u;
+                it.tree_old = it.tree, it.tree += appended, it.appended = appended;
+                it.faccept = accept_rate(p, iter, it.tree);
+                it.n_exp += n;
+                it.iter = iter + 1u, it.epoch += 1u;
+                it.goal |= goal_any ? 1u : 0u;
+                it.stop = (it.goal && stop_at_goal) || iter >= max_iters;
+            }
+        }
+        __syncthreads();
+        stamp(2, 0);
+        if(it.stop) break;
+    }
+    if(tid == 0) {
+        if(tot.valid) atomicAdd(&ctl->n_valid, tot.valid);
+        if(tot.steps) atomicAdd(&ctl->n_steps, tot.steps);
+        if(cb == 0) {
+            ctl->t_front_ns += s_ns[0], ctl->t_expand_ns += s_ns[1], ctl->t_score_ns += s_ns[2];
+            ctl->k = it.k, ctl->E = it.E, ctl->n = it.n;
+            if constexpr(PART != kIterBack) ctl->R = it.R, ctl->full = it.full;
+            if constexpr(PART != kIterFront) {
+                ctl->tree = it.tree, ctl->tree_old = it.tree_old, ctl->appended = it.appended;
+                ctl->faccept = it.faccept, ctl->score_total = it.total, ctl->scores_ready = it.ready;
+                ctl->n_exp = it.n_exp, ctl->iter = it.iter, ctl->iters_done = it.iter - 1u, ctl->epoch = it.epoch;
+            }
+            if(it.full || it.stop) finish_query(ctl, active);
+        }
     }
 }
 

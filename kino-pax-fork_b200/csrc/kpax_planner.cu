@@ -22,8 +22,11 @@ using namespace kpax::plan;
 namespace {
 
 constexpr int kFrontierCTAs = kFrontierMinBlocks * 148;  // one round over the tiles of a 600k-node tree
-constexpr int kScoreCTAs = 128;
 constexpr size_t kAlign = 256;
+// Iterations between two looks at the done flag (kpax_config.unroll_iters = 0): a captured graph's, and
+// one fused launch's, which ends by itself when the plan does, so that more iterations cost nothing
+// and spare the host's round trip (~15 us each, 0.2 us per iteration at 64).
+constexpr int kGraphIters = 8, kFusedIters = 64;
 
 // Sub-allocations of one device allocation.
 struct Carver {
@@ -108,14 +111,17 @@ void* iterate_kernel(int bs)
 }
 
 template <int M, int PART = kIterWhole>
-void launch_iterate(int bs, uint32_t gx, cudaStream_t s, const QueryDev* dq, const Ctl* ctl, uint32_t* active)
+void launch_iterate(int bs, uint32_t gx, cudaStream_t s, const QueryDev* dq, const Ctl* ctl, uint32_t* active, uint32_t inner)
 {
     const size_t smem = PART == kIterFront ? 0 : save_bytes(M, bs);
+    // not a cooperative launch: its residency check costs 70-100 us per launch, and a grid sized by the
+    // kernel's occupancy becomes resident as a whole once the SMs are free (the waits are bounded)
+    auto go = [&](auto kernel, unsigned block) { launch_chained(kernel, dim3(gx), block, smem, s, dq, ctl, active, inner); };
     switch(bs) {
-        case 128: launch_chained(k_iterate<M, 128, PART>, dim3(gx), 128, smem, s, dq, ctl, active); break;
-        case 256: launch_chained(k_iterate<M, 256, PART>, dim3(gx), 256, smem, s, dq, ctl, active); break;
-        case 512: launch_chained(k_iterate<M, 512, PART>, dim3(gx), 512, smem, s, dq, ctl, active); break;
-        default: launch_chained(k_iterate<M, kExpandBS, PART>, dim3(gx), kExpandBS, smem, s, dq, ctl, active); break;
+        case 128: go(k_iterate<M, 128, PART>, 128); break;
+        case 256: go(k_iterate<M, 256, PART>, 256); break;
+        case 512: go(k_iterate<M, 512, PART>, 512); break;
+        default: go(k_iterate<M, kExpandBS, PART>, kExpandBS); break;
     }
 }
 
@@ -209,7 +215,7 @@ struct PlanBatch {
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     cudaGraphExec_t graph = nullptr;
     std::vector<const void*> graph_key;
-    int unroll = 8;
+    int unroll = kGraphIters;
     uint32_t plans = 0;
     bool begun = false;
     // single-query extras: debug capture and benchmark timing
@@ -237,14 +243,11 @@ struct PlanBatch {
         env.resize(n);
         hq.assign(n, QueryDev{});
         path_off.resize(n);
-        int unroll_cfg = 0;
         for(uint32_t q = 0; q < n; ++q) {
             kpax_status st = derive_params(cfg[q], &prm[q]);
             if(st != KPAX_OK) return st;
             s_max = std::max<uint32_t>(s_max, (uint32_t)prm[q].S);
-            unroll_cfg = std::max(unroll_cfg, cfg[q].unroll_iters);
         }
-        unroll = unroll_cfg > 0 ? unroll_cfg : 8;
         // two passes: size the pool, then carve it
         for(int pass = 0; pass < 2; ++pass) {
             Carver cv;
@@ -270,8 +273,8 @@ struct PlanBatch {
                 d.partials = cv.take<float>(kPartials);
                 d.farr = cv.take<uint32_t>(1);
                 d.sarr = cv.take<uint32_t>(1);
-                d.bar = cv.take<uint32_t>(2);
-                d.ctas = cv.take<uint32_t>(kIterMaxCTAs);
+                d.entry_words = n == 1 ? cv.take<unsigned long long>(p.budget) : nullptr;
+                d.words = n == 1 ? cv.take<unsigned long long>(kGathers * gather_words(kIterMaxCTAs)) : nullptr;
                 d.path_rows = cfg[q].max_iter + 2;
                 path_off[q] = prow;
                 prow += d.path_rows;
@@ -436,6 +439,9 @@ struct PlanBatch {
     {
         fused = nq == 1 && gx_iter > 0 && cfg[0].iteration_kernels == 0 && n_learned == 0;
         fused_split = nq == 1 && gx_split > 0 && cfg[0].iteration_kernels == 0 && n_learned == 1;
+        int asked = 0;
+        for(const kpax_config& c : cfg) asked = std::max(asked, c.unroll_iters);
+        unroll = asked > 0 ? asked : (fused ? kFusedIters : kGraphIters);
     }
 
     void release()
@@ -499,22 +505,22 @@ struct PlanBatch {
 
     // ev (optional): four events recorded before the frontier, expansion and score kernels and after;
     // with split == false only the first and the last, so the launches still overlap.
-    void launch_iteration(cudaEvent_t* ev = nullptr, bool split = true)
+    void launch_iteration(cudaEvent_t* ev = nullptr, bool split = true, uint32_t inner = 1)
     {
         if(ev) cudaEventRecord(ev[0], stream);
         if(fused_split) {  // front launch, proposal pass, back launch; phase times from the device clock
-            launch_iterate<KPAX_MODEL_QUADROTOR, kIterFront>(expand_bs[2], gx_split, stream, dq, d_ctl, d_active);
+            launch_iterate<KPAX_MODEL_QUADROTOR, kIterFront>(expand_bs[2], gx_split, stream, dq, d_ctl, d_active, 1);
             launch_proposal(stream);
-            launch_iterate<KPAX_MODEL_QUADROTOR, kIterBack>(expand_bs[2], gx_split, stream, dq, d_ctl, d_active);
+            launch_iterate<KPAX_MODEL_QUADROTOR, kIterBack>(expand_bs[2], gx_split, stream, dq, d_ctl, d_active, 1);
             if(ev) cudaEventRecord(ev[3], stream);
             return;
         }
-        if(fused) {  // one launch: its phase times come from the device clock (Ctl::t_*_ns)
+        if(fused) {  // one launch of up to `inner` iterations: phase times from the device clock (Ctl::t_*_ns)
             const int m = prm[0].model - 1;
             const Ctl* c0 = d_ctl;  // the single query's control block
-            if(m == 0) launch_iterate<KPAX_MODEL_DOUBLE_INTEGRATOR>(expand_bs[m], gx_iter, stream, dq, c0, d_active);
-            else if(m == 1) launch_iterate<KPAX_MODEL_DUBINS_AIRPLANE>(expand_bs[m], gx_iter, stream, dq, c0, d_active);
-            else launch_iterate<KPAX_MODEL_QUADROTOR>(expand_bs[m], gx_iter, stream, dq, c0, d_active);
+            if(m == 0) launch_iterate<KPAX_MODEL_DOUBLE_INTEGRATOR>(expand_bs[m], gx_iter, stream, dq, c0, d_active, inner);
+            else if(m == 1) launch_iterate<KPAX_MODEL_DUBINS_AIRPLANE>(expand_bs[m], gx_iter, stream, dq, c0, d_active, inner);
+            else launch_iterate<KPAX_MODEL_QUADROTOR>(expand_bs[m], gx_iter, stream, dq, c0, d_active, inner);
             if(ev) cudaEventRecord(ev[3], stream);
             return;
         }
@@ -697,6 +703,7 @@ struct PlanBatch {
 
     kpax_status ensure_graph()
     {
+        if(fused) return KPAX_OK;  // one kernel runs the iterations
         std::vector<const void*> key;
         for(uint32_t q = 0; q < nq; ++q) key.push_back(env[q].d_ent), key.push_back(env[q].d_obs);
         key.push_back(cap.rows);
@@ -747,14 +754,20 @@ struct PlanBatch {
         return ensure_graph();
     }
 
-    // Runs graphs until no query is active; `guard` bounds the number of graph launches.  With
+    // Runs graphs (or fused launches) until no query is active; `guard` bounds their number.  With
     // poll = false all launches are queued first and the stream is synchronised once.
     kpax_status run(uint32_t guard, bool poll = true)
     {
         NvtxRange range("kpax plan iterations");
         for(uint32_t g = 0; g < guard; ++g) {
-            KPAX_CUDA(cudaGraphLaunch(graph, stream));
-            count_launch(kernels_per_iteration() * (uint64_t)unroll);
+            if(fused) {
+                launch_iteration(nullptr, true, (uint32_t)unroll);
+                KPAX_CHECK_LAUNCH();
+                count_launch(1);
+            } else {
+                KPAX_CUDA(cudaGraphLaunch(graph, stream));
+                count_launch(kernels_per_iteration() * (uint64_t)unroll);
+            }
             if(!poll) continue;
             KPAX_CUDA(cudaMemcpyAsync(h_active, d_active, sizeof(uint32_t), cudaMemcpyDeviceToHost, stream));
             KPAX_CUDA(cudaStreamSynchronize(stream));
