@@ -207,7 +207,7 @@ __global__ void __launch_bounds__(BS, (kExpandAllMinBlocks<M, BS>)) k_expand_all
                                                                                 const uint32_t* __restrict__ qidx,
                                                                                 uint32_t nq, uint32_t* __restrict__ active)
 {
-    extern __shared__ float s_save[];  // kept states, then the offsets
+    extern __shared__ __align__(16) float s_save[];  // kept states, then the offsets
     uint32_t* s_off = reinterpret_cast<uint32_t*>(s_save + kSaveBytes<M, BS, kGroupAll<M, BS>> / sizeof(float));
     __shared__ QueryDev sq;
     __shared__ ExpandSmem<BS / 32> sm;
@@ -239,7 +239,7 @@ __global__ void __launch_bounds__(BS, (512 / BS > 0 ? 512 / BS : 1)) k_expand_mi
                                                                                   const uint32_t* __restrict__ qidx,
                                                                                   uint32_t nq, uint32_t* __restrict__ active)
 {
-    extern __shared__ float s_save[];  // kept states, then the offsets
+    extern __shared__ __align__(16) float s_save[];  // kept states, then the offsets
     uint32_t* s_off = reinterpret_cast<uint32_t*>(s_save + kSaveBytes<KPAX_MODEL_QUADROTOR, BS> / sizeof(float));
     __shared__ QueryDev sq;
     __shared__ ExpandSmem<BS / 32> sm;

@@ -75,7 +75,10 @@ constexpr float kTrigFastMax = 8192.0f;
 
 __device__ __forceinline__ void sincos_fast(float x, float* sn, float* cs)
 {
-    const float n = rintf(x * 0.636619772367581343f);  // 2 / pi
+    // nearest integer of x * 2 / pi by adding 1.5 * 2^23, whose low mantissa bits then hold it
+    const float t = __fadd_rn(__fmul_rn(x, 0.636619772367581343f), 12582912.0f);
+    const float n = __fsub_rn(t, 12582912.0f);
+    const uint32_t q = __float_as_uint(t);
     float r = fmaf(n, -1.5703125f, x);
     r = fmaf(n, -4.837512969970703125e-4f, r);
     r = fmaf(n, -7.54978995489188216e-8f, r);
@@ -83,16 +86,50 @@ __device__ __forceinline__ void sincos_fast(float x, float* sn, float* cs)
     const float ps = fmaf(fmaf(fmaf(-1.9515295891e-4f, z, 8.3321608736e-3f), z, -1.6666654611e-1f), z * r, r);
     const float pc = fmaf(fmaf(fmaf(2.443315711809948e-5f, z, -1.388731625493765e-3f), z, 4.166664568298827e-2f), z * z,
                           fmaf(-0.5f, z, 1.0f));
-    const int q = (int)n & 3;
-    const float a = (q & 1) ? pc : ps, b = (q & 1) ? ps : pc;
-    *sn = (q & 2) ? -a : a;
-    *cs = ((q + 1) & 2) ? -b : b;
+    const bool odd = (q & 1u) != 0u;
+    const float a = odd ? pc : ps, b = odd ? ps : pc;
+    *sn = __uint_as_float(__float_as_uint(a) ^ ((q & 2u) << 30));
+    *cs = __uint_as_float(__float_as_uint(b) ^ (((q + 1u) & 2u) << 30));
 }
 
 __device__ __forceinline__ void sincos_checked(float x, float* sn, float* cs)
 {
     sincos_fast(x, sn, cs);
     if(!(fabsf(x) <= kTrigFastMax)) sincosf(x, sn, cs);  // huge or non-finite arguments
+}
+
+// (sin, cos) of up to four arguments on a path that a step rarely takes: one copy of the code for all,
+// so that it does not crowd the step's instructions.  Each as sincos_checked; `huge_only` leaves the
+// arguments within kTrigFastMax as they are.
+template <int N>
+__device__ __forceinline__ void sincos_rare(const float (&x)[N], float* sc, bool huge_only)
+{
+#pragma unroll 1
+    for(int d = 0; d < N; ++d) {
+        float v = x[0], s, c;
+#pragma unroll
+        for(int j = 1; j < N; ++j) v = d == j ? x[j] : v;
+        if(huge_only && fabsf(v) <= kTrigFastMax) continue;
+        sincos_checked(v, &s, &c);
+#pragma unroll
+        for(int j = 0; j < N; ++j) {
+            sc[2 * j] = d == j ? s : sc[2 * j];
+            sc[2 * j + 1] = d == j ? c : sc[2 * j + 1];
+        }
+    }
+}
+
+// N arguments with one test for the common case (a NaN or infinity fails it).
+template <int N>
+__device__ __forceinline__ void sincos_all(const float (&x)[N], float* sc)
+{
+    bool fast = true;
+#pragma unroll
+    for(int d = 0; d < N; ++d) {
+        sincos_fast(x[d], &sc[2 * d], &sc[2 * d + 1]);
+        fast = fast && fabsf(x[d]) <= kTrigFastMax;
+    }
+    if(!fast) sincos_rare(x, sc, true);
 }
 
 // sin and cos of a0 + d from s0 = sin(a0), c0 = cos(a0) by the angle-sum identity, with the
@@ -139,6 +176,38 @@ __device__ __forceinline__ float rcp_approx(float x)
     float y;
     asm("rcp.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
+}
+
+// Two FP32 values per instruction (fma.rn.f32x2 and friends of sm_100a): each half rounds as the scalar
+// operation does.  The quadrotor's step is bound by its instruction count (559 of 800 instructions per
+// step on the FMA pipes); its element-wise updates take half as many this way: 2^20 segments without
+// obstacles 701 -> 663 us, 2^16 62.2 -> 58.2 us.
+typedef unsigned long long F2;
+
+__device__ __forceinline__ F2 f2(float lo, float hi)
+{
+    F2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ F2 f2(float x) { return f2(x, x); }
+__device__ __forceinline__ float2 unpack(F2 v)
+{
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c)
+{
+    F2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ F2 mul2(F2 a, F2 b)
+{
+    F2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
 }
 
 // float -> int with the reference's device semantics (saturating, NaN -> 0).
@@ -330,14 +399,14 @@ __device__ __forceinline__ int first_hit(const Grid& g, const float lo[3], const
 }
 
 // x * 0 is +-0 for a finite x and NaN for an infinite or NaN one, so the sum of those products is
-// 0 exactly when every value is finite (two chains for a shorter dependency).
+// 0 exactly when every value is finite (n even).
 __device__ __forceinline__ bool finite_all(const float* s, int n)
 {
-    float a = 0.0f, b = 0.0f;
+    F2 a = f2(0.0f);
 #pragma unroll
-    for(int i = 0; i + 1 < n; i += 2) a = __fmaf_rn(s[i], 0.0f, a), b = __fmaf_rn(s[i + 1], 0.0f, b);
-    if(n & 1) a = __fmaf_rn(s[n - 1], 0.0f, a);
-    return __fadd_rn(a, b) == 0.0f;
+    for(int i = 0; i + 1 < n; i += 2) a = fma2(f2(s[i], s[i + 1]), f2(0.0f), a);
+    const float2 v = unpack(a);
+    return __fadd_rn(v.x, v.y) == 0.0f;
 }
 
 // ------------------------------------------------------------------ controls
@@ -428,18 +497,22 @@ __device__ __forceinline__ bool step_dubins(const StepParams& p, float* s, const
     const float a = c[0], yr = c[1], pr = c[2];
     const float yaw = s[3], pitch = s[4], v = s[5];
     float sp0, cp0, sy0, cy0, sp1, cp1, sy1, cy1, sp2, cp2, sy2, cy2;
-    sincos_checked(pitch, &sp0, &cp0);
-    sincos_checked(yaw, &sy0, &cy0);
+    {
+        const float x[2] = {pitch, yaw};
+        float sc[4];
+        sincos_all(x, sc);
+        sp0 = sc[0], cp0 = sc[1], sy0 = sc[2], cy0 = sc[3];
+    }
     if(k.shift) {
         sincos_apply(sp0, cp0, k.p1, &sp1, &cp1);
         sincos_apply(sy0, cy0, k.y1, &sy1, &cy1);
         sincos_apply(sp0, cp0, k.p2, &sp2, &cp2);
         sincos_apply(sy0, cy0, k.y2, &sy2, &cy2);
     } else {
-        sincos_checked(__fmaf_rn(hh, pr, pitch), &sp1, &cp1);
-        sincos_checked(__fmaf_rn(hh, yr, yaw), &sy1, &cy1);
-        sincos_checked(__fmaf_rn(h, pr, pitch), &sp2, &cp2);
-        sincos_checked(__fmaf_rn(h, yr, yaw), &sy2, &cy2);
+        const float x[4] = {__fmaf_rn(hh, pr, pitch), __fmaf_rn(hh, yr, yaw), __fmaf_rn(h, pr, pitch), __fmaf_rn(h, yr, yaw)};
+        float sc[8] = {};
+        sincos_rare(x, sc, false);
+        sp1 = sc[0], cp1 = sc[1], sy1 = sc[2], cy1 = sc[3], sp2 = sc[4], cp2 = sc[5], sy2 = sc[6], cy2 = sc[7];
     }
     // every rounding written out (as the quadrotor's): the same bits wherever the step is inlined
     const float vm = __fmaf_rn(hh, a, v), ve = __fmaf_rn(h, a, v);
@@ -526,24 +599,26 @@ __device__ __forceinline__ QuadTrig quad_stage_trig(const float* a0, const float
         sincos_shift(trig0[2], trig0[3], d1, &t.st, &t.ct);
         sincos_shift(trig0[4], trig0[5], d2, &t.sp, &t.cp);
     } else {
-        sincos_checked(__fadd_rn(a0[0], d0), &t.sf, &t.cf);
-        sincos_checked(__fadd_rn(a0[1], d1), &t.st, &t.ct);
-        sincos_checked(__fadd_rn(a0[2], d2), &t.sp, &t.cp);
+        const float x[3] = {__fadd_rn(a0[0], d0), __fadd_rn(a0[1], d1), __fadd_rn(a0[2], d2)};
+        float sc[6] = {};
+        sincos_rare(x, sc, false);
+        t = {sc[0], sc[1], sc[2], sc[3], sc[4], sc[5]};
     }
     return t;
 }
 
 __device__ __forceinline__ QuadRates quad_stage_rates(const float* v0, const float* kv, float delta)
 {
-    return {__fmaf_rn(delta, kv[0], v0[0]), __fmaf_rn(delta, kv[1], v0[1]), __fmaf_rn(delta, kv[2], v0[2]),
-            __fmaf_rn(delta, kv[3], v0[3]), __fmaf_rn(delta, kv[4], v0[4]), __fmaf_rn(delta, kv[5], v0[5])};
+    const F2 d = f2(delta);
+    const float2 a = unpack(fma2(d, f2(kv[0], kv[1]), f2(v0[0], v0[1]))), b = unpack(fma2(d, f2(kv[2], kv[3]), f2(v0[2], v0[3]))),
+                 c = unpack(fma2(d, f2(kv[4], kv[5]), f2(v0[4], v0[5])));
+    return {a.x, a.y, b.x, b.y, c.x, c.y};
 }
 
 __device__ __forceinline__ void quad_trig0(const float* a0, float* trig0)
 {
-    sincos_checked(a0[0], &trig0[0], &trig0[1]);
-    sincos_checked(a0[1], &trig0[2], &trig0[3]);
-    sincos_checked(a0[2], &trig0[4], &trig0[5]);
+    const float x[3] = {a0[0], a0[1], a0[2]};
+    sincos_all(x, trig0);
 }
 
 // The per-step bounds checks of each half (velocity box; workspace; finite).
@@ -571,7 +646,8 @@ __device__ __forceinline__ bool quad_kin_ok(const StepParams& p, const float* x)
 __device__ __forceinline__ bool step_quad(const StepParams& p, float* s, const float* c)
 {
     const float h = p.h, hh = p.hh, h6 = p.h6;
-    float k[12], acc[12], trig0[6];
+    float k[12], trig0[6];
+    F2 acc[6];
     quad_trig0(s + 3, trig0);
     {
         const QuadTrig t = quad_first_trig(trig0);
@@ -580,7 +656,7 @@ __device__ __forceinline__ bool step_quad(const StepParams& p, float* s, const f
         quad_dyn(k + 6, t.sf, t.cf, t.st, t.ct, b, c);
     }
 #pragma unroll
-    for(int j = 0; j < 12; ++j) acc[j] = k[j];
+    for(int j = 0; j < 6; ++j) acc[j] = f2(k[2 * j], k[2 * j + 1]);
 #pragma unroll 1
     for(int stage = 1; stage < 4; ++stage) {
         const float delta = stage == 3 ? h : hh, w = stage == 3 ? 1.0f : 2.0f;
@@ -589,10 +665,13 @@ __device__ __forceinline__ bool step_quad(const StepParams& p, float* s, const f
         quad_kin(k, t, b);
         quad_dyn(k + 6, t.sf, t.cf, t.st, t.ct, b, c);
 #pragma unroll
-        for(int j = 0; j < 12; ++j) acc[j] = __fmaf_rn(w, k[j], acc[j]);
+        for(int j = 0; j < 6; ++j) acc[j] = fma2(f2(w), f2(k[2 * j], k[2 * j + 1]), acc[j]);
     }
 #pragma unroll
-    for(int j = 0; j < 12; ++j) s[j] = __fmaf_rn(h6, acc[j], s[j]);
+    for(int j = 0; j < 6; ++j) {
+        const float2 v = unpack(fma2(f2(h6), acc[j], f2(s[2 * j], s[2 * j + 1])));
+        s[2 * j] = v.x, s[2 * j + 1] = v.y;
+    }
     return quad_dyn_ok(p, s + 6) && quad_kin_ok(p, s);
 }
 
@@ -640,13 +719,45 @@ struct ModelDims<KPAX_MODEL_QUADROTOR> {
 // shared memory of the states.  B200, groups of five against a query per step: expansion of 2^16
 // quadrotor children in the building scene 83.2 -> 67.3 us, 2^14 children 67 -> 57 us, Dubins in the
 // forest 27.0 -> 22.7 us; 2^22 Dubins segments 848 -> 672 us; the double integrator, whose expansion
-// is mostly its fixed part, 18 us either way.  save: K x SD floats of this thread, `stride` floats
-// apart.
+// is mostly its fixed part, 18 us either way.  save: this thread's SD floats of the first
+// step of the block's K x `threads` x SD (a warp's 16- or 8-byte accesses to them are conflict-free).
+template <int SD>
+__device__ __forceinline__ void save_state(float* dst, const float* s)
+{
+    if constexpr(SD == 12) {
+#pragma unroll
+        for(int q = 0; q < 3; ++q)
+            reinterpret_cast<float4*>(dst)[q] = make_float4(s[4 * q], s[4 * q + 1], s[4 * q + 2], s[4 * q + 3]);
+    } else {
+#pragma unroll
+        for(int q = 0; q < SD / 2; ++q) reinterpret_cast<float2*>(dst)[q] = make_float2(s[2 * q], s[2 * q + 1]);
+    }
+}
+
+template <int SD>
+__device__ __forceinline__ void take_state(const float* src, float* s)
+{
+    if constexpr(SD == 12) {
+#pragma unroll
+        for(int q = 0; q < 3; ++q) {
+            const float4 v = reinterpret_cast<const float4*>(src)[q];
+            s[4 * q] = v.x, s[4 * q + 1] = v.y, s[4 * q + 2] = v.z, s[4 * q + 3] = v.w;
+        }
+    } else {
+#pragma unroll
+        for(int q = 0; q < SD / 2; ++q) {
+            const float2 v = reinterpret_cast<const float2*>(src)[q];
+            s[2 * q] = v.x, s[2 * q + 1] = v.y;
+        }
+    }
+}
+
 template <int M, int K, class C>
 __device__ __forceinline__ bool run_steps(const StepParams& p, const Grid& g, float* s, const float* c, const C& k, int end,
-                                          int& done, float* save, int stride)
+                                          int& done, float* save, int threads)
 {
     constexpr int SD = ModelDims<M>::SD;
+    const int stride = threads * SD;
     while(done < end) {
         const int m = min(K, end - done);
         const float p0[3] = {s[0], s[1], s[2]};
@@ -656,17 +767,15 @@ __device__ __forceinline__ bool run_steps(const StepParams& p, const Grid& g, fl
 #pragma unroll 1
         while(n < m) {
             ok = model_step<M>(p, s, c, k);
-#pragma unroll
-            for(int d = 0; d < SD; ++d) save[(n * SD + d) * stride] = s[d];
+            save_state<SD>(save + n * stride, s);
             if(!ok) break;
 #pragma unroll
             for(int d = 0; d < 3; ++d) lo[d] = fminf(lo[d], s[d]), hi[d] = fmaxf(hi[d], s[d]);
             ++n;
         }
-        const int hit = n ? first_hit(g, lo, hi, n, [&](int j, int d) { return j ? save[((j - 1) * SD + d) * stride] : p0[d]; }) : 0;
+        const int hit = n ? first_hit(g, lo, hi, n, [&](int j, int d) { return j ? save[(j - 1) * stride + d] : p0[d]; }) : 0;
         if(hit < n) {
-#pragma unroll
-            for(int d = 0; d < SD; ++d) s[d] = save[(hit * SD + d) * stride];
+            take_state<SD>(save + hit * stride, s);
             ok = false;
         }
         if(!ok) {
@@ -682,13 +791,13 @@ __device__ __forceinline__ bool run_steps(const StepParams& p, const Grid& g, fl
 // steps executed (the failing one included).
 template <int M, int K>
 __device__ __forceinline__ bool propagate(const KParams& p, const Grid& g, float* s, const float* c, int steps, int& done,
-                                          float* save, int stride)
+                                          float* save, int threads)
 {
     const auto k = segment_consts<M>(p, c);
     const StepParams sp = step_params(p);
     const Grid gl = g;  // register copy of the grid's pointers and cell map
     done = min(0, steps);  // a caller's draws may ask for no step
-    return run_steps<M, K>(sp, gl, s, c, k, steps, done, save, stride);
+    return run_steps<M, K>(sp, gl, s, c, k, steps, done, save, threads);
 }
 
 // Controls as stored in the row: Dubins stores (yawRate, pitchRate, a) (statePropagatorSpatialHash.cu:223-225).

@@ -136,19 +136,24 @@ inline uint32_t warp_blocks(uint32_t n) { return (uint32_t)(((uint64_t)n * 32 + 
 
 // ---------------------------------------------------------------- batch kernels
 
-// Steps per collision query of the batch kernels (run_steps): 256-thread CTAs, four per SM, so the
-// kept states of a CTA must stay below the 48 KB of static shared memory.
+// CTAs of the batch kernels: 256 threads, four per SM (64 registers), for the 6-state models; the
+// quadrotor's step keeps over 100 values, and at 64 registers its spills cost more than the warps
+// gain (30011 segments in the building scene 70 us spilling, 53 us at 128 registers; 2^20 555 -> 448 us).
+// kBatchGroup: steps per collision query (run_steps), whose kept states must stay below the
+// 48 KB of static shared memory.
 template <int M>
-constexpr int kBatchGroup = M == KPAX_MODEL_QUADROTOR ? 3 : 5;
+constexpr int kBatchBS = M == KPAX_MODEL_QUADROTOR ? 128 : 256;
+constexpr int kBatchBlocks = 4;
+constexpr int kBatchGroup = 5;
 
 template <int M>
-__global__ void __launch_bounds__(256, 4) k_propagate_batch(KParams p, Grid g, const float* __restrict__ parents,
+__global__ void __launch_bounds__(kBatchBS<M>, kBatchBlocks) k_propagate_batch(KParams p, Grid g, const float* __restrict__ parents,
                                                          const float* __restrict__ draws, uint32_t stream_id, uint32_t n,
                                                          float* __restrict__ rows, uint8_t* __restrict__ valid,
                                                          int32_t* __restrict__ steps_out)
 {
     constexpr int SD = ModelDims<M>::SD, CD = ModelDims<M>::CD, S = SD + CD + 1;
-    __shared__ float s_save[kBatchGroup<M> * SD * 256];
+    __shared__ __align__(16) float s_save[kBatchGroup * SD * kBatchBS<M>];
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if(i >= n) return;
     float s[SD], u[6], c[4], rc[4];
@@ -163,7 +168,7 @@ __global__ void __launch_bounds__(256, 4) k_propagate_batch(KParams p, Grid g, c
     }
     const int steps = draw_controls(p, u, c);
     int done = 0;
-    const bool ok = propagate<M, kBatchGroup<M>>(p, g, s, c, steps, done, s_save + threadIdx.x, 256);
+    const bool ok = propagate<M, kBatchGroup>(p, g, s, c, steps, done, s_save + threadIdx.x * SD, kBatchBS<M>);
     row_controls<M>(c, rc);
     float* dst = rows + (size_t)i * S;
 #pragma unroll
@@ -244,13 +249,13 @@ __device__ __forceinline__ void append_live(const LiveList& live, bool alive, in
 // Segments i of one round (pointers offset to the round's first segment; i0 = that segment's index
 // in the batch, which keys its draws).
 template <int M>
-__global__ void __launch_bounds__(256, 4) k_propagate_head(KParams p, Grid g, const float* __restrict__ parents,
+__global__ void __launch_bounds__(kBatchBS<M>, kBatchBlocks) k_propagate_head(KParams p, Grid g, const float* __restrict__ parents,
                                                         const float* __restrict__ draws, uint32_t stream_id, uint32_t n,
                                                         uint32_t i0, float* __restrict__ rows, uint8_t* __restrict__ valid,
                                                         int32_t* __restrict__ steps_out, LiveList live)
 {
     constexpr int SD = ModelDims<M>::SD, CD = ModelDims<M>::CD;
-    __shared__ float s_save[kHeadSteps * SD * 256];
+    __shared__ __align__(16) float s_save[kHeadSteps * SD * kBatchBS<M>];
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     const int lane = threadIdx.x & 31;
     bool alive = false;
@@ -271,7 +276,7 @@ __global__ void __launch_bounds__(256, 4) k_propagate_head(KParams p, Grid g, co
         const auto k = segment_consts<M>(p, c);
         const StepParams sp = step_params(p);
         int done = 0;
-        const bool ok = run_steps<M, kHeadSteps>(sp, g, s, c, k, min(steps, kHeadSteps), done, s_save + threadIdx.x, 256);
+        const bool ok = run_steps<M, kHeadSteps>(sp, g, s, c, k, min(steps, kHeadSteps), done, s_save + threadIdx.x * SD, kBatchBS<M>);
         alive = ok && done < steps;
         if(!alive) write_segment<M>(p, i, s, c, steps, ok, done, rows, valid, steps_out);
     }
@@ -279,12 +284,12 @@ __global__ void __launch_bounds__(256, 4) k_propagate_head(KParams p, Grid g, co
 }
 
 template <int M>
-__global__ void __launch_bounds__(256, 4) k_propagate_tail(KParams p, Grid g, float* __restrict__ rows,
+__global__ void __launch_bounds__(kBatchBS<M>, kBatchBlocks) k_propagate_tail(KParams p, Grid g, float* __restrict__ rows,
                                                         uint8_t* __restrict__ valid, int32_t* __restrict__ steps_out,
                                                         LiveList live, int from, int until, LiveList next)
 {
     constexpr int SD = ModelDims<M>::SD, CD = ModelDims<M>::CD;
-    __shared__ float s_save[kBatchGroup<M> * SD * 256];
+    __shared__ __align__(16) float s_save[kBatchGroup * SD * kBatchBS<M>];
     const uint32_t count = *live.count;
     if(blockIdx.x * blockDim.x >= count) return;  // whole block past the list: the ballot below needs full warps
     const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
@@ -303,7 +308,7 @@ __global__ void __launch_bounds__(256, 4) k_propagate_tail(KParams p, Grid g, fl
         const auto kc = segment_consts<M>(p, c);
         const StepParams sp = step_params(p);
         int done = from;
-        const bool ok = run_steps<M, kBatchGroup<M>>(sp, g, s, c, kc, min(steps, until), done, s_save + threadIdx.x, 256);
+        const bool ok = run_steps<M, kBatchGroup>(sp, g, s, c, kc, min(steps, until), done, s_save + threadIdx.x * SD, kBatchBS<M>);
         alive = next.count && ok && done < steps;
         if(!alive) write_segment<M>(p, i, s, c, steps, ok, done, rows, valid, steps_out);
     }
@@ -319,15 +324,15 @@ void launch_phases(const KParams& p, const Grid& g, const float* parents, const 
 {
     const int SD = p.sd, S = p.S, mid = mid_steps(p);
     for(uint32_t o = 0; o < n; o += kPhaseChunk) {
-        const uint32_t m = std::min(kPhaseChunk, n - o), blocks = (m + 255) / 256;
+        const uint32_t m = std::min(kPhaseChunk, n - o), bs = kBatchBS<M>, blocks = (m + bs - 1) / bs;
         float* r = rows + (size_t)o * S;
         uint8_t* v = valid + o;
         int32_t* st = steps_out ? steps_out + o : nullptr;
         cudaMemsetAsync(counts, 0, 256, s);
-        k_propagate_head<M><<<blocks, 256, 0, s>>>(p, g, parents + (size_t)o * SD, draws ? draws + (size_t)o * 5 : nullptr,
+        k_propagate_head<M><<<blocks, bs, 0, s>>>(p, g, parents + (size_t)o * SD, draws ? draws + (size_t)o * 5 : nullptr,
                                                    stream_id, m, o, r, v, st, first);
-        k_propagate_tail<M><<<blocks, 256, 0, s>>>(p, g, r, v, st, first, kHeadSteps, mid, second);
-        k_propagate_tail<M><<<blocks, 256, 0, s>>>(p, g, r, v, st, second, mid, INT_MAX, none);
+        k_propagate_tail<M><<<blocks, bs, 0, s>>>(p, g, r, v, st, first, kHeadSteps, mid, second);
+        k_propagate_tail<M><<<blocks, bs, 0, s>>>(p, g, r, v, st, second, mid, INT_MAX, none);
         count_launch(3);
     }
 }
@@ -436,17 +441,13 @@ kpax_status launch_propagate(const KParams& p, const Grid& g, const float* paren
                              uint32_t n, float* rows, uint8_t* valid, int32_t* steps, cudaStream_t stream)
 {
     if(!n) return KPAX_OK;
-    const uint32_t blocks = (n + 255) / 256;
+    auto go = [&](auto kernel, uint32_t bs) {
+        kernel<<<(n + bs - 1) / bs, bs, 0, stream>>>(p, g, parents, draws, stream_id, n, rows, valid, steps);
+    };
     switch(p.model) {
-        case KPAX_MODEL_DOUBLE_INTEGRATOR:
-            k_propagate_batch<KPAX_MODEL_DOUBLE_INTEGRATOR><<<blocks, 256, 0, stream>>>(p, g, parents, draws, stream_id, n, rows, valid, steps);
-            break;
-        case KPAX_MODEL_DUBINS_AIRPLANE:
-            k_propagate_batch<KPAX_MODEL_DUBINS_AIRPLANE><<<blocks, 256, 0, stream>>>(p, g, parents, draws, stream_id, n, rows, valid, steps);
-            break;
-        default:
-            k_propagate_batch<KPAX_MODEL_QUADROTOR><<<blocks, 256, 0, stream>>>(p, g, parents, draws, stream_id, n, rows, valid, steps);
-            break;
+        case KPAX_MODEL_DOUBLE_INTEGRATOR: go(k_propagate_batch<KPAX_MODEL_DOUBLE_INTEGRATOR>, kBatchBS<KPAX_MODEL_DOUBLE_INTEGRATOR>); break;
+        case KPAX_MODEL_DUBINS_AIRPLANE: go(k_propagate_batch<KPAX_MODEL_DUBINS_AIRPLANE>, kBatchBS<KPAX_MODEL_DUBINS_AIRPLANE>); break;
+        default: go(k_propagate_batch<KPAX_MODEL_QUADROTOR>, kBatchBS<KPAX_MODEL_QUADROTOR>); break;
     }
     KPAX_CHECK_LAUNCH();
     count_launch();

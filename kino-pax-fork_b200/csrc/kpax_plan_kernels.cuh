@@ -677,7 +677,7 @@ __device__ __forceinline__ bool expand_tiles(QueryDev& sq, const ExpandState st,
                 if(sq.mix) mlp::mixture_draws(p, sq.mix + (size_t)(c / k) * mlp::kMixFloats, sq.prop_eps, st.plan, st.iter, c, u);
             }
             steps = draw_controls(p, u, cc);
-            valid = propagate<M, K>(p, sq.g, s, cc, steps, steps_done, save + threadIdx.x, BS);
+            valid = propagate<M, K>(p, sq.g, s, cc, steps, steps_done, save + threadIdx.x * SD, BS);
             r1v = region_r1<SD>(p, s);
             r2v = region_r2<SD>(p, s, r1v);
             atomicAdd(rg.counter + r1v, 1);
@@ -794,7 +794,7 @@ template <int M, int BS>
 __global__ void __launch_bounds__(BS, (512 / BS > 0 ? 512 / BS : 1)) k_expand(const QueryDev* __restrict__ qs, const uint32_t* __restrict__ qidx,
                                                uint32_t* __restrict__ active)
 {
-    extern __shared__ float s_save[];
+    extern __shared__ __align__(16) float s_save[];
     __shared__ QueryDev sq;
     __shared__ ExpandSmem<BS / 32> sm;
     load_query(qs, qidx, sq);
@@ -990,7 +990,7 @@ __global__ void __launch_bounds__(BS, (512 / BS > 0 ? 512 / BS : 1)) k_iterate(c
                                                                              uint32_t max_inner)
 {
     constexpr int NW = BS / 32;
-    extern __shared__ float s_save[];  // not used by kIterFront
+    extern __shared__ __align__(16) float s_save[];  // not used by kIterFront
     __shared__ QueryDev sq;
     __shared__ ExpandSmem<NW> sm;
     __shared__ uint32_t s_warp[NW];

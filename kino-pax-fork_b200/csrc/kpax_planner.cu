@@ -339,14 +339,7 @@ struct PlanBatch {
         const uint32_t groups0 = ((uint32_t)prm[0].num_r1 + 31) / 32;
         gx_score = n == 1 ? std::min<uint32_t>(kScoreCTAs, std::max<uint32_t>(1, (groups0 + 7) / 8))
                           : std::max<uint32_t>(1, 1024 / n);
-        for(int m = 0; m < 3; ++m) {
-            if(groups[m].empty()) continue;
-            const void* fn = m == 0 ? expand_kernel<KPAX_MODEL_DOUBLE_INTEGRATOR>(expand_bs[m])
-                                    : m == 1 ? expand_kernel<KPAX_MODEL_DUBINS_AIRPLANE>(expand_bs[m])
-                                             : expand_kernel<KPAX_MODEL_QUADROTOR>(expand_bs[m]);
-            kpax_status st = allow_smem(fn, save_bytes(m + 1, expand_bs[m]));
-            if(st != KPAX_OK) return st;
-        }
+        if(const char* e = getenv("KPAX_BATCH_EXPAND")) expand_mode = atoi(e) == 0 ? 0 : atoi(e) == 2 ? 2 : 1;
         if(n == 1) {  // the fused iteration: as many CTAs as the expansion wants and can stay resident
             int dev = 0, sms = 148, per_sm = 0;
             KPAX_CUDA(cudaGetDevice(&dev));
@@ -407,7 +400,6 @@ struct PlanBatch {
                 if(!bs0) bs0 = expand_bs[m];
                 same_bs = same_bs && expand_bs[m] == bs0;
             }
-            if(const char* e = getenv("KPAX_BATCH_EXPAND")) expand_mode = atoi(e) == 0 ? 0 : atoi(e) == 2 ? 2 : 1;
             if(persistent && ngroups > 1 && same_bs) {
                 std::vector<uint32_t> order;
                 for(int m = 2; m >= 0; --m) order.insert(order.end(), groups[m].begin(), groups[m].end());
@@ -418,6 +410,18 @@ struct PlanBatch {
                 if((st = resident(expand_mixed_kernel(bs0), bs0, save_bytes(KPAX_MODEL_QUADROTOR, bs0) + 4 * ((size_t)n + 1), gx)) != KPAX_OK) return st;
                 if(gx) mixed_bs = bs0, gx_mixed = gx;
             }
+        }
+        // the per-query-grid expansion serves single plans by stages, and batches in that mode or without
+        // the persistent stages
+        const bool staged = n == 1 ? cfg[0].iteration_kernels != 0 || !gx_iter || (prm[0].model == KPAX_MODEL_QUADROTOR && !gx_split)
+                                   : !persistent || expand_mode == 0;
+        for(int m = 0; m < 3 && staged; ++m) {
+            if(groups[m].empty()) continue;
+            const void* fn = m == 0 ? expand_kernel<KPAX_MODEL_DOUBLE_INTEGRATOR>(expand_bs[m])
+                                    : m == 1 ? expand_kernel<KPAX_MODEL_DUBINS_AIRPLANE>(expand_bs[m])
+                                             : expand_kernel<KPAX_MODEL_QUADROTOR>(expand_bs[m]);
+            kpax_status st = allow_smem(fn, save_bytes(m + 1, expand_bs[m]));
+            if(st != KPAX_OK) return st;
         }
         update_fused();
         // control blocks, counters and arrival flags start at zero; no node is in a frontier

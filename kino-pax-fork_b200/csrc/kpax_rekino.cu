@@ -67,7 +67,7 @@ __global__ void __launch_bounds__(32) k_rekino(const RekinoDev d)
 {
     constexpr int SD = ModelDims<M>::SD, CD = ModelDims<M>::CD, S = SD + CD + 1;
     constexpr int kGroup = 5;  // steps per collision query (run_steps)
-    __shared__ float s_save[kGroup * SD * 32];
+    __shared__ __align__(16) float s_save[kGroup * SD * 32];
     extern __shared__ float s_cand[];  // [spt * 32][S] candidate rows, then [spt * 32] distances
     const KParams& p = d.p;
     const uint32_t w = blockIdx.x, lane = threadIdx.x, spt = d.spt, nsamp = 32u * spt;
@@ -100,7 +100,7 @@ __global__ void __launch_bounds__(32) k_rekino(const RekinoDev d)
 #pragma unroll
             for(int q = 0; q < SD; ++q) s[q] = cur[q];
             int done = 0;
-            const bool valid = propagate<M, kGroup>(p, d.g, s, cc, steps, done, s_save + lane, 32);
+            const bool valid = propagate<M, kGroup>(p, d.g, s, cc, steps, done, s_save + lane * SD, 32);
             row_controls<M>(cc, rc);
             float* row = s_cand + (size_t)j * S;
 #pragma unroll
