@@ -1,8 +1,8 @@
 // kpax_learn.cu — training and inference entry points of the learned proposal network.
 //
-// Training runs in FP32 on the SIMT cores with hand-written kernels: a tiled SGEMM for the six
-// products of the forward and backward passes, fused bias/SiLU and SiLU-gradient passes, the
-// mixture-density loss and its gradient, fixed-order column and loss reductions, and Adam.
+// Training runs in FP32 on the SIMT cores with hand-written kernels: one for a block of rows through the
+// forward pass, the mixture-density loss and the backward pass, one for the weight gradients of all
+// layers, and one for their fixed-order sums and Adam.
 // Every reduction has a fixed order, so a training step is deterministic.  Inference for the
 // planner runs on the tensor cores (kpax_mlp_tc.cuh) from a BF16 image packed here.
 // The reference planner has no learned component; the network replaces nothing in it and only
@@ -27,185 +27,374 @@ using namespace kpax::mlp;
 namespace {
 
 // ---------------------------------------------------------------------------------------------
-// SIMT kernels
+// FP32 training kernels.  A gradient is three launches:
+//   k_mlp_rows  a CTA takes R rows through the three layers, the loss and back to the first layer's
+//               pre-activation gradient, its activations in shared memory and the weights streamed
+//               through two 36 KB buffers; it leaves what the weight gradients need in global memory
+//   k_mlp_dw    dW = dZ^T A of all layers, 64 x 64 tiles, the rows split over up to kSplits partial sums
+//   k_mlp_grad  partial sums added in split order (and Adam)
+// Products accumulate in pairs of FP32 values (fma.rn.f32x2), each output in a fixed order.
+// B200, loss and gradient of 4096 rows: 1766 us with one 64 x 64-tile SGEMM per product (8-16 CTAs
+// summing all rows for a weight gradient, 645-695 us each) and one thread per column for the bias
+// gradients (230 us each); now 120 us: rows 75, weight gradients 34 (46 with 4 x 8 outputs per thread),
+// sums 5.5.  Both products are bound by shared memory's return bandwidth, 21-26 of 72.6 TFLOP/s.
+// Error of the gradient against 64 bits: 2.5e-6 before, 2.2e-6 now.
 
-constexpr int kGemmBS = 256, kGT = 64, kGK = 16;
+constexpr int kRowThreads = 256;
+constexpr int kChunkK = 32, kWStride = kChunkK + 4;  // weights chunk: [columns][32], rows 36 floats apart (conflict-free)
+constexpr int kActStride = kH + 4, kXStride = kInPad + 4, kOStride = kOutPad + 4;
+constexpr int kWBuf = kH * kWStride;
+// Transposed copies for the backward products: W3^T [kH][kOutPad], then W2^T [kH][kH].
+constexpr size_t kOffW3T = 0, kOffW2T = kOffW3T + kH * kOutPad, kNumT = kOffW2T + kH * kH;
+constexpr int kSplits = 16;
 
-// C[M x N] = op(A) op(B) (+ C when accumulate); op(A)[m][k] = TA ? A[k*lda+m] : A[m*lda+k],
-// op(B)[k][n] = TB ? B[n*ldb+k] : B[k*ldb+n].  64x64 tiles, 4x4 outputs per thread, each output
-// summed over k in ascending order by one thread.
-template <bool TA, bool TB>
-__global__ void __launch_bounds__(kGemmBS) k_sgemm(int M, int N, int K, const float* __restrict__ A, int lda,
-                                                   const float* __restrict__ B, int ldb, float* __restrict__ C, int ldc,
-                                                   int accumulate)
-{
-    __shared__ float As[kGK][kGT + 4], Bs[kGK][kGT + 4];
-    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-    const int m0 = blockIdx.y * kGT, n0 = blockIdx.x * kGT;
-    float acc[4][4] = {};
-    for(int k0 = 0; k0 < K; k0 += kGK) {
-        for(int i = threadIdx.x; i < kGT * kGK; i += kGemmBS) {
-            const int mm = TA ? i % kGT : i / kGK, kk = TA ? i / kGT : i % kGK;
-            const int gm = m0 + mm, gk = k0 + kk;
-            As[kk][mm] = (gm < M && gk < K) ? (TA ? A[(size_t)gk * lda + gm] : A[(size_t)gm * lda + gk]) : 0.0f;
-            const int nn = TB ? i / kGK : i % kGT, kb = TB ? i % kGK : i / kGT;
-            const int gn = n0 + nn, gkb = k0 + kb;
-            Bs[kb][nn] = (gn < N && gkb < K) ? (TB ? B[(size_t)gn * ldb + gkb] : B[(size_t)gkb * ldb + gn]) : 0.0f;
-        }
-        __syncthreads();
-#pragma unroll
-        for(int kk = 0; kk < kGK; ++kk) {
-            float a[4], b[4];
-#pragma unroll
-            for(int i = 0; i < 4; ++i) a[i] = As[kk][ty * 4 + i], b[i] = Bs[kk][tx * 4 + i];
-#pragma unroll
-            for(int i = 0; i < 4; ++i)
-#pragma unroll
-                for(int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-        }
-        __syncthreads();
-    }
-#pragma unroll
-    for(int i = 0; i < 4; ++i)
-#pragma unroll
-        for(int j = 0; j < 4; ++j) {
-            const int m = m0 + ty * 4 + i, n = n0 + tx * 4 + j;
-            if(m < M && n < N) {
-                float* c = C + (size_t)m * ldc + n;
-                *c = accumulate ? *c + acc[i][j] : acc[i][j];
-            }
-        }
-}
+template <int R>
+constexpr size_t kRowSmem = sizeof(float) * (R * (kXStride + 2 * kActStride + kOStride) + 2 * kWBuf);
+
+struct RowArgs {
+    const float* x;        // rows of kInPad features
+    const float* y;        // rows of kDim targets
+    const uint32_t* idx;   // row indices (null: 0, 1, ...)
+    uint32_t n;
+    const float* w;
+    const float* wt;
+    const float* mask;
+    float inv_n;
+    float *xb, *a1, *a2, *dz1, *dz2, *d_o, *ls;  // for the weight gradients
+    float* out;            // forward only: n x kOutPad
+};
 
 __device__ __forceinline__ float sigmoid_f(float z) { return 1.0f / (1.0f + expf(-z)); }
 
-// Z += b; A = SiLU(Z)  (rows x cols, row-major)
-__global__ void k_bias_silu(float* __restrict__ Z, const float* __restrict__ b, float* __restrict__ A, uint32_t rows, int cols)
+__device__ __forceinline__ void cp_async16(float* dst, const float* src, bool valid = true)
 {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if(i >= (size_t)rows * cols) return;
-    const float z = Z[i] + b[i % cols];
-    Z[i] = z;
-    A[i] = z * sigmoid_f(z);
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(valid ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
+
+// Weight chunks in the order the layers read them: W1 (2 chunks of 32 inputs), W2 (8), W3 (8), and back
+// W3^T (3), W2^T (8).
+constexpr int kChunksForward = 18, kChunksTrain = 29;
+__device__ __forceinline__ void load_chunk(const RowArgs& p, int id, float* buf)
+{
+    const float* src;
+    int K, cols = kH;
+    if(id < 2) src = p.w + kOffW1 + id * kChunkK, K = kInPad;
+    else if(id < 10) src = p.w + kOffW2 + (id - 2) * kChunkK, K = kH;
+    else if(id < 18) src = p.w + kOffW3 + (id - 10) * kChunkK, K = kH, cols = kOutPad;
+    else if(id < 21) src = p.wt + kOffW3T + (id - 18) * kChunkK, K = kOutPad;
+    else src = p.wt + kOffW2T + (id - 21) * kChunkK, K = kH;
+    for(int i = threadIdx.x; i < cols * (kChunkK / 4); i += kRowThreads) {
+        const int c = i >> 3, q = i & 7;
+        cp_async16(buf + c * kWStride + 4 * q, src + (size_t)c * K + 4 * q);
+    }
+    cp_commit();
 }
 
-__global__ void k_bias(float* __restrict__ Z, const float* __restrict__ b, uint32_t rows, int cols)
+// acc[i][j] += sum over `chunks` chunks of A[row i][k] W[col + 32 j][k], even and odd k in the halves of
+// acc.  a: the thread's first row (stride lda); chunk id + 1 is loaded while chunk id is used.  Shared
+// memory returns 128 bytes per clock whether or not the lanes' addresses agree, so a 16-byte vector of
+// k costs 4 (RT + CT) clocks per warp against RT CT for its FMAs on the SM.  256 x 256 layer of 32 rows,
+// whole kernel: 8 x 4 outputs per thread and eight warps 75 us; 8 x 2 and sixteen warps 85 us; 8 x 8 and
+// four warps (the balanced tile, but one warp per scheduler) 91 us.
+template <int RT, int CT>
+__device__ __forceinline__ void mac_chunks(const RowArgs& p, const float* a, int lda, int col, int first, int chunks, int total,
+                                           float* wbuf, F2 (&acc)[RT][CT])
 {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if(i < (size_t)rows * cols) Z[i] += b[i % cols];
+    for(int c = 0; c < chunks; ++c) {
+        const int id = first + c;
+        cp_wait();
+        __syncthreads();  // chunk id is there, and the other buffer is no longer read
+        if(id + 1 < total) load_chunk(p, id + 1, wbuf + ((id + 1) & 1) * kWBuf);
+        const float* w = wbuf + (id & 1) * kWBuf + col * kWStride;
+        const float* ac = a + c * kChunkK;
+#pragma unroll 2  // 150 instructions: a chunk unrolled as a whole stalls on instruction fetches (80 us)
+        for(int q = 0; q < kChunkK / 4; ++q) {
+            ulonglong2 wv[CT];
+#pragma unroll
+            for(int j = 0; j < CT; ++j) wv[j] = *reinterpret_cast<const ulonglong2*>(w + 32 * j * kWStride + 4 * q);
+#pragma unroll
+            for(int i = 0; i < RT; ++i) {
+                const ulonglong2 av = *reinterpret_cast<const ulonglong2*>(ac + i * lda + 4 * q);
+#pragma unroll
+                for(int j = 0; j < CT; ++j) acc[i][j] = fma2(av.y, wv[j].y, fma2(av.x, wv[j].x, acc[i][j]));
+            }
+        }
+    }
 }
 
-// dZ = dA * SiLU'(Z), SiLU'(z) = sig(z) (1 + z (1 - sig(z)))
-__global__ void k_silu_grad(const float* __restrict__ dA, const float* __restrict__ Z, float* __restrict__ dZ, size_t n)
+__device__ __forceinline__ float halves(F2 v)
 {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if(i >= n) return;
-    const float z = Z[i], s = sigmoid_f(z);
-    dZ[i] = dA[i] * (s * (1.0f + z * (1.0f - s)));
+    const float2 f = unpack(v);
+    return f.x + f.y;
 }
 
 // Mixture-density negative log-likelihood of the logit targets y (masked dimensions only) and its
-// gradient with respect to the 96 outputs, scaled by inv_n.  One thread per sample.
-__global__ void k_mdn(const float* __restrict__ O, const float* __restrict__ Y, const float* __restrict__ mask, uint32_t n,
-                      float inv_n, float* __restrict__ dO, float* __restrict__ loss)
+// gradient with respect to the outputs, scaled by inv_n, in place: eight lanes per sample, one component
+// each (o: the sample's kOutPad outputs; lane k its component's 11).  Returns the loss.
+__device__ __forceinline__ float mdn(float* o, const float* y, const float* mask, float inv_n, int k)
 {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if(i >= n) return;
-    const float* o = O + (size_t)i * kOutPad;
-    float y[kDim], m[kDim];
-#pragma unroll
-    for(int d = 0; d < kDim; ++d) y[d] = Y[(size_t)i * kDim + d], m[d] = mask[d];
     constexpr float kHalfLog2Pi = 0.918938533204672742f;
-    float amax = o[0];
+    auto max8 = [](float v) {
 #pragma unroll
-    for(int k = 1; k < kComp; ++k) amax = fmaxf(amax, o[k * kCompStride]);
-    float asum = 0.0f;
+        for(int d = 4; d > 0; d >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, d));
+        return v;
+    };
+    auto sum8 = [](float v) {
 #pragma unroll
-    for(int k = 0; k < kComp; ++k) asum += expf(o[k * kCompStride] - amax);
-    const float alse = amax + logf(asum);
-    float lp[kComp];
+        for(int d = 4; d > 0; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
+        return v;
+    };
+    float* c = o + k * kCompStride;
+    const float logit = c[0], amax = max8(logit);
+    const float alse = amax + logf(sum8(expf(logit - amax)));
+    float th[kDim], e[kDim], is[kDim], m[kDim], lp = logit - alse;
 #pragma unroll
-    for(int k = 0; k < kComp; ++k) {
-        float acc = o[k * kCompStride] - alse;
-#pragma unroll
-        for(int d = 0; d < kDim; ++d) {
-            const float th = tanhf(o[k * kCompStride + 1 + kDim + d] * (1.0f / kSigHalf));
-            const float s = kSigMid + kSigHalf * th, r = (y[d] - o[k * kCompStride + 1 + d]) * expf(-s);
-            acc += m[d] * (-0.5f * r * r - s - kHalfLog2Pi);
-        }
-        lp[k] = acc;
+    for(int d = 0; d < kDim; ++d) {
+        m[d] = mask[d];
+        th[d] = tanhf(c[1 + kDim + d] * (1.0f / kSigHalf));
+        const float s = kSigMid + kSigHalf * th[d];
+        is[d] = expf(-s);
+        e[d] = (y[d] - c[1 + d]) * is[d];
+        lp += m[d] * (-0.5f * e[d] * e[d] - s - kHalfLog2Pi);
     }
-    float lmax = lp[0];
+    const float lmax = max8(lp), lse = lmax + logf(sum8(expf(lp - lmax)));
+    const float r = expf(lp - lse), pi = expf(logit - alse);
+    c[0] = (pi - r) * inv_n;
 #pragma unroll
-    for(int k = 1; k < kComp; ++k) lmax = fmaxf(lmax, lp[k]);
-    float lsum = 0.0f;
-#pragma unroll
-    for(int k = 0; k < kComp; ++k) lsum += expf(lp[k] - lmax);
-    const float lse = lmax + logf(lsum);
-    loss[i] = -lse;
-    float* g = dO + (size_t)i * kOutPad;
-#pragma unroll
-    for(int k = 0; k < kComp; ++k) {
-        const float r = expf(lp[k] - lse), pi = expf(o[k * kCompStride] - alse);
-        g[k * kCompStride] = (pi - r) * inv_n;
-#pragma unroll
-        for(int d = 0; d < kDim; ++d) {
-            const float th = tanhf(o[k * kCompStride + 1 + kDim + d] * (1.0f / kSigHalf));
-            const float s = kSigMid + kSigHalf * th, is = expf(-s);
-            const float e = (y[d] - o[k * kCompStride + 1 + d]) * is;
-            g[k * kCompStride + 1 + d] = -r * m[d] * e * is * inv_n;
-            g[k * kCompStride + 1 + kDim + d] = -r * m[d] * (e * e - 1.0f) * (1.0f - th * th) * inv_n;
-        }
+    for(int d = 0; d < kDim; ++d) {
+        c[1 + d] = -r * m[d] * e[d] * is[d] * inv_n;
+        c[1 + kDim + d] = -r * m[d] * (e[d] * e[d] - 1.0f) * (1.0f - th[d] * th[d]) * inv_n;
     }
-#pragma unroll
-    for(int j = kOut; j < kOutPad; ++j) g[j] = 0.0f;
+    o[kOut + k] = 0.0f;  // padding outputs
+    return -lse;
 }
 
-// db[c] = sum over rows of dZ[r][c], rows in ascending order (one thread per column).
-__global__ void k_colsum(const float* __restrict__ dZ, uint32_t rows, int cols, float* __restrict__ db)
+// R rows (32, or 16 where 32 would leave SMs without a CTA).  Warp w holds rows (w & 3) * R / 4 ... of the
+// 256-column products and columns (w >> 2) * 128 + lane + 32 j: weights are read a 16-byte vector of k per
+// column, activations as broadcasts.
+template <int R, bool kTrain>
+__global__ void __launch_bounds__(kRowThreads, 1) k_mlp_rows(const RowArgs p)
 {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if(c >= cols) return;
-    float acc = 0.0f;
-    for(uint32_t r = 0; r < rows; ++r) acc += dZ[(size_t)r * cols + c];
-    db[c] = acc;
-}
-
-// Sum of n values: 1024 strided partial sums, then a fixed halving tree (one block).
-__global__ void __launch_bounds__(1024) k_sum(const float* __restrict__ v, uint32_t n, float* __restrict__ out)
-{
-    __shared__ float s[1024];
-    float acc = 0.0f;
-    for(uint32_t i = threadIdx.x; i < n; i += 1024) acc += v[i];
-    s[threadIdx.x] = acc;
-    __syncthreads();
-    for(int h = 512; h > 0; h >>= 1) {
-        if((int)threadIdx.x < h) s[threadIdx.x] += s[threadIdx.x + h];
+    static_assert(kOutPad - kOut == kComp, "one padding output per lane of a sample");
+    constexpr int RT = R / 4, RO = R / 8, kTotal = kTrain ? kChunksTrain : kChunksForward;
+    extern __shared__ __align__(16) float smem_f[];
+    float* sX = smem_f;
+    float* sA1 = sX + R * kXStride;
+    float* sA2 = sA1 + R * kActStride;
+    float* sO = sA2 + R * kActStride;
+    float* wbuf = sO + R * kOStride;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t row0 = blockIdx.x * R;
+    const int rows = (int)min((uint32_t)R, p.n - row0);
+    load_chunk(p, 0, wbuf);
+    for(int i = tid; i < R * kInPad; i += kRowThreads) {
+        const int r = i / kInPad, c = i % kInPad;
+        float v = 0.0f;
+        if(r < rows) {
+            v = p.x[(size_t)(p.idx ? p.idx[row0 + r] : row0 + r) * kInPad + c];
+            if constexpr(kTrain) p.xb[(size_t)(row0 + r) * kInPad + c] = v;
+        }
+        sX[r * kXStride + c] = v;
+    }
+    const int r0 = (warp & 3) * RT, col = (warp >> 2) * 128 + lane;
+    float g1[RT][4], g2[RT][4];  // SiLU' of both hidden layers (training)
+    auto hidden = [&](F2 (&acc)[RT][4], const float* bias, float* s_act, float* d_act, float (&g)[RT][4]) {
+#pragma unroll
+        for(int j = 0; j < 4; ++j) {
+            const float b = __ldg(bias + col + 32 * j);
+#pragma unroll
+            for(int i = 0; i < RT; ++i) {
+                const float z = halves(acc[i][j]) + b, sg = sigmoid_f(z), a = z * sg;
+                s_act[(r0 + i) * kActStride + col + 32 * j] = a;
+                if constexpr(kTrain) {
+                    g[i][j] = sg * (1.0f + z * (1.0f - sg));
+                    if(r0 + i < rows) d_act[(size_t)(row0 + r0 + i) * kH + col + 32 * j] = a;
+                }
+                acc[i][j] = 0ull;
+            }
+        }
+    };
+    F2 acc[RT][4] = {};
+    mac_chunks(p, sX + r0 * kXStride, kXStride, col, 0, 2, kTotal, wbuf, acc);
+    hidden(acc, p.w + kOffB1, sA1, p.a1, g1);
+    mac_chunks(p, sA1 + r0 * kActStride, kActStride, col, 2, 8, kTotal, wbuf, acc);
+    hidden(acc, p.w + kOffB2, sA2, p.a2, g2);
+    {
+        F2 ao[RO][3] = {};
+        mac_chunks(p, sA2 + warp * RO * kActStride, kActStride, lane, 10, 8, kTotal, wbuf, ao);
+#pragma unroll
+        for(int j = 0; j < 3; ++j) {
+            const float b = __ldg(p.w + kOffB3 + lane + 32 * j);
+#pragma unroll
+            for(int i = 0; i < RO; ++i) {
+                const float v = halves(ao[i][j]) + b;
+                const int r = warp * RO + i;
+                if constexpr(kTrain) sO[r * kOStride + lane + 32 * j] = v;
+                else if(r < rows) p.out[(size_t)(row0 + r) * kOutPad + lane + 32 * j] = v;
+            }
+        }
+    }
+    if constexpr(kTrain) {
         __syncthreads();
+        if(tid < 8 * R) {
+            const int r = tid >> 3, k = tid & 7;
+            const size_t src = r < rows ? (p.idx ? p.idx[row0 + r] : row0 + r) : 0;
+            float y[kDim];
+#pragma unroll
+            for(int d = 0; d < kDim; ++d) y[d] = r < rows ? p.y[src * kDim + d] : 0.0f;
+            const float loss = mdn(sO + r * kOStride, y, p.mask, r < rows ? p.inv_n : 0.0f, k);
+            if(k == 0 && r < rows) p.ls[row0 + r] = loss;
+        }
+        __syncthreads();
+        for(int i = tid; i < rows * kOutPad; i += kRowThreads)
+            p.d_o[(size_t)row0 * kOutPad + i] = sO[(i / kOutPad) * kOStride + i % kOutPad];
+        mac_chunks(p, sO + r0 * kOStride, kOStride, col, 18, 3, kTotal, wbuf, acc);
+        // dZ2 takes A2's place (every warp is past the products that read A2)
+#pragma unroll
+        for(int j = 0; j < 4; ++j)
+#pragma unroll
+            for(int i = 0; i < RT; ++i) {
+                const float d = halves(acc[i][j]) * g2[i][j];
+                sA2[(r0 + i) * kActStride + col + 32 * j] = d;
+                if(r0 + i < rows) p.dz2[(size_t)(row0 + r0 + i) * kH + col + 32 * j] = d;
+                acc[i][j] = 0ull;
+            }
+        mac_chunks(p, sA2 + r0 * kActStride, kActStride, col, 21, 8, kTotal, wbuf, acc);
+#pragma unroll
+        for(int j = 0; j < 4; ++j)
+#pragma unroll
+            for(int i = 0; i < RT; ++i)
+                if(r0 + i < rows) p.dz1[(size_t)(row0 + r0 + i) * kH + col + 32 * j] = halves(acc[i][j]) * g1[i][j];
     }
-    if(threadIdx.x == 0) *out = s[0];
 }
 
-// Adam with bias corrections folded into c1 = lr / (1 - b1^t) and c2 = 1 / (1 - b2^t).
-__global__ void k_adam(float* __restrict__ w, const float* __restrict__ g, float* __restrict__ m, float* __restrict__ v, size_t n,
-                       float b1, float b2, float c1, float c2, float eps)
+// Tile blockIdx.x (layer 3: 2 x 4 tiles, layer 2: 4 x 4, layer 1: 4 x 1) of the weight gradients
+// over the rows of split blockIdx.y: part[split][parameter].  Thread (tm, tj) holds the 8 x 8 outputs of
+// rows 4 tm .., 32 + 4 tm .. and columns 4 tj .., 32 + 4 tj .. (conflict-free 16-byte loads).
+constexpr int kDwThreads = 64, kDwRows = 32, kDwTiles = 8 + 16 + 4;
+__global__ void __launch_bounds__(kDwThreads) k_mlp_dw(const float* __restrict__ d_o, const float* __restrict__ dz2,
+                                                       const float* __restrict__ dz1, const float* __restrict__ a2,
+                                                       const float* __restrict__ a1, const float* __restrict__ xb, uint32_t n,
+                                                       uint32_t rows_per_split, float* __restrict__ part)
+{
+    __shared__ __align__(16) float sP[2][kDwRows * 64], sQ[2][kDwRows * 64];
+    const int tid = threadIdx.x, tm = tid >> 3, tj = tid & 7;
+    const int tile = blockIdx.x;
+    const float *P, *Q;
+    int ldp, ldq, mt, jt, M;
+    size_t off_w, off_b;
+    if(tile < 8) P = d_o, Q = a2, ldp = M = kOutPad, ldq = kH, mt = tile >> 2, jt = tile & 3, off_w = kOffW3, off_b = kOffB3;
+    else if(tile < 24) P = dz2, Q = a1, ldp = M = kH, ldq = kH, mt = (tile - 8) >> 2, jt = tile & 3, off_w = kOffW2, off_b = kOffB2;
+    else P = dz1, Q = xb, ldp = M = kH, ldq = kInPad, mt = tile - 24, jt = 0, off_w = kOffW1, off_b = kOffB1;
+    const uint32_t lo = min(n, blockIdx.y * rows_per_split), hi = min(n, lo + rows_per_split);
+    auto load = [&](uint32_t r, int b) {  // rows r .. r + 31 (zero past the split's end and past column M)
+        for(int i = tid; i < kDwRows * 16; i += kDwThreads) {
+            const uint32_t row = r + (i >> 4);
+            const int q = 4 * (i & 15);
+            const bool in = row < hi, inp = in && 64 * mt + q < M;
+            cp_async16(&sP[b][(i >> 4) * 64 + q], P + (inp ? (size_t)row * ldp + 64 * mt + q : 0), inp);
+            cp_async16(&sQ[b][(i >> 4) * 64 + q], Q + (in ? (size_t)row * ldq + 64 * jt + q : 0), in);
+        }
+        cp_commit();
+    };
+    F2 acc[8][4] = {};
+    float bsum[8] = {};
+    const bool bias = jt == 0 && tj == 0;
+    if(lo < hi) load(lo, 0);
+    int b = 0;
+    for(uint32_t r = lo; r < hi; r += kDwRows, b ^= 1) {
+        cp_wait();
+        __syncthreads();
+        if(r + kDwRows < hi) load(r + kDwRows, b ^ 1);
+#pragma unroll 2
+        for(int k = 0; k < kDwRows; ++k) {
+            const float4 p0 = *reinterpret_cast<const float4*>(&sP[b][k * 64 + 4 * tm]);
+            const float4 p1 = *reinterpret_cast<const float4*>(&sP[b][k * 64 + 32 + 4 * tm]);
+            const ulonglong2 q0 = *reinterpret_cast<const ulonglong2*>(&sQ[b][k * 64 + 4 * tj]);
+            const ulonglong2 q1 = *reinterpret_cast<const ulonglong2*>(&sQ[b][k * 64 + 32 + 4 * tj]);
+            const float pa[8] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
+#pragma unroll
+            for(int i = 0; i < 8; ++i) {
+                const F2 d = f2(pa[i]);
+                acc[i][0] = fma2(d, q0.x, acc[i][0]), acc[i][1] = fma2(d, q0.y, acc[i][1]);
+                acc[i][2] = fma2(d, q1.x, acc[i][2]), acc[i][3] = fma2(d, q1.y, acc[i][3]);
+            }
+            if(bias) {
+#pragma unroll
+                for(int i = 0; i < 8; ++i) bsum[i] += pa[i];
+            }
+        }
+    }
+    float* out = part + (size_t)blockIdx.y * kNumParams;
+#pragma unroll
+    for(int i = 0; i < 8; ++i) {
+        const int m = 64 * mt + 32 * (i >> 2) + 4 * tm + (i & 3);
+        if(m >= M) continue;
+        float* w = out + off_w + (size_t)m * ldq + 64 * jt + 4 * tj;
+        *reinterpret_cast<ulonglong2*>(w) = make_ulonglong2(acc[i][0], acc[i][1]);
+        *reinterpret_cast<ulonglong2*>(w + 32) = make_ulonglong2(acc[i][2], acc[i][3]);
+        if(bias) out[off_b + m] = bsum[i];
+    }
+}
+
+struct AdamArgs {
+    float *w, *wt, *m, *v;
+    float b1, b2, c1, c2, eps;  // bias corrections folded into c1 = lr / (1 - b1^t) and c2 = 1 / (1 - b2^t)
+};
+
+// Index of parameter i in the transposed copies, or kNumT.
+__device__ __forceinline__ size_t transposed(size_t i)
+{
+    if(i >= kOffW2 && i < kOffB2) return kOffW2T + ((i - kOffW2) % kH) * kH + (i - kOffW2) / kH;
+    if(i >= kOffW3 && i < kOffB3) return kOffW3T + ((i - kOffW3) % kH) * kOutPad + (i - kOffW3) / kH;
+    return kNumT;
+}
+
+// g = the splits' partial sums in split order; with kAdam also the optimiser's step.  The last block
+// adds the rows' losses (strided partial sums, then a fixed halving tree).
+template <bool kAdam>
+__global__ void __launch_bounds__(256) k_mlp_grad(const float* __restrict__ part, int splits, float* __restrict__ g,
+                                                  const float* __restrict__ ls, uint32_t n, float* __restrict__ loss,
+                                                  const AdamArgs o)
+{
+    if(blockIdx.x == gridDim.x - 1) {
+        __shared__ float s[256];
+        float acc = 0.0f;
+        for(uint32_t i = threadIdx.x; i < n; i += 256) acc += ls[i];
+        s[threadIdx.x] = acc;
+        __syncthreads();
+        for(int h = 128; h > 0; h >>= 1) {
+            if((int)threadIdx.x < h) s[threadIdx.x] += s[threadIdx.x + h];
+            __syncthreads();
+        }
+        if(threadIdx.x == 0) *loss = s[0];
+        return;
+    }
+    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if(i >= kNumParams) return;
+    float gi = 0.0f;
+#pragma unroll 8
+    for(int s = 0; s < splits; ++s) gi += part[(size_t)s * kNumParams + i];
+    g[i] = gi;
+    if constexpr(kAdam) {
+        const float mi = o.b1 * o.m[i] + (1.0f - o.b1) * gi, vi = o.b2 * o.v[i] + (1.0f - o.b2) * gi * gi;
+        o.m[i] = mi, o.v[i] = vi;
+        const float w = o.w[i] - o.c1 * mi / (sqrtf(vi * o.c2) + o.eps);
+        o.w[i] = w;
+        const size_t t = transposed(i);
+        if(t < kNumT) o.wt[t] = w;
+    }
+}
+
+__global__ void k_transpose(const float* __restrict__ w, float* __restrict__ wt)
 {
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if(i >= n) return;
-    const float gi = g[i];
-    const float mi = b1 * m[i] + (1.0f - b1) * gi, vi = b2 * v[i] + (1.0f - b2) * gi * gi;
-    m[i] = mi, v[i] = vi;
-    w[i] -= c1 * mi / (sqrtf(vi * c2) + eps);
-}
-
-__global__ void k_gather(const float* __restrict__ X, const float* __restrict__ Y, const uint32_t* __restrict__ idx, uint32_t n,
-                         float* __restrict__ Xb, float* __restrict__ Yb)
-{
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if(i >= n * (kInPad + kDim)) return;
-    const uint32_t r = i / (kInPad + kDim), c = i % (kInPad + kDim), src = idx[r];
-    if(c < (uint32_t)kInPad) Xb[(size_t)r * kInPad + c] = X[(size_t)src * kInPad + c];
-    else Yb[(size_t)r * kDim + c - kInPad] = Y[(size_t)src * kDim + c - kInPad];
+    if(i >= kNumParams) return;
+    const size_t t = transposed(i);
+    if(t < kNumT) wt[t] = w[i];
 }
 
 // FP32 master -> BF16 image in the MMA's shared-memory layout, plus the FP32 biases.
@@ -335,9 +524,10 @@ struct kpax_mlp {
     float* mask = nullptr;  // 5 loss-dimension weights
     float* loss = nullptr;  // scalar
     float* h_loss = nullptr;  // pinned scalar
-    // activations of a batch
-    float *xb = nullptr, *yb = nullptr, *z1 = nullptr, *a1 = nullptr, *z2 = nullptr, *a2 = nullptr, *o = nullptr;
-    float *d_o = nullptr, *d_a = nullptr, *d_z = nullptr, *ls = nullptr;
+    float* wt = nullptr;    // transposed copies of W3 and W2
+    // a batch's gathered rows, activations, gradients and losses, and the splits' partial gradients
+    float *xb = nullptr, *a1 = nullptr, *a2 = nullptr, *dz1 = nullptr, *dz2 = nullptr, *d_o = nullptr, *ls = nullptr, *part = nullptr;
+    int sms = 148;
     uint64_t step = 0;
     bool packed = false;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;  // around the last tensor-core pass
@@ -346,42 +536,40 @@ struct kpax_mlp {
 
 namespace kpax {
 
-// Forward pass of a batch already in (x, n) into the activation buffers.
-static kpax_status mlp_forward_f32(kpax_mlp* n, const float* x, uint32_t rows, cudaStream_t st)
+// Splits of the weight gradients' rows: enough 64 x 64 tiles for three CTAs per SM, at least two chunks
+// of rows each (partial sums cost a write and a read of every parameter).
+static int grad_splits(uint32_t rows) { return (int)std::min<uint32_t>(kSplits, std::max<uint32_t>(1, rows / (2 * kDwRows))); }
+
+template <bool kTrain>
+static kpax_status launch_rows(const kpax_mlp* n, const RowArgs& a, cudaStream_t st)
 {
-    const dim3 g1(blocks(kH, kGT), blocks(rows, kGT)), g3(blocks(kOutPad, kGT), blocks(rows, kGT));
-    k_sgemm<false, true><<<g1, kGemmBS, 0, st>>>(rows, kH, kInPad, x, kInPad, n->w + kOffW1, kInPad, n->z1, kH, 0);
-    k_bias_silu<<<blocks((size_t)rows * kH, 256), 256, 0, st>>>(n->z1, n->w + kOffB1, n->a1, rows, kH);
-    k_sgemm<false, true><<<g1, kGemmBS, 0, st>>>(rows, kH, kH, n->a1, kH, n->w + kOffW2, kH, n->z2, kH, 0);
-    k_bias_silu<<<blocks((size_t)rows * kH, 256), 256, 0, st>>>(n->z2, n->w + kOffB2, n->a2, rows, kH);
-    k_sgemm<false, true><<<g3, kGemmBS, 0, st>>>(rows, kOutPad, kH, n->a2, kH, n->w + kOffW3, kH, n->o, kOutPad, 0);
-    k_bias<<<blocks((size_t)rows * kOutPad, 256), 256, 0, st>>>(n->o, n->w + kOffB3, rows, kOutPad);
-    count_launch(6);
+    // 16 rows per CTA while that gives no SM a second one: less work per CTA, the same weights to stream
+    const bool small = a.n <= 16u * (uint32_t)n->sms;
+    const void* fn = small ? (const void*)k_mlp_rows<16, kTrain> : (const void*)k_mlp_rows<32, kTrain>;
+    const size_t smem = small ? kRowSmem<16> : kRowSmem<32>;
+    KPAX_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if(small) k_mlp_rows<16, kTrain><<<blocks(a.n, 16), kRowThreads, smem, st>>>(a);
+    else k_mlp_rows<32, kTrain><<<blocks(a.n, 32), kRowThreads, smem, st>>>(a);
+    count_launch();
     KPAX_CHECK_LAUNCH();
     return KPAX_OK;
 }
 
-// Loss and gradients (into n->g) of the batch (x, y); the loss sum lands in n->loss.
-static kpax_status mlp_backward_f32(kpax_mlp* n, const float* x, const float* y, uint32_t rows, cudaStream_t st)
+// Loss sum (into n->loss) and gradient (into g) of the rows idx (null: all) of (x, y); with adam the
+// optimiser's step as well.
+static kpax_status mlp_gradient(kpax_mlp* n, const float* x, const float* y, const uint32_t* idx, uint32_t rows, float* g,
+                                const AdamArgs* adam, cudaStream_t st)
 {
-    k_mdn<<<blocks(rows, 128), 128, 0, st>>>(n->o, y, n->mask, rows, 1.0f / (float)rows, n->d_o, n->ls);
-    k_sum<<<1, 1024, 0, st>>>(n->ls, rows, n->loss);
-    const dim3 gw3(blocks(kH, kGT), blocks(kOutPad, kGT)), gw2(blocks(kH, kGT), blocks(kH, kGT)), gw1(blocks(kInPad, kGT), blocks(kH, kGT));
-    const dim3 ga(blocks(kH, kGT), blocks(rows, kGT));
-    // layer 3: dW3 = dO^T A2, db3 = colsum(dO), dA2 = dO W3
-    k_sgemm<true, false><<<gw3, kGemmBS, 0, st>>>(kOutPad, kH, rows, n->d_o, kOutPad, n->a2, kH, n->g + kOffW3, kH, 0);
-    k_colsum<<<1, 128, 0, st>>>(n->d_o, rows, kOutPad, n->g + kOffB3);
-    k_sgemm<false, false><<<ga, kGemmBS, 0, st>>>(rows, kH, kOutPad, n->d_o, kOutPad, n->w + kOffW3, kH, n->d_a, kH, 0);
-    k_silu_grad<<<blocks((size_t)rows * kH, 256), 256, 0, st>>>(n->d_a, n->z2, n->d_z, (size_t)rows * kH);
-    // layer 2
-    k_sgemm<true, false><<<gw2, kGemmBS, 0, st>>>(kH, kH, rows, n->d_z, kH, n->a1, kH, n->g + kOffW2, kH, 0);
-    k_colsum<<<blocks(kH, 128), 128, 0, st>>>(n->d_z, rows, kH, n->g + kOffB2);
-    k_sgemm<false, false><<<ga, kGemmBS, 0, st>>>(rows, kH, kH, n->d_z, kH, n->w + kOffW2, kH, n->d_a, kH, 0);
-    k_silu_grad<<<blocks((size_t)rows * kH, 256), 256, 0, st>>>(n->d_a, n->z1, n->d_z, (size_t)rows * kH);
-    // layer 1
-    k_sgemm<true, false><<<gw1, kGemmBS, 0, st>>>(kH, kInPad, rows, n->d_z, kH, x, kInPad, n->g + kOffW1, kInPad, 0);
-    k_colsum<<<blocks(kH, 128), 128, 0, st>>>(n->d_z, rows, kH, n->g + kOffB1);
-    count_launch(12);
+    RowArgs a{x, y, idx, rows, n->w, n->wt, n->mask, 1.0f / (float)rows, n->xb, n->a1, n->a2, n->dz1, n->dz2, n->d_o, n->ls, nullptr};
+    kpax_status s = launch_rows<true>(n, a, st);
+    if(s != KPAX_OK) return s;
+    const int splits = grad_splits(rows);
+    const uint32_t per = (rows + (uint32_t)splits - 1) / (uint32_t)splits;
+    k_mlp_dw<<<dim3(kDwTiles, splits), kDwThreads, 0, st>>>(n->d_o, n->dz2, n->dz1, n->a2, n->a1, n->xb, rows, per, n->part);
+    const uint32_t grid = blocks(kNumParams, 256) + 1;
+    if(adam) k_mlp_grad<true><<<grid, 256, 0, st>>>(n->part, splits, g, n->ls, rows, n->loss, *adam);
+    else k_mlp_grad<false><<<grid, 256, 0, st>>>(n->part, splits, g, n->ls, rows, n->loss, AdamArgs{});
+    count_launch(2);
     KPAX_CHECK_LAUNCH();
     return KPAX_OK;
 }
@@ -445,22 +633,23 @@ kpax_status kpax_mlp_create(uint32_t max_batch, kpax_mlp** out)
     KPAX_MLP_ALLOC(n->err, 4);
     KPAX_MLP_ALLOC(n->mask, kDim * 4);
     KPAX_MLP_ALLOC(n->loss, 4);
+    KPAX_MLP_ALLOC(n->wt, kNumT * 4);
     KPAX_MLP_ALLOC(n->xb, B * kInPad * 4);
-    KPAX_MLP_ALLOC(n->yb, B * kDim * 4);
-    KPAX_MLP_ALLOC(n->z1, B * kH * 4);
     KPAX_MLP_ALLOC(n->a1, B * kH * 4);
-    KPAX_MLP_ALLOC(n->z2, B * kH * 4);
     KPAX_MLP_ALLOC(n->a2, B * kH * 4);
-    KPAX_MLP_ALLOC(n->o, B * kOutPad * 4);
+    KPAX_MLP_ALLOC(n->dz1, B * kH * 4);
+    KPAX_MLP_ALLOC(n->dz2, B * kH * 4);
     KPAX_MLP_ALLOC(n->d_o, B * kOutPad * 4);
-    KPAX_MLP_ALLOC(n->d_a, B * kH * 4);
-    KPAX_MLP_ALLOC(n->d_z, B * kH * 4);
     KPAX_MLP_ALLOC(n->ls, B * 4);
+    KPAX_MLP_ALLOC(n->part, P * 4 * (size_t)grad_splits(max_batch));
 #undef KPAX_MLP_ALLOC
     if(cudaMallocHost(&n->h_loss, 4) != cudaSuccess) return set_error("kpax_mlp_create: pinned alloc"), fail(KPAX_ENOMEM);
     if(cudaEventCreate(&n->ev0) != cudaSuccess || cudaEventCreate(&n->ev1) != cudaSuccess)
         return set_error("kpax_mlp_create: event creation failed"), fail(KPAX_ECUDA);
-    if(cudaMemset(n->w, 0, P * 4) != cudaSuccess || cudaMemset(n->m, 0, P * 4) != cudaSuccess ||
+    int dev = 0;
+    if(cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n->sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        return set_error("kpax_mlp_create: no device"), fail(KPAX_ECUDA);
+    if(cudaMemset(n->w, 0, P * 4) != cudaSuccess || cudaMemset(n->wt, 0, kNumT * 4) != cudaSuccess || cudaMemset(n->m, 0, P * 4) != cudaSuccess ||
        cudaMemset(n->v, 0, P * 4) != cudaSuccess || cudaMemset(n->err, 0, 4) != cudaSuccess ||
        cudaMemset(n->img, 0, kImgBytes) != cudaSuccess)
         return set_error("kpax_mlp_create: memset failed"), fail(KPAX_ECUDA);
@@ -474,7 +663,7 @@ kpax_status kpax_mlp_create(uint32_t max_batch, kpax_mlp** out)
 kpax_status kpax_mlp_destroy(kpax_mlp* n)
 {
     if(!n) return KPAX_OK;
-    void* dev[] = {n->w, n->g, n->m, n->v, n->img, n->err, n->mask, n->loss, n->xb, n->yb, n->z1, n->a1, n->z2, n->a2, n->o, n->d_o, n->d_a, n->d_z, n->ls};
+    void* dev[] = {n->w, n->g, n->m, n->v, n->img, n->err, n->mask, n->loss, n->wt, n->xb, n->a1, n->a2, n->dz1, n->dz2, n->d_o, n->ls, n->part};
     for(void* p : dev)
         if(p) cudaFree(p);
     if(n->h_loss) cudaFreeHost(n->h_loss);
@@ -495,6 +684,9 @@ kpax_status kpax_mlp_set_params(kpax_mlp* n, const float* h_params, void* stream
     KPAX_CUDA(cudaMemcpyAsync(n->w, h_params, kNumParams * 4, cudaMemcpyHostToDevice, st));
     KPAX_CUDA(cudaMemsetAsync(n->m, 0, kNumParams * 4, st));
     KPAX_CUDA(cudaMemsetAsync(n->v, 0, kNumParams * 4, st));
+    k_transpose<<<blocks(kNumParams, 256), 256, 0, st>>>(n->w, n->wt);
+    count_launch();
+    KPAX_CHECK_LAUNCH();
     KPAX_CUDA(cudaStreamSynchronize(st));
     n->step = 0;
     return kpax_mlp_pack(n, stream);
@@ -531,11 +723,9 @@ kpax_status kpax_mlp_forward(kpax_mlp* n, const float* d_x, uint32_t rows, float
 {
     if(!n || !d_x || !d_out || rows > n->max_batch) return set_error("kpax_mlp_forward: bad arguments"), KPAX_EINVAL;
     if(!rows) return KPAX_OK;
-    cudaStream_t st = (cudaStream_t)stream;
-    kpax_status s = mlp_forward_f32(n, d_x, rows, st);
-    if(s != KPAX_OK) return s;
-    KPAX_CUDA(cudaMemcpyAsync(d_out, n->o, (size_t)rows * kOutPad * 4, cudaMemcpyDeviceToDevice, st));
-    return KPAX_OK;
+    RowArgs a{};
+    a.x = d_x, a.n = rows, a.w = n->w, a.wt = n->wt, a.out = d_out;
+    return launch_rows<false>(n, a, (cudaStream_t)stream);
 }
 
 kpax_status kpax_mlp_loss_grad(kpax_mlp* n, const float* d_x, const float* d_y, uint32_t rows, float* h_loss, float* d_grad,
@@ -543,10 +733,8 @@ kpax_status kpax_mlp_loss_grad(kpax_mlp* n, const float* d_x, const float* d_y, 
 {
     if(!n || !d_x || !d_y || !rows || rows > n->max_batch) return set_error("kpax_mlp_loss_grad: bad arguments"), KPAX_EINVAL;
     cudaStream_t st = (cudaStream_t)stream;
-    kpax_status s = mlp_forward_f32(n, d_x, rows, st);
-    if(s == KPAX_OK) s = mlp_backward_f32(n, d_x, d_y, rows, st);
+    kpax_status s = mlp_gradient(n, d_x, d_y, nullptr, rows, d_grad ? d_grad : n->g, nullptr, st);
     if(s != KPAX_OK) return s;
-    if(d_grad) KPAX_CUDA(cudaMemcpyAsync(d_grad, n->g, kNumParams * 4, cudaMemcpyDeviceToDevice, st));
     if(h_loss) {
         KPAX_CUDA(cudaMemcpyAsync(n->h_loss, n->loss, 4, cudaMemcpyDeviceToHost, st));
         KPAX_CUDA(cudaStreamSynchronize(st));
@@ -561,17 +749,11 @@ kpax_status kpax_mlp_train_step(kpax_mlp* n, const float* d_x, const float* d_y,
     if(!n || !d_x || !d_y || !d_idx || !batch || batch > n->max_batch || !(lr > 0.0f))
         return set_error("kpax_mlp_train_step: bad arguments"), KPAX_EINVAL;
     cudaStream_t st = (cudaStream_t)stream;
-    k_gather<<<blocks((size_t)batch * (kInPad + kDim), 256), 256, 0, st>>>(d_x, d_y, d_idx, batch, n->xb, n->yb);
-    count_launch();
-    kpax_status s = mlp_forward_f32(n, n->xb, batch, st);
-    if(s == KPAX_OK) s = mlp_backward_f32(n, n->xb, n->yb, batch, st);
+    const double b1 = 0.9, b2 = 0.999, t = (double)(n->step + 1);
+    const AdamArgs o{n->w, n->wt, n->m, n->v, (float)b1, (float)b2, (float)(lr / (1.0 - pow(b1, t))), (float)(1.0 / (1.0 - pow(b2, t))), 1e-8f};
+    kpax_status s = mlp_gradient(n, d_x, d_y, d_idx, batch, n->g, &o, st);
     if(s != KPAX_OK) return s;
     n->step += 1;
-    const double b1 = 0.9, b2 = 0.999;
-    const float c1 = (float)(lr / (1.0 - pow(b1, (double)n->step))), c2 = (float)(1.0 / (1.0 - pow(b2, (double)n->step)));
-    k_adam<<<blocks(kNumParams, 256), 256, 0, st>>>(n->w, n->g, n->m, n->v, kNumParams, (float)b1, (float)b2, c1, c2, 1e-8f);
-    count_launch();
-    KPAX_CHECK_LAUNCH();
     n->packed = false;
     if(h_loss) {
         KPAX_CUDA(cudaMemcpyAsync(n->h_loss, n->loss, 4, cudaMemcpyDeviceToHost, st));
