@@ -187,19 +187,13 @@ __global__ void __launch_bounds__(kFrontierBS) k_write_all(const QueryDev* __res
 // query without children, which publishes its empty append).  Look-back waits only on lower tiles
 // of the same query, which lower global units hold: every CTA must be resident (the host sizes the
 // grid by occupancy), and the successor is released only at completion.
-// CTAs per SM the batch expansion is compiled for.  A batch has children for every SM many times
-// over, so its expansion is bound by how many warps each SM interleaves: 256-child tiles run four
-// (quadrotor, 64 registers a thread) or five (the 6-state models, 48) CTAs per SM, whatever that
-// spills.  1024 mixed queries on a B200: 790 M valid expansions/s, against 785 at four CTAs for
-// every model, 757 at three, 683 at one 512-child CTA (16 warps) and 629 at one 448-child CTA.
-// Other tile sizes keep the single-query bound.
+// CTAs per SM the batch expansion is compiled for.  A batch has children for every SM many times over,
+// so registers are traded for warps: 256-child tiles run two (quadrotor, 128 registers a thread) or
+// four (the 6-state models, 64) CTAs per SM.  96 mixed queries of 150 iterations on a B200: 157 ms, 159
+// with three CTAs of the 6-state models and 164 with five, 159 with three of the quadrotor and 178
+// with four, which spill 300 bytes in the step's loop.  Other tile sizes keep the single-query bound.
 template <int M, int BS>
-constexpr int kExpandAllMinBlocks = BS == 256 ? (M == KPAX_MODEL_QUADROTOR ? 4 : 5) : (512 / BS > 0 ? 512 / BS : 1);
-
-// Steps per collision query: the kept states of four quadrotor or five 6-state CTAs of 256 threads
-// must fit in an SM beside the queries' offsets.
-template <int M, int BS>
-constexpr int kGroupAll = BS == 256 && M == KPAX_MODEL_QUADROTOR ? 3 : kGroup;
+constexpr int kExpandAllMinBlocks = BS == 256 ? (M == KPAX_MODEL_QUADROTOR ? 2 : 4) : (512 / BS > 0 ? 512 / BS : 1);
 
 template <int M, int BS>
 __global__ void __launch_bounds__(BS, (kExpandAllMinBlocks<M, BS>)) k_expand_all(const QueryDev* __restrict__ qs,
@@ -208,7 +202,7 @@ __global__ void __launch_bounds__(BS, (kExpandAllMinBlocks<M, BS>)) k_expand_all
                                                                                 uint32_t nq, uint32_t* __restrict__ active)
 {
     extern __shared__ __align__(16) float s_save[];  // kept states, then the offsets
-    uint32_t* s_off = reinterpret_cast<uint32_t*>(s_save + kSaveBytes<M, BS, kGroupAll<M, BS>> / sizeof(float));
+    uint32_t* s_off = reinterpret_cast<uint32_t*>(s_save + kSaveBytes<M, BS> / sizeof(float));
     __shared__ QueryDev sq;
     __shared__ ExpandSmem<BS / 32> sm;
     __shared__ uint32_t s_warp[BS / 32];
@@ -225,7 +219,7 @@ __global__ void __launch_bounds__(BS, (kExpandAllMinBlocks<M, BS>)) k_expand_all
             n = sq.ctl->n, k = sq.ctl->k;
             cur = i;
         }
-        if(!expand_query_tiles<M, BS, kGroupAll<M, BS>, true>(sq, n, k, g - s_off[i], 0x80000000u, active, sm, s_save, true)) return;
+        if(!expand_query_tiles<M, BS, kGroup, true>(sq, n, k, g - s_off[i], 0x80000000u, active, sm, s_save, true)) return;
     }
 }
 

@@ -84,10 +84,10 @@ void* expand_kernel(int bs)
 }
 
 // Shared memory of the kept states of a block of bs children (run_steps), by model 1..3.
-size_t save_bytes(int model, int bs, int group = kGroup)
+size_t save_bytes(int model, int bs)
 {
     const size_t sd = model == KPAX_MODEL_QUADROTOR ? 12 : 6;
-    return sizeof(float) * (size_t)group * sd * (size_t)bs;
+    return sizeof(float) * (size_t)kGroup * sd * (size_t)bs;
 }
 
 // Allows a kernel its dynamic shared memory (more than the 48 KB a launch may ask for by default).
@@ -434,9 +434,7 @@ struct PlanBatch {
     // Dynamic shared memory of the persistent expansion of model group m with g queries.
     size_t expand_all_smem(int m, size_t g) const
     {
-        const int bs = expand_bs[m];
-        const int group = m == 2 && bs == 256 ? kGroupAll<KPAX_MODEL_QUADROTOR, 256> : kGroup;
-        return save_bytes(m + 1, bs, group) + 4 * (g + 1);
+        return save_bytes(m + 1, expand_bs[m]) + 4 * (g + 1);
     }
 
     void update_fused()
