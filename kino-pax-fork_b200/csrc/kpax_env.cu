@@ -180,22 +180,32 @@ __global__ void __launch_bounds__(kBatchBS<M>, kBatchBlocks) k_propagate_batch(K
     if(steps_out) steps_out[i] = done;
 }
 
-// Large batches run in phases so that lanes do not idle behind their warp's longest segment: the
-// head runs every segment for its first kHeadSteps steps and finishes the segments that end there
-// (a fifth of them fail in their first steps); the others are appended, state and controls, to a
-// compact list.  A middle phase carries that list to 3/5 of the longest segment (mid_steps),
-// finishes the segments that end by then and appends the rest to a second list, which the tail
-// carries to the end, each with full warps.  Every phase runs the same per-step code in the same
-// order, so rows, verdicts and step counts equal the one-pass kernel's.  Dubins microbench, 2^22
-// segments of 20 steps: 2.15 G valid segments/s in two phases; 2.15 / 2.18 / 2.19 G/s with the
-// middle phase ending after step 6 / 8 / 12.
-constexpr int kHeadSteps = 2;
-inline int mid_steps(const KParams& p) { return std::max(kHeadSteps + 1, (p.nsteps + 1) * 3 / 5); }
-constexpr uint32_t kPhasedMin = 1u << 18;   // segments; below this the one-pass kernel is used
-// Segments per round of the three phases (bounds the survivor lists' scratch).  Each round pays the
-// latency of its longest segment in every phase, so rounds are as large as the scratch allows:
-// rounds of 2^19 segments (lists resident in L2 between the phases) measured 1.73 G segments/s
-// on the Dubins microbench against 2.18 G/s in one round of 2^22.
+// Large batches run in two phases so that lanes do not idle behind their warp's longest segment: the
+// head runs every segment for its first kHeadSteps steps and finishes the segments that end there; the
+// others are appended, state and controls, to a compact list, which the tail carries to the end with
+// full warps.  Both run the same per-step code in the same order, so rows, verdicts and step counts
+// equal the one-pass kernel's.
+// What bounds the kernels is instruction issue (Dubins, 2^20 segments: 70-77 % of the issue slots, 24 of
+// 32 lanes), so a phase must save more steps and walks than its appends and reloads cost.  A head of one
+// query group asks for no more queries than one pass would; only the quadrotor, whose step costs most,
+// gains by dropping its dead sooner.  B200, us, one pass / head of 2 / of 5 / of 2 and a middle phase:
+// Dubins 2^22, 200 obstacles 615 / 625 / 579 / 639, 1500 obstacles 859 / 637 / 633 / 656;
+// quadrotor 2^21, 200 obstacles 1302 / 1191 / 1173 / 1201, 2000 obstacles 1418 / 582 / 661 / 579.
+template <int M>
+constexpr int kHeadSteps = M == KPAX_MODEL_QUADROTOR ? 2 : kBatchGroup;
+// The phases need a few waves of CTAs to fill the chip twice (one pass / two phases, us: Dubins 2^18, 200
+// obstacles 58 / 66, 2^19 93 / 96, with 1500 obstacles 130 / 113; quadrotor 2^18, 200 obstacles 181 / 182,
+// with 2000 208 / 125), and segments of more than two query groups: those of ten steps leave the tail
+// too little (double integrator 2^22, 20 obstacles 235 / 266, 200 obstacles 263 / 291).
+template <int M>
+constexpr uint32_t kPhasedMin = 2048u * kBatchBS<M>;
+template <int M>
+inline bool phased(const KParams& p, uint32_t n)
+{
+    return n >= kPhasedMin<M> && p.nsteps > 2 * kBatchGroup;
+}
+// Segments per round of the two phases (bounds the survivor list's scratch).  Each round pays the
+// latency of its longest segment in both phases, so rounds are as large as the scratch allows.
 constexpr uint32_t kPhaseChunk = 1u << 24;
 
 struct LiveList {
@@ -255,7 +265,7 @@ __global__ void __launch_bounds__(kBatchBS<M>, kBatchBlocks) k_propagate_head(KP
                                                         int32_t* __restrict__ steps_out, LiveList live)
 {
     constexpr int SD = ModelDims<M>::SD, CD = ModelDims<M>::CD;
-    __shared__ __align__(16) float s_save[kHeadSteps * SD * kBatchBS<M>];
+    __shared__ __align__(16) float s_save[kHeadSteps<M> * SD * kBatchBS<M>];
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     const int lane = threadIdx.x & 31;
     bool alive = false;
@@ -276,7 +286,8 @@ __global__ void __launch_bounds__(kBatchBS<M>, kBatchBlocks) k_propagate_head(KP
         const auto k = segment_consts<M>(p, c);
         const StepParams sp = step_params(p);
         int done = 0;
-        const bool ok = run_steps<M, kHeadSteps>(sp, g, s, c, k, min(steps, kHeadSteps), done, s_save + threadIdx.x * SD, kBatchBS<M>);
+        const bool ok = run_steps<M, kHeadSteps<M>>(sp, g, s, c, k, min(steps, kHeadSteps<M>), done, s_save + threadIdx.x * SD,
+                                                    kBatchBS<M>);
         alive = ok && done < steps;
         if(!alive) write_segment<M>(p, i, s, c, steps, ok, done, rows, valid, steps_out);
     }
@@ -286,54 +297,42 @@ __global__ void __launch_bounds__(kBatchBS<M>, kBatchBlocks) k_propagate_head(KP
 template <int M>
 __global__ void __launch_bounds__(kBatchBS<M>, kBatchBlocks) k_propagate_tail(KParams p, Grid g, float* __restrict__ rows,
                                                         uint8_t* __restrict__ valid, int32_t* __restrict__ steps_out,
-                                                        LiveList live, int from, int until, LiveList next)
+                                                        LiveList live)
 {
     constexpr int SD = ModelDims<M>::SD, CD = ModelDims<M>::CD;
     __shared__ __align__(16) float s_save[kBatchGroup * SD * kBatchBS<M>];
-    const uint32_t count = *live.count;
-    if(blockIdx.x * blockDim.x >= count) return;  // whole block past the list: the ballot below needs full warps
     const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-    const int lane = threadIdx.x & 31;
-    bool alive = false;
-    uint32_t i = 0;
-    int steps = 0;
+    if(j >= *live.count) return;
+    const uint32_t i = live.idx[j];
+    const int steps = live.steps ? live.steps[j] : p.nsteps;
     float s[SD], c[4];
-    if(j < count) {
-        i = live.idx[j];
-        steps = live.steps ? live.steps[j] : p.nsteps;
 #pragma unroll
-        for(int k = 0; k < 4; ++k) c[k] = k < CD ? live.ctl[(size_t)j * CD + k] : 0.0f;
+    for(int k = 0; k < 4; ++k) c[k] = k < CD ? live.ctl[(size_t)j * CD + k] : 0.0f;
 #pragma unroll
-        for(int k = 0; k < SD; ++k) s[k] = live.state[(size_t)j * SD + k];
-        const auto kc = segment_consts<M>(p, c);
-        const StepParams sp = step_params(p);
-        int done = from;
-        const bool ok = run_steps<M, kBatchGroup>(sp, g, s, c, kc, min(steps, until), done, s_save + threadIdx.x * SD, kBatchBS<M>);
-        alive = next.count && ok && done < steps;
-        if(!alive) write_segment<M>(p, i, s, c, steps, ok, done, rows, valid, steps_out);
-    }
-    if(next.count) append_live<SD, CD>(next, alive, lane, i, steps, c, s);
+    for(int k = 0; k < SD; ++k) s[k] = live.state[(size_t)j * SD + k];
+    const auto kc = segment_consts<M>(p, c);
+    const StepParams sp = step_params(p);
+    int done = kHeadSteps<M>;
+    const bool ok = run_steps<M, kBatchGroup>(sp, g, s, c, kc, steps, done, s_save + threadIdx.x * SD, kBatchBS<M>);
+    write_segment<M>(p, i, s, c, steps, ok, done, rows, valid, steps_out);
 }
 
-// The three phases over rounds of kPhaseChunk segments; `counts` (two words, 128 bytes apart) are
-// cleared before every round.
+// The two phases over rounds of kPhaseChunk segments; the list's count is cleared before every round.
 template <int M>
 void launch_phases(const KParams& p, const Grid& g, const float* parents, const float* draws, uint32_t stream_id, uint32_t n,
-                   float* rows, uint8_t* valid, int32_t* steps_out, const LiveList& first, const LiveList& second,
-                   const LiveList& none, void* counts, cudaStream_t s)
+                   float* rows, uint8_t* valid, int32_t* steps_out, const LiveList& live, cudaStream_t s)
 {
-    const int SD = p.sd, S = p.S, mid = mid_steps(p);
+    const int SD = p.sd, S = p.S;
     for(uint32_t o = 0; o < n; o += kPhaseChunk) {
         const uint32_t m = std::min(kPhaseChunk, n - o), bs = kBatchBS<M>, blocks = (m + bs - 1) / bs;
         float* r = rows + (size_t)o * S;
         uint8_t* v = valid + o;
         int32_t* st = steps_out ? steps_out + o : nullptr;
-        cudaMemsetAsync(counts, 0, 256, s);
+        cudaMemsetAsync(live.count, 0, sizeof(uint32_t), s);
         k_propagate_head<M><<<blocks, bs, 0, s>>>(p, g, parents + (size_t)o * SD, draws ? draws + (size_t)o * 5 : nullptr,
-                                                   stream_id, m, o, r, v, st, first);
-        k_propagate_tail<M><<<blocks, bs, 0, s>>>(p, g, r, v, st, first, kHeadSteps, mid, second);
-        k_propagate_tail<M><<<blocks, bs, 0, s>>>(p, g, r, v, st, second, mid, INT_MAX, none);
-        count_launch(3);
+                                                   stream_id, m, o, r, v, st, live);
+        k_propagate_tail<M><<<blocks, bs, 0, s>>>(p, g, r, v, st, live);
+        count_launch(2);
     }
 }
 
@@ -634,44 +633,39 @@ kpax_status kpax_propagate_batch(const kpax_config* cfg, kpax_env* env, const fl
     if(st != KPAX_OK) return st;
     if(p.gdim != env->env.dim || p.cell != env->env.cell || p.wmin != env->env.wmin)
         return set_error("kpax_propagate_batch: env was built for another workspace grid"), KPAX_EINVAL;
-    if(n < kPhasedMin)
+    const bool two = p.model == KPAX_MODEL_DOUBLE_INTEGRATOR ? phased<KPAX_MODEL_DOUBLE_INTEGRATOR>(p, n)
+                     : p.model == KPAX_MODEL_DUBINS_AIRPLANE ? phased<KPAX_MODEL_DUBINS_AIRPLANE>(p, n)
+                                                             : phased<KPAX_MODEL_QUADROTOR>(p, n);
+    if(!two)
         return launch_propagate(p, env->env.view(), d_parents, d_draws, draw_stream, n, d_rows, d_valid, d_steps,
                                 (cudaStream_t)stream);
-    // phases: the two live lists of a round live in the env's scratch, grown on demand (counts at
-    // bytes 0 and 128, then each list's index, step-count (drawn durations only), control and state
-    // arrays)
+    // phases: the live list of a round lives in the env's scratch, grown on demand (its count, then its
+    // index, step-count (drawn durations only), control and state arrays)
     Env& e = env->env;
     auto align = [](size_t b) { return (b + 255) / 256 * 256; };
     const size_t m = std::min(n, kPhaseChunk);
-    const size_t l_idx = 0, l_steps = align(4ull * m), l_ctl = l_steps + (p.fixed_steps ? 0 : align(4ull * m)),
-                 l_state = l_ctl + align(4ull * p.cd * m), l_bytes = l_state + align(4ull * p.sd * m), bytes = 256 + 2 * l_bytes;
+    const size_t l_idx = 256, l_steps = l_idx + align(4ull * m), l_ctl = l_steps + (p.fixed_steps ? 0 : align(4ull * m)),
+                 l_state = l_ctl + align(4ull * p.cd * m), bytes = l_state + align(4ull * p.sd * m);
     if(bytes > e.live_cap) {
         if(e.d_live) cudaFree(e.d_live), e.d_live = nullptr, e.live_cap = 0;
         KPAX_CUDA(cudaMalloc(&e.d_live, bytes));
         e.live_cap = bytes;
     }
-    char* base = static_cast<char*>(e.d_live);
-    auto list = [&](int k) {
-        char* l = base + 256 + (size_t)k * l_bytes;
-        return LiveList{reinterpret_cast<uint32_t*>(base + 128 * k), reinterpret_cast<uint32_t*>(l + l_idx),
+    char* l = static_cast<char*>(e.d_live);
+    const LiveList live{reinterpret_cast<uint32_t*>(l), reinterpret_cast<uint32_t*>(l + l_idx),
                         p.fixed_steps ? nullptr : reinterpret_cast<int32_t*>(l + l_steps), reinterpret_cast<float*>(l + l_ctl),
                         reinterpret_cast<float*>(l + l_state)};
-    };
-    const LiveList first = list(0), second = list(1), none{};
     cudaStream_t s = (cudaStream_t)stream;
     const Grid g = e.view();
     switch(p.model) {
         case KPAX_MODEL_DOUBLE_INTEGRATOR:
-            launch_phases<KPAX_MODEL_DOUBLE_INTEGRATOR>(p, g, d_parents, d_draws, draw_stream, n, d_rows, d_valid, d_steps, first,
-                                                       second, none, base, s);
+            launch_phases<KPAX_MODEL_DOUBLE_INTEGRATOR>(p, g, d_parents, d_draws, draw_stream, n, d_rows, d_valid, d_steps, live, s);
             break;
         case KPAX_MODEL_DUBINS_AIRPLANE:
-            launch_phases<KPAX_MODEL_DUBINS_AIRPLANE>(p, g, d_parents, d_draws, draw_stream, n, d_rows, d_valid, d_steps, first,
-                                                     second, none, base, s);
+            launch_phases<KPAX_MODEL_DUBINS_AIRPLANE>(p, g, d_parents, d_draws, draw_stream, n, d_rows, d_valid, d_steps, live, s);
             break;
         default:
-            launch_phases<KPAX_MODEL_QUADROTOR>(p, g, d_parents, d_draws, draw_stream, n, d_rows, d_valid, d_steps, first, second,
-                                               none, base, s);
+            launch_phases<KPAX_MODEL_QUADROTOR>(p, g, d_parents, d_draws, draw_stream, n, d_rows, d_valid, d_steps, live, s);
             break;
     }
     KPAX_CHECK_LAUNCH();
