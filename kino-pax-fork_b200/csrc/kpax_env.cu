@@ -132,6 +132,76 @@ __global__ void k_env_fill(Grid g, const float4* __restrict__ packed, uint32_t n
     for(int k = lane; k < total; k += 32) ent[atomicAdd(cursor + box_cell(g, c0, c1, k), 1u)] = o;
 }
 
+// The three passes in one CTA with the counts in shared memory, for grids and obstacle counts that one
+// SM gets through sooner than the launches of three kernels and a memset take; its latency is a chain of
+// atomics and scattered stores per obstacle, eight lanes each.  Entries are filled in when they fit `cap`;
+// otherwise `cursor` holds the offsets for k_env_fill.  B200, the allocation-free batch with 1021
+// segments on an 8000-cell grid, host us, three kernels / one: 1 obstacle 54 / 41, 20 54 / 46, 300 56 / 52,
+// 1000 58 / 88.
+constexpr int kEnvBuildBS = 1024;
+constexpr uint32_t kEnvBuildCells = 12000;  // 48 KB of shared memory with the scan's
+constexpr uint32_t kEnvBuildObstacles = 256;
+inline bool env_build_once(uint32_t cells, uint32_t n) { return cells <= kEnvBuildCells && n <= kEnvBuildObstacles; }
+
+__global__ void __launch_bounds__(kEnvBuildBS) k_env_build(Grid g, const float* __restrict__ obs, uint32_t n, uint32_t cells,
+                                                           float4* __restrict__ packed, uint32_t* __restrict__ off,
+                                                           uint32_t* __restrict__ cursor, uint32_t* __restrict__ ent, uint32_t cap)
+{
+    extern __shared__ uint32_t s_cell[];  // counts, then offsets, then the next free entry
+    __shared__ uint32_t s_warp[32];
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    for(uint32_t i = tid; i < cells; i += kEnvBuildBS) s_cell[i] = 0u;
+    __syncthreads();
+    auto each_cell = [&](bool pack, auto f) {
+        for(uint32_t o = tid >> 3; o < n; o += kEnvBuildBS / 8) {
+            const float* b = obs + (size_t)6 * o;
+            const float4 lo = make_float4(b[0], b[1], b[2], 0.0f), hi = make_float4(b[3], b[4], b[5], 0.0f);
+            if(pack && (tid & 7u) == 0) packed[2 * o] = lo, packed[2 * o + 1] = hi;
+            int c0[3], c1[3];
+            obstacle_cells(g, lo, hi, c0, c1);
+            const int total = box_cells(c0, c1);
+            for(int k = (int)(tid & 7u); k < total; k += 8) {
+                const uint32_t c = (uint32_t)box_cell(g, c0, c1, k);
+                if(c < cells) f(o, c);  // an inverted box can name cells outside the grid
+            }
+        }
+    };
+    each_cell(true, [&](uint32_t, uint32_t c) { atomicAdd(s_cell + c, 1u); });
+    __syncthreads();
+    const uint32_t per = (cells + kEnvBuildBS - 1) / kEnvBuildBS | 1u;  // odd: no bank conflicts
+    const uint32_t i0 = min(tid * per, cells), i1 = min(i0 + per, cells);
+    uint32_t sum = 0;
+    for(uint32_t i = i0; i < i1; ++i) sum += s_cell[i];
+    auto warp_scan = [&](uint32_t v) {
+#pragma unroll
+        for(int d = 1; d < 32; d <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, v, d);
+            if(lane >= (uint32_t)d) v += y;
+        }
+        return v;
+    };
+    const uint32_t x = warp_scan(sum);
+    if(lane == 31u) s_warp[warp] = x;
+    __syncthreads();
+    if(warp == 0) s_warp[lane] = warp_scan(s_warp[lane]);
+    __syncthreads();
+    uint32_t acc = (warp ? s_warp[warp - 1] : 0u) + x - sum;
+    for(uint32_t i = i0; i < i1; ++i) {
+        const uint32_t v = s_cell[i];
+        s_cell[i] = acc, acc += v;
+    }
+    const uint32_t total = s_warp[31];
+    __syncthreads();
+    for(uint32_t i = tid; i < cells; i += kEnvBuildBS) {
+        off[i] = s_cell[i];
+        if(total > cap) cursor[i] = s_cell[i];
+    }
+    if(tid == 0) off[cells] = total;
+    if(total > cap) return;
+    __syncthreads();
+    each_cell(false, [&](uint32_t o, uint32_t c) { ent[atomicAdd(s_cell + c, 1u)] = o; });
+}
+
 inline uint32_t warp_blocks(uint32_t n) { return (uint32_t)(((uint64_t)n * 32 + 255) / 256); }
 
 // ---------------------------------------------------------------- batch kernels
@@ -431,7 +501,7 @@ __global__ void k_sincos_pair(const float* __restrict__ x, uint32_t n, float* __
 
 }  // namespace
 
-kpax_status Env::build(const KParams& p, const float* d_obstacles, uint32_t n, cudaStream_t stream)
+kpax_status Env::build_start(const KParams& p, const float* d_obstacles, uint32_t n, cudaStream_t stream)
 {
     cell = p.cell;
     wmin = p.wmin;
@@ -451,38 +521,59 @@ kpax_status Env::build(const KParams& p, const float* d_obstacles, uint32_t n, c
         obs_cap = n;
     }
     n_obs = n;
-    KPAX_CUDA(cudaMemsetAsync(d_off, 0, sizeof(uint32_t) * (cells + 1), stream));
-    const Grid g0 = view();
-    if(n) {
-        k_env_count<<<warp_blocks(n), 256, 0, stream>>>(g0, d_obstacles, n, d_obs, d_off);
-        KPAX_CHECK_LAUNCH();
-        k_env_scan<<<1, 1024, 0, stream>>>(d_off, cells, d_cursor);
-        KPAX_CHECK_LAUNCH();
-        count_launch(2);
-        KPAX_CUDA(cudaMemcpyAsync(h_total, d_off + cells, sizeof(uint32_t), cudaMemcpyDeviceToHost, stream));
-        KPAX_CUDA(cudaStreamSynchronize(stream));
-        n_ent = *h_total;
-        if(n_ent > ent_cap) {
-            if(d_ent) cudaFree(d_ent), d_ent = nullptr;
-            const uint32_t want = n_ent + n_ent / 4 + 1024;
-            KPAX_CUDA(cudaMalloc(&d_ent, sizeof(uint32_t) * want));
-            ent_cap = want;
-        }
-        k_env_fill<<<warp_blocks(n), 256, 0, stream>>>(view(), d_obs, n, d_cursor, d_ent);
+    if(!d_ent) {
+        KPAX_CUDA(cudaMalloc(&d_ent, sizeof(uint32_t) * 1024));
+        ent_cap = 1024;
+    }
+    if(!d_obs) {
+        KPAX_CUDA(cudaMalloc(&d_obs, sizeof(float4) * 2));
+        obs_cap = 1;
+    }
+    filled = false;
+    if(n && env_build_once(cells, n)) {
+        k_env_build<<<1, kEnvBuildBS, sizeof(uint32_t) * cells, stream>>>(view(), d_obstacles, n, cells, d_obs, d_off, d_cursor, d_ent, ent_cap);
         KPAX_CHECK_LAUNCH();
         count_launch(1);
+        filled = true;
     } else {
-        n_ent = 0;
-        if(!d_ent) {
-            KPAX_CUDA(cudaMalloc(&d_ent, sizeof(uint32_t) * 1024));
-            ent_cap = 1024;
-        }
-        if(!d_obs) {
-            KPAX_CUDA(cudaMalloc(&d_obs, sizeof(float4) * 2));
-            obs_cap = 1;
+        KPAX_CUDA(cudaMemsetAsync(d_off, 0, sizeof(uint32_t) * (cells + 1), stream));
+        if(n) {
+            k_env_count<<<warp_blocks(n), 256, 0, stream>>>(view(), d_obstacles, n, d_obs, d_off);
+            KPAX_CHECK_LAUNCH();
+            k_env_scan<<<1, 1024, 0, stream>>>(d_off, cells, d_cursor);
+            KPAX_CHECK_LAUNCH();
+            count_launch(2);
         }
     }
+    *h_total = 0;
+    if(n) KPAX_CUDA(cudaMemcpyAsync(h_total, d_off + cells, sizeof(uint32_t), cudaMemcpyDeviceToHost, stream));
     return KPAX_OK;
+}
+
+kpax_status Env::build_finish(cudaStream_t stream)
+{
+    n_ent = *h_total;
+    if(n_ent > ent_cap) {
+        filled = false;
+        if(d_ent) cudaFree(d_ent), d_ent = nullptr, ent_cap = 0;
+        const uint32_t want = n_ent + n_ent / 4 + 1024;
+        KPAX_CUDA(cudaMalloc(&d_ent, sizeof(uint32_t) * want));
+        ent_cap = want;
+    }
+    if(n_obs && !filled) {
+        k_env_fill<<<warp_blocks(n_obs), 256, 0, stream>>>(view(), d_obs, n_obs, d_cursor, d_ent);
+        KPAX_CHECK_LAUNCH();
+        count_launch(1);
+    }
+    return KPAX_OK;
+}
+
+kpax_status Env::build(const KParams& p, const float* d_obstacles, uint32_t n, cudaStream_t stream)
+{
+    kpax_status st = build_start(p, d_obstacles, n, stream);
+    if(st != KPAX_OK) return st;
+    if(n) KPAX_CUDA(cudaStreamSynchronize(stream));
+    return build_finish(stream);
 }
 
 void Env::release()
@@ -780,14 +871,23 @@ extern "C" kpax_status kpax_propagate_batch_noalloc(const kpax_config* cfg, cons
     if((st = noalloc_scratch(&s)) != KPAX_OK) return st;
     cudaStream_t cs = (cudaStream_t)stream;
     const Grid g{s->obs, s->off, s->ent, p.wmin, 1.0f / p.cell, p.gdim};
-    // the array keeps the previous call's grid: the counts must start from zero
-    KPAX_CUDA(cudaMemsetAsync(s->off, 0, sizeof(uint32_t) * (cells + 1), cs));
+    const bool once = n_obs && env_build_once(cells, n_obs);
+    if(once) {
+        k_env_build<<<1, kEnvBuildBS, sizeof(uint32_t) * cells, cs>>>(g, d_obstacles, n_obs, cells, s->obs, s->off, s->cursor, s->ent, kNoAllocMaxEntries);
+        KPAX_CHECK_LAUNCH();
+        count_launch(1);
+    } else {
+        // the array keeps the previous call's grid: the counts must start from zero
+        KPAX_CUDA(cudaMemsetAsync(s->off, 0, sizeof(uint32_t) * (cells + 1), cs));
+        if(n_obs) {
+            k_env_count<<<warp_blocks(n_obs), 256, 0, cs>>>(g, d_obstacles, n_obs, s->obs, s->off);
+            KPAX_CHECK_LAUNCH();
+            k_env_scan<<<1, 1024, 0, cs>>>(s->off, cells, s->cursor);
+            KPAX_CHECK_LAUNCH();
+            count_launch(2);
+        }
+    }
     if(n_obs) {
-        k_env_count<<<warp_blocks(n_obs), 256, 0, cs>>>(g, d_obstacles, n_obs, s->obs, s->off);
-        KPAX_CHECK_LAUNCH();
-        k_env_scan<<<1, 1024, 0, cs>>>(s->off, cells, s->cursor);
-        KPAX_CHECK_LAUNCH();
-        count_launch(2);
         uint32_t total = 0;
         KPAX_CUDA(cudaMemcpyAsync(&total, s->off + cells, sizeof(uint32_t), cudaMemcpyDeviceToHost, cs));
         KPAX_CUDA(cudaStreamSynchronize(cs));
@@ -795,9 +895,11 @@ extern "C" kpax_status kpax_propagate_batch_noalloc(const kpax_config* cfg, cons
             return set_error("kpax_propagate_batch_noalloc: %u (cell, obstacle) pairs exceed the limit of %u", total,
                              kNoAllocMaxEntries),
                    KPAX_ECAPACITY;
-        k_env_fill<<<warp_blocks(n_obs), 256, 0, cs>>>(g, s->obs, n_obs, s->cursor, s->ent);
-        KPAX_CHECK_LAUNCH();
-        count_launch(1);
+        if(!once) {
+            k_env_fill<<<warp_blocks(n_obs), 256, 0, cs>>>(g, s->obs, n_obs, s->cursor, s->ent);
+            KPAX_CHECK_LAUNCH();
+            count_launch(1);
+        }
     }
     return launch_propagate(p, g, d_parents, d_draws, draw_stream, n, d_rows, d_valid, d_steps, cs);
 }

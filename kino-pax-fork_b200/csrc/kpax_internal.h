@@ -67,6 +67,7 @@ struct Env {
     uint32_t* d_ent = nullptr;
     uint32_t* h_total = nullptr;  // pinned
     uint32_t obs_cap = 0, ent_cap = 0;
+    bool filled = false;  // the entries fit and are in place (build_start)
     bool owned_by_planner = false;
     void* d_live = nullptr;  // scratch of the phased segment batch (grown on demand)
     size_t live_cap = 0;
@@ -74,6 +75,10 @@ struct Env {
     Grid view() const { return Grid{d_obs, d_off, d_ent, wmin, 1.0f / cell, dim}; }
     // Build from n x 6 device floats on `stream` (synchronises once to size the entry list).
     kpax_status build(const KParams& p, const float* d_obstacles, uint32_t n, cudaStream_t stream);
+    // The same in two halves, so that several environments can share one synchronisation of `stream`
+    // between them; view() is final after the second.
+    kpax_status build_start(const KParams& p, const float* d_obstacles, uint32_t n, cudaStream_t stream);
+    kpax_status build_finish(cudaStream_t stream);
     void release();
 };
 
