@@ -729,25 +729,33 @@ struct PlanBatch {
     {
         if(!h_init || !h_goal) return set_error("plan: null start or goal"), KPAX_EINVAL;
         if(record_start) KPAX_CUDA(cudaEventRecord(ev0, stream));
+        // the grids of all queries are counted, then one synchronisation sizes their entry lists
+        bool counted = false;
         for(uint32_t q = 0; q < nq; ++q) {
             if(n_obs[q] && !d_obstacles[q]) return set_error("plan: null obstacle buffer for query %u", q), KPAX_EINVAL;
-            kpax_status st = env[q].build(prm[q], d_obstacles[q], n_obs[q], stream);
+            kpax_status st = env[q].build_start(prm[q], d_obstacles[q], n_obs[q], stream);
+            if(st != KPAX_OK) return st;
+            counted = counted || n_obs[q];
+            const uint32_t S = (uint32_t)prm[q].S;
+            memcpy(h_ig + (size_t)q * 2 * s_max, h_init + (size_t)q * stride, sizeof(float) * S);
+            memcpy(h_ig + (size_t)q * 2 * s_max + S, h_goal + (size_t)q * stride, sizeof(float) * S);
+        }
+        KPAX_CUDA(cudaMemcpyAsync(d_ig, h_ig, sizeof(float) * nq * 2 * s_max, cudaMemcpyHostToDevice, stream));
+        KPAX_CUDA(cudaMemsetAsync(pool + region_lo, 0, region_hi - region_lo, stream));
+        *h_active = nq;
+        KPAX_CUDA(cudaMemcpyAsync(d_active, h_active, sizeof(uint32_t), cudaMemcpyHostToDevice, stream));
+        if(counted) KPAX_CUDA(cudaStreamSynchronize(stream));
+        for(uint32_t q = 0; q < nq; ++q) {
+            kpax_status st = env[q].build_finish(stream);
             if(st != KPAX_OK) return st;
             hq[q].g = env[q].view();
             if(hq[q].occ) {
                 st = launch_occupancy(prm[q], hq[q].g, const_cast<uint32_t*>(hq[q].occ), stream);
                 if(st != KPAX_OK) return st;
             }
-            const uint32_t S = (uint32_t)prm[q].S;
-            memcpy(h_ig + (size_t)q * 2 * s_max, h_init + (size_t)q * stride, sizeof(float) * S);
-            memcpy(h_ig + (size_t)q * 2 * s_max + S, h_goal + (size_t)q * stride, sizeof(float) * S);
         }
         kpax_status st = upload_descriptors();
         if(st != KPAX_OK) return st;
-        KPAX_CUDA(cudaMemcpyAsync(d_ig, h_ig, sizeof(float) * nq * 2 * s_max, cudaMemcpyHostToDevice, stream));
-        KPAX_CUDA(cudaMemsetAsync(pool + region_lo, 0, region_hi - region_lo, stream));
-        *h_active = nq;
-        KPAX_CUDA(cudaMemcpyAsync(d_active, h_active, sizeof(uint32_t), cudaMemcpyHostToDevice, stream));
         k_begin<<<dim3(1, nq), 128, 0, stream>>>(dq, plans, max_iters, stop);
         KPAX_CHECK_LAUNCH();
         count_launch();
@@ -772,8 +780,9 @@ struct PlanBatch {
             }
             if(!poll) continue;
             KPAX_CUDA(cudaMemcpyAsync(h_active, d_active, sizeof(uint32_t), cudaMemcpyDeviceToHost, stream));
+            KPAX_CUDA(cudaMemcpyAsync(h_ctl, d_ctl, sizeof(Ctl) * nq, cudaMemcpyDeviceToHost, stream));
             KPAX_CUDA(cudaStreamSynchronize(stream));
-            if(*h_active == 0u) break;
+            if(*h_active == 0u) return check_ctl();
         }
         return sync_ctl();
     }
@@ -782,6 +791,11 @@ struct PlanBatch {
     {
         KPAX_CUDA(cudaMemcpyAsync(h_ctl, d_ctl, sizeof(Ctl) * nq, cudaMemcpyDeviceToHost, stream));
         KPAX_CUDA(cudaStreamSynchronize(stream));
+        return check_ctl();
+    }
+
+    kpax_status check_ctl() const
+    {
         for(uint32_t q = 0; q < nq; ++q) {
             if(h_ctl[q].error & kErrTimeout) return set_error("query %u: a device-side wait gave up", q), KPAX_ETIMEOUT;
             if(h_ctl[q].error & kErrCapacity) return set_error("query %u: tree capacity exceeded", q), KPAX_ECAPACITY;
