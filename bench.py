@@ -1025,7 +1025,7 @@ def run_batch(args) -> None:
                 tuned_models[m] = best
         cfgs = [kpax_autotune.apply(c, tuned_models[c.model]) if c.model in tuned_models else c for c in cfgs]
     # children per expansion tile of every query: a batch expands millions of children per
-    # iteration, where the batch expansion's 256-child tiles at four or five CTAs per SM hide more
+    # iteration, where the batch expansion's 256-child tiles at two or four CTAs per SM hide more
     # latency than the single 14-warp CTA the single-query tuning picks
     if args.batch_block:
         for c in cfgs:
@@ -1245,7 +1245,7 @@ def main() -> None:
     ap.add_argument("--batch-iters", type=int, default=0, help="iteration cap of every batched query (0 = presets)")
     ap.add_argument("--batch-block", type=int, default=256, choices=[0, 128, 256, 448, 512],
                     help="children per expansion tile of every batched query (0 = the single-query tuning / "
-                         "presets; 256 measured fastest for batches: four or five CTAs per SM)")
+                         "presets; 256 measured fastest for batches: two or four CTAs per SM)")
     ap.add_argument("--seeds", type=int, default=256, help="held-out scenes of the learned workload")
     ap.add_argument("--eps", type=float, default=0.2, help="uniform fraction of the learned proposal")
     ap.add_argument("--proposal", choices=["on", "off"], default="on", help="learned proposal for batched quadrotor queries")
