@@ -7,7 +7,6 @@
 // (collisionCheck.cu:49-62) for every box: the cell map is monotone, so any strictly
 // overlapping obstacle shares at least one cell with the box.
 #include <stdio.h>
-#include <limits.h>
 #include <algorithm>
 #include <string.h>
 
