@@ -90,12 +90,17 @@ size_t save_bytes(int model, int bs)
     return sizeof(float) * (size_t)kGroup * sd * (size_t)bs;
 }
 
-// Allows a kernel its dynamic shared memory (more than the 48 KB a launch may ask for by default).
-kpax_status allow_smem(const void* fn, size_t bytes)
+// Allows a kernel up to `most` bytes of dynamic shared memory (the default limit is 48 KB).  The limit
+// belongs to the kernel, not to the planner or batch that sets it, and a launch above it is refused, so
+// every caller passes the same number for a kernel: the most that any planner or batch can need.
+kpax_status allow_smem(const void* fn, size_t most)
 {
-    KPAX_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    KPAX_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
     return KPAX_OK;
 }
+
+// Shared memory of the per-query offsets of a persistent batch stage over n queries.
+constexpr size_t offset_bytes(size_t n) { return sizeof(uint32_t) * (n + 1); }
 
 // The fused iteration kernel (or one of its two parts around the proposal pass) at one of its
 // block sizes.
@@ -369,25 +374,24 @@ struct PlanBatch {
             int dev = 0, sms = 148;
             KPAX_CUDA(cudaGetDevice(&dev));
             KPAX_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-            auto resident = [&](const void* fn, int bs, size_t smem, uint32_t& gx) -> kpax_status {
+            // a kernel with kept states of `save` bytes and offsets of `queries` queries
+            auto resident = [&](const void* fn, int bs, size_t save, size_t queries, uint32_t& gx) -> kpax_status {
                 int per_sm = 0;
-                kpax_status sst = allow_smem(fn, smem);
+                kpax_status sst = allow_smem(fn, save + offset_bytes(kBatchMaxQueries));
                 if(sst != KPAX_OK) return sst;
-                KPAX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, bs, smem));
+                KPAX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, bs, save + offset_bytes(queries)));
                 gx = (uint32_t)std::max(per_sm, 0) * (uint32_t)sms;
                 return KPAX_OK;
             };
-            const size_t sq = 4 * ((size_t)n + 1);
-            kpax_status st = resident((const void*)k_count_all, kFrontierBS, sq, gx_count_all);
-            if(st == KPAX_OK) st = resident((const void*)k_write_all, kFrontierBS, sq, gx_write_all);
-            if(st == KPAX_OK) st = resident((const void*)k_scores_all, kScoreBS, sq, gx_scores_all);
+            kpax_status st = resident((const void*)k_count_all, kFrontierBS, 0, n, gx_count_all);
+            if(st == KPAX_OK) st = resident((const void*)k_write_all, kFrontierBS, 0, n, gx_write_all);
+            if(st == KPAX_OK) st = resident((const void*)k_scores_all, kScoreBS, 0, n, gx_scores_all);
             for(int m = 0; m < 3 && st == KPAX_OK; ++m) {
                 if(groups[m].empty()) continue;
-                const size_t sg = expand_all_smem(m, groups[m].size());
                 const void* fn = m == 0 ? expand_all_kernel<KPAX_MODEL_DOUBLE_INTEGRATOR>(expand_bs[m])
                                         : m == 1 ? expand_all_kernel<KPAX_MODEL_DUBINS_AIRPLANE>(expand_bs[m])
                                                  : expand_all_kernel<KPAX_MODEL_QUADROTOR>(expand_bs[m]);
-                st = resident(fn, expand_bs[m], sg, gx_expand_all[m]);
+                st = resident(fn, expand_bs[m], save_bytes(m + 1, expand_bs[m]), groups[m].size(), gx_expand_all[m]);
             }
             if(st != KPAX_OK) return st;
             persistent = gx_count_all && gx_write_all && gx_scores_all && (groups[0].empty() || gx_expand_all[0]) &&
@@ -407,7 +411,7 @@ struct PlanBatch {
                 KPAX_CUDA(cudaMemcpyAsync(d_mixed, order.data(), sizeof(uint32_t) * order.size(), cudaMemcpyHostToDevice,
                                           stream));
                 uint32_t gx = 0;
-                if((st = resident(expand_mixed_kernel(bs0), bs0, save_bytes(KPAX_MODEL_QUADROTOR, bs0) + 4 * ((size_t)n + 1), gx)) != KPAX_OK) return st;
+                if((st = resident(expand_mixed_kernel(bs0), bs0, save_bytes(KPAX_MODEL_QUADROTOR, bs0), n, gx)) != KPAX_OK) return st;
                 if(gx) mixed_bs = bs0, gx_mixed = gx;
             }
         }
@@ -434,7 +438,7 @@ struct PlanBatch {
     // Dynamic shared memory of the persistent expansion of model group m with g queries.
     size_t expand_all_smem(int m, size_t g) const
     {
-        return save_bytes(m + 1, expand_bs[m]) + 4 * (g + 1);
+        return save_bytes(m + 1, expand_bs[m]) + offset_bytes(g);
     }
 
     void update_fused()
@@ -527,7 +531,7 @@ struct PlanBatch {
             return;
         }
         if(persistent) {  // one launch per stage over all queries; model groups one after another
-            const size_t sq = 4 * ((size_t)nq + 1);
+            const size_t sq = offset_bytes(nq);
             launch_chained(k_batch_start, dim3((nq + kBatchStartBS - 1) / kBatchStartBS), kBatchStartBS, 0, stream, d_ctl, nq,
                            d_active);
             launch_chained(k_count_all, dim3(gx_count_all), kFrontierBS, sq, stream, dq, (const Ctl*)d_ctl, nq);
@@ -712,9 +716,15 @@ struct PlanBatch {
         if(graph && key == graph_key) return KPAX_OK;
         if(graph) cudaGraphExecDestroy(graph), graph = nullptr;
         cudaGraph_t g = nullptr;
+        cudaGetLastError();  // an older call's error is not this capture's
         KPAX_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
         for(int i = 0; i < unroll; ++i) launch_iteration();
+        const cudaError_t launched = cudaGetLastError();
         cudaError_t e = cudaStreamEndCapture(stream, &g);
+        if(launched != cudaSuccess) {  // a refused launch ends the capture too: report the launch's reason
+            if(g) cudaGraphDestroy(g);
+            return set_error("launch of an iteration kernel failed: %s", cudaGetErrorString(launched)), KPAX_ECUDA;
+        }
         if(e != cudaSuccess) return set_error("graph capture failed: %s", cudaGetErrorString(e)), KPAX_ECUDA;
         e = cudaGraphInstantiate(&graph, g, 0);
         cudaGraphDestroy(g);
