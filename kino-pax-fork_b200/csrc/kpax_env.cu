@@ -773,7 +773,8 @@ kpax_status kpax_collide_batch(kpax_env* env, const float* d_bbmin, const float*
         int dev = 0, sms = 0;
         KPAX_CUDA(cudaGetDevice(&dev));
         KPAX_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        KPAX_CUDA(cudaFuncSetAttribute(k_collide_shared, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        // the limit belongs to the kernel: every call sets the same one, whatever its own grid needs
+        KPAX_CUDA(cudaFuncSetAttribute(k_collide_shared, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCollideMaxSmem));
         const uint32_t grid = (uint32_t)sms * (smem <= kCollideMaxSmem / 2 ? 2u : 1u);
         k_collide_shared<<<grid, kCollideBS, smem, (cudaStream_t)stream>>>(e.view(), e.n_cells, e.n_ent, e.n_obs, d_bbmin, d_bbmax, n, d_free);
         KPAX_CHECK_LAUNCH();

@@ -1,5 +1,9 @@
 """Objects that live side by side: a batch plans the same whether or not another batch of another size
-was created after it."""
+was created after it, and swept-box queries of environments of different sizes run from several threads
+at once."""
+import threading
+
+import numpy as np
 import pytest
 
 import kpax
@@ -45,3 +49,39 @@ def test_a_batch_plans_the_same_after_another_one_was_created(cuda, block):
     assert small.plan(b) == want[1]
     a.close()
     b.close()
+
+
+def test_swept_box_queries_of_two_grids_from_two_threads(cuda):
+    import torch
+
+    cfg = kpax.preset(kpax.PRESET_QUAD)
+    n, calls = 1 << 21, 3000  # from 2^21 boxes on the grid is held in shared memory, of the size that it needs
+    rng = np.random.default_rng(3)
+    lo = rng.uniform(0, 100, (n, 3)).astype(np.float32)
+    d_lo, d_hi = torch.from_numpy(lo).cuda(), torch.from_numpy(lo + np.float32(0.2)).cuda()
+    work = []
+    for obstacles in (500, 3000):
+        obs = torch.from_numpy(E.random_boxes(obstacles, seed=obstacles, side=(5.0, 8.0))).cuda()
+        env = kpax.Env(cfg, obs.data_ptr(), obstacles)
+        out = [torch.zeros(n, dtype=torch.uint8, device="cuda") for _ in range(2)]
+        kpax.collide_batch(env, d_lo.data_ptr(), d_hi.data_ptr(), n, out[0].data_ptr())
+        work.append((env, out, torch.cuda.Stream()))
+    torch.cuda.synchronize()
+    errors = []
+
+    def loop(env, out, stream):
+        try:
+            for _ in range(calls):
+                kpax.collide_batch(env, d_lo.data_ptr(), d_hi.data_ptr(), n, out[1].data_ptr(), stream.cuda_stream)
+        except kpax.KpaxError as e:
+            errors.append(str(e))
+
+    threads = [threading.Thread(target=loop, args=w) for w in work]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert not errors, errors
+    for _, out, _ in work:
+        assert torch.equal(out[0], out[1])
