@@ -35,9 +35,12 @@ __device__ __forceinline__ int box_cell(const Grid& g, const int c0[3], const in
     return x + g.dim * (y + g.dim * z);
 }
 
+// Cells of an obstacle's cell box: none when it is inverted in a dimension (the product of two negative
+// extents is positive, and box_cell would name cells outside the grid).
 __device__ __forceinline__ int box_cells(const int c0[3], const int c1[3])
 {
-    return (c1[0] - c0[0] + 1) * (c1[1] - c0[1] + 1) * (c1[2] - c0[2] + 1);
+    const int nx = c1[0] - c0[0] + 1, ny = c1[1] - c0[1] + 1, nz = c1[2] - c0[2] + 1;
+    return nx > 0 && ny > 0 && nz > 0 ? nx * ny * nz : 0;
 }
 
 // One warp per obstacle: pack n x 6 floats into float4 pairs and count (cell, obstacle) pairs.
@@ -159,13 +162,10 @@ __global__ void __launch_bounds__(kEnvBuildBS) k_env_build(Grid g, const float* 
             int c0[3], c1[3];
             obstacle_cells(g, lo, hi, c0, c1);
             const int total = box_cells(c0, c1);
-            for(int k = (int)(tid & 7u); k < total; k += 8) {
-                const uint32_t c = (uint32_t)box_cell(g, c0, c1, k);
-                if(c < cells) f(o, c);  // an inverted box can name cells outside the grid
-            }
+            for(int k = (int)(tid & 7u); k < total; k += 8) f(o, box_cell(g, c0, c1, k));
         }
     };
-    each_cell(true, [&](uint32_t, uint32_t c) { atomicAdd(s_cell + c, 1u); });
+    each_cell(true, [&](uint32_t, int c) { atomicAdd(s_cell + c, 1u); });
     __syncthreads();
     const uint32_t per = (cells + kEnvBuildBS - 1) / kEnvBuildBS | 1u;  // odd: no bank conflicts
     const uint32_t i0 = min(tid * per, cells), i1 = min(i0 + per, cells);
@@ -198,7 +198,7 @@ __global__ void __launch_bounds__(kEnvBuildBS) k_env_build(Grid g, const float* 
     if(tid == 0) off[cells] = total;
     if(total > cap) return;
     __syncthreads();
-    each_cell(false, [&](uint32_t o, uint32_t c) { ent[atomicAdd(s_cell + c, 1u)] = o; });
+    each_cell(false, [&](uint32_t o, int c) { ent[atomicAdd(s_cell + c, 1u)] = o; });
 }
 
 inline uint32_t warp_blocks(uint32_t n) { return (uint32_t)(((uint64_t)n * 32 + 255) / 256); }
