@@ -468,10 +468,11 @@ __global__ void __launch_bounds__(kCollideBS, 2) k_collide_shared(Grid g, uint32
         }
         return true;
     };
-    // a warp takes 32 consecutive boxes at a time, so that its lanes' corners share cache lines
-    for(uint32_t i = blockIdx.x * kCollideBS + threadIdx.x; i < n; i += gridDim.x * kCollideBS) {
-        const float lo[3] = {__ldcs(bbmin + 3 * (size_t)i), __ldcs(bbmin + 3 * (size_t)i + 1), __ldcs(bbmin + 3 * (size_t)i + 2)};
-        const float hi[3] = {__ldcs(bbmax + 3 * (size_t)i), __ldcs(bbmax + 3 * (size_t)i + 1), __ldcs(bbmax + 3 * (size_t)i + 2)};
+    // a warp takes 32 consecutive boxes at a time, so that its lanes' corners share cache lines; 64 bits,
+    // since the last stride may pass 2^32
+    for(size_t i = (size_t)blockIdx.x * kCollideBS + threadIdx.x; i < n; i += (size_t)gridDim.x * kCollideBS) {
+        const float lo[3] = {__ldcs(bbmin + 3 * i), __ldcs(bbmin + 3 * i + 1), __ldcs(bbmin + 3 * i + 2)};
+        const float hi[3] = {__ldcs(bbmax + 3 * i), __ldcs(bbmax + 3 * i + 1), __ldcs(bbmax + 3 * i + 2)};
         free_out[i] = query(lo, hi) ? 1 : 0;
     }
 }
