@@ -223,6 +223,7 @@ struct PlanBatch {
     int unroll = kGraphIters;
     uint32_t plans = 0;
     bool begun = false;
+    bool grids = false;  // every query's grid is complete: a begin that failed in between leaves none to read
     // single-query extras: debug capture and benchmark timing
     CaptureDev cap{};
     bool capture_on = false;
@@ -679,7 +680,7 @@ struct PlanBatch {
                 KPAX_CUDA(cudaMemsetAsync(d_prop_off, 0, sizeof(uint32_t) * (n_learned + 2), stream));
                 gx_prop_all = (uint32_t)std::max(1, per_sm) * (uint32_t)sms;
             }
-            if(begun)  // a plan in progress: occupancy of the current environments
+            if(begun && grids)  // a plan in progress: occupancy of the current environments
                 for(uint32_t q : sel) {
                     kpax_status st = launch_occupancy(prm[q], env[q].view(), const_cast<uint32_t*>(hq[q].occ), stream);
                     if(st != KPAX_OK) return st;
@@ -738,11 +739,13 @@ struct PlanBatch {
                       const uint32_t* n_obs, uint32_t max_iters, uint32_t stop, bool record_start = true)
     {
         if(!h_init || !h_goal) return set_error("plan: null start or goal"), KPAX_EINVAL;
+        for(uint32_t q = 0; q < nq; ++q)
+            if(n_obs[q] && !d_obstacles[q]) return set_error("plan: null obstacle buffer for query %u", q), KPAX_EINVAL;
+        grids = false;
         if(record_start) KPAX_CUDA(cudaEventRecord(ev0, stream));
         // the grids of all queries are counted, then one synchronisation sizes their entry lists
         bool counted = false;
         for(uint32_t q = 0; q < nq; ++q) {
-            if(n_obs[q] && !d_obstacles[q]) return set_error("plan: null obstacle buffer for query %u", q), KPAX_EINVAL;
             kpax_status st = env[q].build_start(prm[q], d_obstacles[q], n_obs[q], stream);
             if(st != KPAX_OK) return st;
             counted = counted || n_obs[q];
@@ -764,6 +767,7 @@ struct PlanBatch {
                 if(st != KPAX_OK) return st;
             }
         }
+        grids = true;
         kpax_status st = upload_descriptors();
         if(st != KPAX_OK) return st;
         k_begin<<<dim3(1, nq), 128, 0, stream>>>(dq, plans, max_iters, stop);
@@ -1033,7 +1037,7 @@ kpax_status kpax_plan_begin(kpax_planner* pl, const float* h_init, const float* 
 kpax_status kpax_plan_iterate(kpax_planner* pl, uint32_t n_iters, int32_t stop_at_goal)
 {
     return no_throw("kpax_plan_iterate", [&]() -> kpax_status {
-        if(!pl || !pl->b.begun) return set_error("kpax_plan_iterate: call kpax_plan_begin first"), KPAX_EINVAL;
+        if(!pl || !pl->b.begun || !pl->b.grids) return set_error("kpax_plan_iterate: call kpax_plan_begin first"), KPAX_EINVAL;
         if(!n_iters) return KPAX_OK;
         return pl->b.iterate(n_iters, stop_at_goal ? 1u : 0u);
     });
@@ -1043,7 +1047,7 @@ kpax_status kpax_plan_iterate_timed(kpax_planner* pl, uint32_t n_iters, uint64_t
                                     kpax_iter_timing* h_times, uint64_t* h_totals)
 {
     return no_throw("kpax_plan_iterate_timed", [&]() -> kpax_status {
-        if(!pl || !pl->b.begun) return set_error("kpax_plan_iterate_timed: call kpax_plan_begin first"), KPAX_EINVAL;
+        if(!pl || !pl->b.begun || !pl->b.grids) return set_error("kpax_plan_iterate_timed: call kpax_plan_begin first"), KPAX_EINVAL;
         return pl->b.iterate_timed(n_iters, flush_bytes, split != 0, h_times, h_totals);
     });
 }
