@@ -723,9 +723,18 @@ kpax_status kpax_mlp_forward(kpax_mlp* n, const float* d_x, uint32_t rows, float
 {
     if(!n || !d_x || !d_out || rows > n->max_batch) return set_error("kpax_mlp_forward: bad arguments"), KPAX_EINVAL;
     if(!rows) return KPAX_OK;
+    // a CTA writes its rows' outputs while others still read their inputs: buffers that overlap go through the
+    // net's own (kH floats a row)
+    static_assert(kOutPad <= kH, "outputs fit an activation buffer");
+    const uintptr_t x = (uintptr_t)d_x, o = (uintptr_t)d_out;
+    const size_t bytes = sizeof(float) * (size_t)rows * kOutPad;
+    const bool overlap = x < o + bytes && o < x + sizeof(float) * (size_t)rows * kInPad;
     RowArgs a{};
-    a.x = d_x, a.n = rows, a.w = n->w, a.wt = n->wt, a.out = d_out;
-    return launch_rows<false>(n, a, (cudaStream_t)stream);
+    a.x = d_x, a.n = rows, a.w = n->w, a.wt = n->wt, a.out = overlap ? n->a1 : d_out;
+    kpax_status s = launch_rows<false>(n, a, (cudaStream_t)stream);
+    if(s != KPAX_OK || !overlap) return s;
+    KPAX_CUDA(cudaMemcpyAsync(d_out, n->a1, bytes, cudaMemcpyDeviceToDevice, (cudaStream_t)stream));
+    return KPAX_OK;
 }
 
 kpax_status kpax_mlp_loss_grad(kpax_mlp* n, const float* d_x, const float* d_y, uint32_t rows, float* h_loss, float* d_grad,
