@@ -95,7 +95,7 @@ __device__ __forceinline__ void load_query_at(const QueryDev* __restrict__ qs, u
 }
 
 // Start of an iteration: the finish requests of the previous stages take effect.
-__global__ void __launch_bounds__(kBatchStartBS) k_batch_start(Ctl* __restrict__ ctls, uint32_t nq, uint32_t* __restrict__ active)
+static __global__ void __launch_bounds__(kBatchStartBS) k_batch_start(Ctl* __restrict__ ctls, uint32_t nq, uint32_t* __restrict__ active)
 {
     wait_predecessor();
     release_successor();
@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(kBatchStartBS) k_batch_start(Ctl* __restrict__
 
 // Frontier count over all queries: units are node tiles (k_frontier_count's tiles); the last tile
 // of a query scans its tile sums and sets its budget, or marks the query full.
-__global__ void __launch_bounds__(kFrontierBS) k_count_all(const QueryDev* __restrict__ qs,
+static __global__ void __launch_bounds__(kFrontierBS) k_count_all(const QueryDev* __restrict__ qs,
                                                                               const Ctl* __restrict__ ctls, uint32_t nq)
 {
     extern __shared__ uint32_t s_off[];
@@ -156,7 +156,7 @@ __global__ void __launch_bounds__(kFrontierBS) k_count_all(const QueryDev* __res
 }
 
 // Entry lists of all queries: units are node tiles of the queries that take entries.
-__global__ void __launch_bounds__(kFrontierBS) k_write_all(const QueryDev* __restrict__ qs, const Ctl* __restrict__ ctls,
+static __global__ void __launch_bounds__(kFrontierBS) k_write_all(const QueryDev* __restrict__ qs, const Ctl* __restrict__ ctls,
                                                           uint32_t nq)
 {
     extern __shared__ uint32_t s_off[];
@@ -191,18 +191,21 @@ __global__ void __launch_bounds__(kFrontierBS) k_write_all(const QueryDev* __res
 // so registers are traded for warps: 256-child tiles run two (quadrotor, 128 registers a thread) or
 // four (the 6-state models, 64) CTAs per SM.  96 mixed queries of 150 iterations on a B200: 157 ms, 159
 // with three CTAs of the 6-state models and 164 with five, 159 with three of the quadrotor and 178
-// with four, which spill 300 bytes in the step's loop.  Other tile sizes keep the single-query bound.
-template <int M, int BS>
-constexpr int kExpandAllMinBlocks = BS == 256 ? (M == KPAX_MODEL_QUADROTOR ? 2 : 4) : (512 / BS > 0 ? 512 / BS : 1);
+// with four, which spill 300 bytes in the step's loop.  A query per step (K == 1) waits more and keeps the
+// most warps, four and five CTAs.  Other tile sizes keep the single-query bound.
+template <int M, int BS, int K>
+constexpr int kExpandAllMinBlocks = BS != 256 ? (512 / BS > 0 ? 512 / BS : 1)
+                                    : K > 1   ? (M == KPAX_MODEL_QUADROTOR ? 2 : 4)
+                                              : (M == KPAX_MODEL_QUADROTOR ? 4 : 5);
 
-template <int M, int BS>
-__global__ void __launch_bounds__(BS, (kExpandAllMinBlocks<M, BS>)) k_expand_all(const QueryDev* __restrict__ qs,
+template <int M, int BS, int K>
+__global__ void __launch_bounds__(BS, (kExpandAllMinBlocks<M, BS, K>)) k_expand_all(const QueryDev* __restrict__ qs,
                                                                                 const Ctl* __restrict__ ctls,
                                                                                 const uint32_t* __restrict__ qidx,
                                                                                 uint32_t nq, uint32_t* __restrict__ active)
 {
     extern __shared__ __align__(16) float s_save[];  // kept states, then the offsets
-    uint32_t* s_off = reinterpret_cast<uint32_t*>(s_save + kSaveBytes<M, BS> / sizeof(float));
+    uint32_t* s_off = reinterpret_cast<uint32_t*>(s_save + kSaveBytes<M, BS, K> / sizeof(float));
     __shared__ QueryDev sq;
     __shared__ ExpandSmem<BS / 32> sm;
     __shared__ uint32_t s_warp[BS / 32];
@@ -219,7 +222,7 @@ __global__ void __launch_bounds__(BS, (kExpandAllMinBlocks<M, BS>)) k_expand_all
             n = sq.ctl->n, k = sq.ctl->k;
             cur = i;
         }
-        if(!expand_query_tiles<M, BS, kGroup, true>(sq, n, k, g - s_off[i], 0x80000000u, active, sm, s_save, true)) return;
+        if(!expand_query_tiles<M, BS, K, true>(sq, n, k, g - s_off[i], 0x80000000u, active, sm, s_save, true)) return;
     }
 }
 
@@ -234,7 +237,7 @@ __global__ void __launch_bounds__(BS, (512 / BS > 0 ? 512 / BS : 1)) k_expand_mi
                                                                                   uint32_t nq, uint32_t* __restrict__ active)
 {
     extern __shared__ __align__(16) float s_save[];  // kept states, then the offsets
-    uint32_t* s_off = reinterpret_cast<uint32_t*>(s_save + kSaveBytes<KPAX_MODEL_QUADROTOR, BS> / sizeof(float));
+    uint32_t* s_off = reinterpret_cast<uint32_t*>(s_save + kSaveBytes<KPAX_MODEL_QUADROTOR, BS, kGroup> / sizeof(float));
     __shared__ QueryDev sq;
     __shared__ ExpandSmem<BS / 32> sm;
     __shared__ uint32_t s_warp[BS / 32];
@@ -268,7 +271,7 @@ constexpr int kScoreUnitWarps = kScoreBS / 32;  // partial sums per score unit
 // Region scores of all queries: a unit is kScoreUnitWarps consecutive partial sums of one query (and
 // its share of the R2 snapshot copy); the query's last unit adds the partials and closes its
 // iteration.
-__global__ void __launch_bounds__(kScoreBS) k_scores_all(const QueryDev* __restrict__ qs, const Ctl* __restrict__ ctls,
+static __global__ void __launch_bounds__(kScoreBS) k_scores_all(const QueryDev* __restrict__ qs, const Ctl* __restrict__ ctls,
                                                         uint32_t nq, uint32_t* __restrict__ active)
 {
     extern __shared__ uint32_t s_off[];
@@ -340,7 +343,7 @@ struct BatchEntrySrc {
 // the learned queries before j, off[nl] = all; a query that has finished, or takes no entries
 // this iteration, has none.
 constexpr int kPropTilesBS = 1024;
-__global__ void __launch_bounds__(kPropTilesBS) k_propose_tiles(const QueryDev* __restrict__ qs, const uint32_t* __restrict__ qidx,
+static __global__ void __launch_bounds__(kPropTilesBS) k_propose_tiles(const QueryDev* __restrict__ qs, const uint32_t* __restrict__ qidx,
                                                                 uint32_t nl, uint32_t* __restrict__ off)
 {
     constexpr int kPer = (kBatchMaxQueries + kPropTilesBS - 1) / kPropTilesBS;
@@ -379,7 +382,7 @@ __global__ void __launch_bounds__(kPropTilesBS) k_propose_tiles(const QueryDev* 
     }
 }
 
-__global__ void __launch_bounds__(mlp::tc::kThreads, 1) k_propose_all(const QueryDev* __restrict__ qs, const uint32_t* __restrict__ qidx,
+static __global__ void __launch_bounds__(mlp::tc::kThreads, 1) k_propose_all(const QueryDev* __restrict__ qs, const uint32_t* __restrict__ qidx,
                                                                        uint32_t nl, const uint32_t* __restrict__ off, uint32_t* __restrict__ err)
 {
     extern __shared__ __align__(1024) uint8_t smem[];

@@ -363,6 +363,23 @@ __device__ __forceinline__ bool box_free(const Grid& g, const float lo[3], const
                           grid_coord(g, hi[1]), grid_coord(g, hi[2]));
 }
 
+// The swept box of one step, p0 -> p1.  cells: the cell coordinates of p0 on entry, replaced by p1's (a
+// step's end is the next one's start).  The cell map is non-decreasing, so the box's cells are the range of
+// its two corners' cells.
+__device__ __forceinline__ bool step_free(const Grid& g, const float p0[3], const float p1[3], int cells[3])
+{
+    float lo[3], hi[3];
+    int c0[3], c1[3];
+#pragma unroll
+    for(int d = 0; d < 3; ++d) {
+        lo[d] = fminf(p0[d], p1[d]), hi[d] = fmaxf(p0[d], p1[d]);
+        const int c = grid_coord(g, p1[d]);
+        c0[d] = min(cells[d], c), c1[d] = max(cells[d], c);
+        cells[d] = c;
+    }
+    return box_free_cells(g, lo, hi, c0[0], c0[1], c0[2], c1[0], c1[1], c1[2]);
+}
+
 // First of `limit` consecutive swept boxes, box j from pos(j) to pos(j + 1), that an obstacle
 // overlaps, or `limit` when all are free.  lo / hi: the hull of the boxes.  One walk over the cells
 // of the hull finds the obstacles that overlap it, and only those are tested against the boxes, so
@@ -709,18 +726,6 @@ struct ModelDims<KPAX_MODEL_QUADROTOR> {
     static constexpr int SD = 12, CD = 4;
 };
 
-// Runs a segment from step `done` up to step `end` (in place), checking every step like the
-// reference; returns false when a step fails, and leaves the number of steps executed (the failing
-// one included) in `done`.  Steps are taken in groups of up to K: the group is integrated with the
-// bounds checks only, each step's state kept in `save`, then one walk over the obstacles near the
-// group's hull finds its first colliding step (first_hit), and a segment that collides takes the
-// state after that step back from `save`.  The lookups of a query are a chain of dependent loads
-// walked at the pace of the warp's slowest lane, so the fewer walks the better; K is bounded by the
-// shared memory of the states.  B200, groups of five against a query per step: expansion of 2^16
-// quadrotor children in the building scene 83.2 -> 67.3 us, 2^14 children 67 -> 57 us, Dubins in the
-// forest 27.0 -> 22.7 us; 2^22 Dubins segments 848 -> 672 us; the double integrator, whose expansion
-// is mostly its fixed part, 18 us either way.  save: this thread's SD floats of the first
-// step of the block's K x `threads` x SD (a warp's 16- or 8-byte accesses to them are conflict-free).
 template <int SD>
 __device__ __forceinline__ void save_state(float* dst, const float* s)
 {
@@ -752,11 +757,35 @@ __device__ __forceinline__ void take_state(const float* src, float* s)
     }
 }
 
+// Runs a segment from step `done` up to step `end` (in place), checking every step like the
+// reference; returns false when a step fails, and leaves the number of steps executed (the failing
+// one included) in `done`.
+//
+// K > 1: steps are taken in groups of up to K.  The group is integrated with the bounds checks only, each
+// step's state kept in `save`, then one walk over the obstacles near the group's hull finds its first
+// colliding step (first_hit), and a segment that collides takes the state after that step back from
+// `save`.  The lookups of a query are a chain of dependent loads walked at the pace of the warp's slowest
+// lane, so the fewer walks the better; K is bounded by the shared memory of the states.  B200, groups of
+// five against a query per step: expansion of 2^16 quadrotor children in the building scene 83.2 -> 67.3
+// us, 2^14 children 67 -> 57 us, Dubins in the forest 27.0 -> 22.7 us; 2^22 Dubins segments 848 -> 672 us;
+// the double integrator, whose expansion is mostly its fixed part, 18 us either way.  save: this thread's
+// SD floats of the first step of the block's K x `threads` x SD (a warp's 16- or 8-byte accesses to them
+// are conflict-free).
+// K == 1: a query per step, nothing kept (save is not used): see grouped().
 template <int M, int K, class C>
 __device__ __forceinline__ bool run_steps(const StepParams& p, const Grid& g, float* s, const float* c, const C& k, int end,
                                           int& done, float* save, int threads)
 {
     constexpr int SD = ModelDims<M>::SD;
+    if constexpr(K == 1) {
+        int cells[3] = {grid_coord(g, s[0]), grid_coord(g, s[1]), grid_coord(g, s[2])};
+        while(done < end) {
+            const float p0[3] = {s[0], s[1], s[2]};
+            ++done;
+            if(!model_step<M>(p, s, c, k) || !step_free(g, p0, s, cells)) return false;
+        }
+        return true;
+    }
     const int stride = threads * SD;
     while(done < end) {
         const int m = min(K, end - done);

@@ -208,21 +208,24 @@ inline uint32_t warp_blocks(uint32_t n) { return (uint32_t)(((uint64_t)n * 32 + 
 // CTAs of the batch kernels: 256 threads, four per SM (64 registers), for the 6-state models; the
 // quadrotor's step keeps over 100 values, and at 64 registers its spills cost more than the warps
 // gain (30011 segments in the building scene 70 us spilling, 53 us at 128 registers; 2^20 555 -> 448 us).
-// kBatchGroup: steps per collision query (run_steps), whose kept states must stay below the
-// 48 KB of static shared memory.
-template <int M>
-constexpr int kBatchBS = M == KPAX_MODEL_QUADROTOR ? 128 : 256;
+// With a query per step (K == 1) the waits for lookups prevail: 2^19 of 0.4 s steps 413 us at 64 registers,
+// 506 at 128.
+// The kept states of a group (kSaveFloats) stay below the 48 KB of static shared memory.
+template <int M, int K>
+constexpr int kBatchBS = M == KPAX_MODEL_QUADROTOR && K > 1 ? 128 : 256;
 constexpr int kBatchBlocks = 4;
-constexpr int kBatchGroup = 5;
+template <int M, int BS, int K>
+constexpr int kSaveFloats = K > 1 ? K * ModelDims<M>::SD * BS : 4;
 
-template <int M>
-__global__ void __launch_bounds__(kBatchBS<M>, kBatchBlocks) k_propagate_batch(KParams p, Grid g, const float* __restrict__ parents,
+template <int M, int K>
+__global__ void __launch_bounds__((kBatchBS<M, K>), kBatchBlocks) k_propagate_batch(KParams p, Grid g, const float* __restrict__ parents,
                                                          const float* __restrict__ draws, uint32_t stream_id, uint32_t n,
                                                          float* __restrict__ rows, uint8_t* __restrict__ valid,
                                                          int32_t* __restrict__ steps_out)
 {
     constexpr int SD = ModelDims<M>::SD, CD = ModelDims<M>::CD, S = SD + CD + 1;
-    __shared__ __align__(16) float s_save[kBatchGroup * SD * kBatchBS<M>];
+    constexpr int BS = kBatchBS<M, K>;
+    __shared__ __align__(16) float s_save[kSaveFloats<M, BS, K>];
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if(i >= n) return;
     float s[SD], u[6], c[4], rc[4];
@@ -237,7 +240,7 @@ __global__ void __launch_bounds__(kBatchBS<M>, kBatchBlocks) k_propagate_batch(K
     }
     const int steps = draw_controls(p, u, c);
     int done = 0;
-    const bool ok = propagate<M, kBatchGroup>(p, g, s, c, steps, done, s_save + threadIdx.x * SD, kBatchBS<M>);
+    const bool ok = propagate<M, K>(p, g, s, c, steps, done, s_save + threadIdx.x * SD, BS);
     row_controls<M>(c, rc);
     float* dst = rows + (size_t)i * S;
 #pragma unroll
@@ -260,21 +263,27 @@ __global__ void __launch_bounds__(kBatchBS<M>, kBatchBlocks) k_propagate_batch(K
 // gains by dropping its dead sooner.  B200, us, one pass / head of 2 / of 5 / of 2 and a middle phase:
 // Dubins 2^22, 200 obstacles 615 / 625 / 579 / 639, 1500 obstacles 859 / 637 / 633 / 656;
 // quadrotor 2^21, 200 obstacles 1302 / 1191 / 1173 / 1201, 2000 obstacles 1418 / 582 / 661 / 579.
-template <int M>
-constexpr int kHeadSteps = M == KPAX_MODEL_QUADROTOR ? 2 : kBatchGroup;
+template <int M, int K>
+constexpr int kHeadSteps = M == KPAX_MODEL_QUADROTOR || K == 1 ? 2 : K;
 // The phases need a few waves of CTAs to fill the chip twice (one pass / two phases, us: Dubins 2^18, 200
 // obstacles 58 / 66, 2^19 93 / 96, with 1500 obstacles 130 / 113; quadrotor 2^18, 200 obstacles 181 / 182,
 // with 2000 208 / 125), and segments of more than two query groups: those of ten steps leave the tail
-// too little (double integrator 2^22, 20 obstacles 235 / 266, 200 obstacles 263 / 291).
-template <int M>
-constexpr uint32_t kPhasedMin = 2048u * kBatchBS<M>;
-template <int M>
+// too little (double integrator 2^22, 20 obstacles 235 / 266, 200 obstacles 263 / 291).  With a query per
+// step the quadrotor's steps are worth it from ten on (quad-ref, 200 obstacles, one pass / phases: 2^18
+// 91 / 94, 2^19 169 / 140, 2^21 638 / 466).
+template <int M, int K>
+constexpr uint32_t kPhasedMin = K > 1 ? 2048u * kBatchBS<M, K> : 1u << 18;
+template <int M, int K>
 inline bool phased(const KParams& p, uint32_t n)
 {
-    return n >= kPhasedMin<M> && p.nsteps > 2 * kBatchGroup;
+    return n >= kPhasedMin<M, K> && (p.nsteps > 2 * kGroup || (K == 1 && M == KPAX_MODEL_QUADROTOR));
 }
-// Segments per round of the two phases (bounds the survivor list's scratch).  Each round pays the
-// latency of its longest segment in both phases, so rounds are as large as the scratch allows.
+// With a query per step a middle phase up to 3/5 of the longest segment keeps the tail's lanes full at no
+// further query (quadrotor steps of 0.4 s, 2^21, no obstacles 1482 us without it, 1248 with it).
+template <int K>
+constexpr bool kMiddle = K == 1;
+// Segments per round of the phases (bounds the survivor lists' scratch).  Each round pays the
+// latency of its longest segment in every phase, so rounds are as large as the scratch allows.
 constexpr uint32_t kPhaseChunk = 1u << 24;
 
 struct LiveList {
@@ -284,6 +293,7 @@ struct LiveList {
     float* ctl;      // CD per entry
     float* state;    // SD per entry
 };
+constexpr size_t kCountBytes = 256;  // the counts of both lists, 128 bytes apart
 
 template <int M>
 __device__ __forceinline__ void write_segment(const KParams& p, uint32_t i, const float* s, const float* c, int steps, bool ok,
@@ -327,14 +337,15 @@ __device__ __forceinline__ void append_live(const LiveList& live, bool alive, in
 
 // Segments i of one round (pointers offset to the round's first segment; i0 = that segment's index
 // in the batch, which keys its draws).
-template <int M>
-__global__ void __launch_bounds__(kBatchBS<M>, kBatchBlocks) k_propagate_head(KParams p, Grid g, const float* __restrict__ parents,
+template <int M, int K>
+__global__ void __launch_bounds__((kBatchBS<M, K>), kBatchBlocks) k_propagate_head(KParams p, Grid g, const float* __restrict__ parents,
                                                         const float* __restrict__ draws, uint32_t stream_id, uint32_t n,
                                                         uint32_t i0, float* __restrict__ rows, uint8_t* __restrict__ valid,
                                                         int32_t* __restrict__ steps_out, LiveList live)
 {
     constexpr int SD = ModelDims<M>::SD, CD = ModelDims<M>::CD;
-    __shared__ __align__(16) float s_save[kHeadSteps<M> * SD * kBatchBS<M>];
+    constexpr int BS = kBatchBS<M, K>, kHead = kHeadSteps<M, K>, kQuery = K > 1 ? kHead : 1;
+    __shared__ __align__(16) float s_save[kSaveFloats<M, BS, kQuery>];
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     const int lane = threadIdx.x & 31;
     bool alive = false;
@@ -355,53 +366,66 @@ __global__ void __launch_bounds__(kBatchBS<M>, kBatchBlocks) k_propagate_head(KP
         const auto k = segment_consts<M>(p, c);
         const StepParams sp = step_params(p);
         int done = 0;
-        const bool ok = run_steps<M, kHeadSteps<M>>(sp, g, s, c, k, min(steps, kHeadSteps<M>), done, s_save + threadIdx.x * SD,
-                                                    kBatchBS<M>);
+        const bool ok = run_steps<M, kQuery>(sp, g, s, c, k, min(steps, kHead), done, s_save + threadIdx.x * SD, BS);
         alive = ok && done < steps;
         if(!alive) write_segment<M>(p, i, s, c, steps, ok, done, rows, valid, steps_out);
     }
     append_live<SD, CD>(live, alive, lane, i, steps, c, s);
 }
 
-template <int M>
-__global__ void __launch_bounds__(kBatchBS<M>, kBatchBlocks) k_propagate_tail(KParams p, Grid g, float* __restrict__ rows,
+// Segments of `live` from step `from` on: to their end (kLast), or to step `until` with those that go on
+// appended to `next`.
+template <int M, int K, bool kLast>
+__global__ void __launch_bounds__((kBatchBS<M, K>), kBatchBlocks) k_propagate_tail(KParams p, Grid g, float* __restrict__ rows,
                                                         uint8_t* __restrict__ valid, int32_t* __restrict__ steps_out,
-                                                        LiveList live)
+                                                        LiveList live, int from, int until, LiveList next)
 {
     constexpr int SD = ModelDims<M>::SD, CD = ModelDims<M>::CD;
-    __shared__ __align__(16) float s_save[kBatchGroup * SD * kBatchBS<M>];
-    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-    if(j >= *live.count) return;
-    const uint32_t i = live.idx[j];
-    const int steps = live.steps ? live.steps[j] : p.nsteps;
+    constexpr int BS = kBatchBS<M, K>;
+    __shared__ __align__(16) float s_save[kSaveFloats<M, BS, K>];
+    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x, count = *live.count;
+    if(kLast ? j >= count : blockIdx.x * blockDim.x >= count) return;  // appends need whole warps
+    const bool in = kLast || j < count;
+    const uint32_t e = in ? j : 0u;
+    const uint32_t i = live.idx[e];
+    const int steps = live.steps ? live.steps[e] : p.nsteps;
     float s[SD], c[4];
 #pragma unroll
-    for(int k = 0; k < 4; ++k) c[k] = k < CD ? live.ctl[(size_t)j * CD + k] : 0.0f;
+    for(int k = 0; k < 4; ++k) c[k] = k < CD ? live.ctl[(size_t)e * CD + k] : 0.0f;
 #pragma unroll
-    for(int k = 0; k < SD; ++k) s[k] = live.state[(size_t)j * SD + k];
+    for(int k = 0; k < SD; ++k) s[k] = live.state[(size_t)e * SD + k];
     const auto kc = segment_consts<M>(p, c);
     const StepParams sp = step_params(p);
-    int done = kHeadSteps<M>;
-    const bool ok = run_steps<M, kBatchGroup>(sp, g, s, c, kc, steps, done, s_save + threadIdx.x * SD, kBatchBS<M>);
-    write_segment<M>(p, i, s, c, steps, ok, done, rows, valid, steps_out);
+    int done = from;
+    const int end = kLast ? steps : in ? min(steps, until) : 0;
+    const bool ok = run_steps<M, K>(sp, g, s, c, kc, end, done, s_save + threadIdx.x * SD, BS);
+    const bool alive = !kLast && in && ok && done < steps;
+    if(in && !alive) write_segment<M>(p, i, s, c, steps, ok, done, rows, valid, steps_out);
+    if constexpr(!kLast) append_live<SD, CD>(next, alive, threadIdx.x & 31, i, steps, c, s);
 }
 
-// The two phases over rounds of kPhaseChunk segments; the list's count is cleared before every round.
-template <int M>
+// The phases over rounds of kPhaseChunk segments; the lists' counts are cleared before every round.
+template <int M, int K>
 void launch_phases(const KParams& p, const Grid& g, const float* parents, const float* draws, uint32_t stream_id, uint32_t n,
-                   float* rows, uint8_t* valid, int32_t* steps_out, const LiveList& live, cudaStream_t s)
+                   float* rows, uint8_t* valid, int32_t* steps_out, const LiveList& live, const LiveList& second, cudaStream_t s)
 {
     const int SD = p.sd, S = p.S;
     for(uint32_t o = 0; o < n; o += kPhaseChunk) {
-        const uint32_t m = std::min(kPhaseChunk, n - o), bs = kBatchBS<M>, blocks = (m + bs - 1) / bs;
+        const uint32_t m = std::min(kPhaseChunk, n - o), bs = kBatchBS<M, K>, blocks = (m + bs - 1) / bs;
         float* r = rows + (size_t)o * S;
         uint8_t* v = valid + o;
         int32_t* st = steps_out ? steps_out + o : nullptr;
-        cudaMemsetAsync(live.count, 0, sizeof(uint32_t), s);
-        k_propagate_head<M><<<blocks, bs, 0, s>>>(p, g, parents + (size_t)o * SD, draws ? draws + (size_t)o * 5 : nullptr,
+        int from = kHeadSteps<M, K>;
+        cudaMemsetAsync(live.count, 0, kCountBytes, s);
+        k_propagate_head<M, K><<<blocks, bs, 0, s>>>(p, g, parents + (size_t)o * SD, draws ? draws + (size_t)o * 5 : nullptr,
                                                    stream_id, m, o, r, v, st, live);
-        k_propagate_tail<M><<<blocks, bs, 0, s>>>(p, g, r, v, st, live);
-        count_launch(2);
+        if constexpr(kMiddle<K>) {
+            const int until = std::max(from + 1, p.nsteps * 3 / 5);
+            k_propagate_tail<M, K, false><<<blocks, bs, 0, s>>>(p, g, r, v, st, live, from, until, second);
+            from = until;
+        }
+        k_propagate_tail<M, K, true><<<blocks, bs, 0, s>>>(p, g, r, v, st, kMiddle<K> ? second : live, from, 0, LiveList{});
+        count_launch(kMiddle<K> ? 3 : 2);
     }
 }
 
@@ -592,14 +616,11 @@ kpax_status launch_propagate(const KParams& p, const Grid& g, const float* paren
                              uint32_t n, float* rows, uint8_t* valid, int32_t* steps, cudaStream_t stream)
 {
     if(!n) return KPAX_OK;
-    auto go = [&](auto kernel, uint32_t bs) {
-        kernel<<<(n + bs - 1) / bs, bs, 0, stream>>>(p, g, parents, draws, stream_id, n, rows, valid, steps);
-    };
-    switch(p.model) {
-        case KPAX_MODEL_DOUBLE_INTEGRATOR: go(k_propagate_batch<KPAX_MODEL_DOUBLE_INTEGRATOR>, kBatchBS<KPAX_MODEL_DOUBLE_INTEGRATOR>); break;
-        case KPAX_MODEL_DUBINS_AIRPLANE: go(k_propagate_batch<KPAX_MODEL_DUBINS_AIRPLANE>, kBatchBS<KPAX_MODEL_DUBINS_AIRPLANE>); break;
-        default: go(k_propagate_batch<KPAX_MODEL_QUADROTOR>, kBatchBS<KPAX_MODEL_QUADROTOR>); break;
-    }
+    by_model(p.model, grouped(p) ? kGroup : 1, [&](auto m, auto k) {
+        constexpr int M = decltype(m)::value, K = decltype(k)::value;
+        constexpr uint32_t bs = kBatchBS<M, K>;
+        k_propagate_batch<M, K><<<(n + bs - 1) / bs, bs, 0, stream>>>(p, g, parents, draws, stream_id, n, rows, valid, steps);
+    });
     KPAX_CHECK_LAUNCH();
     count_launch();
     return KPAX_OK;
@@ -724,41 +745,35 @@ kpax_status kpax_propagate_batch(const kpax_config* cfg, kpax_env* env, const fl
     if(st != KPAX_OK) return st;
     if(p.gdim != env->env.dim || p.cell != env->env.cell || p.wmin != env->env.wmin)
         return set_error("kpax_propagate_batch: env was built for another workspace grid"), KPAX_EINVAL;
-    const bool two = p.model == KPAX_MODEL_DOUBLE_INTEGRATOR ? phased<KPAX_MODEL_DOUBLE_INTEGRATOR>(p, n)
-                     : p.model == KPAX_MODEL_DUBINS_AIRPLANE ? phased<KPAX_MODEL_DUBINS_AIRPLANE>(p, n)
-                                                             : phased<KPAX_MODEL_QUADROTOR>(p, n);
+    const int group = grouped(p) ? kGroup : 1;
+    const bool two = by_model(p.model, group, [&](auto m, auto k) { return phased<decltype(m)::value, decltype(k)::value>(p, n); });
     if(!two)
         return launch_propagate(p, env->env.view(), d_parents, d_draws, draw_stream, n, d_rows, d_valid, d_steps,
                                 (cudaStream_t)stream);
-    // phases: the live list of a round lives in the env's scratch, grown on demand (its count, then its
-    // index, step-count (drawn durations only), control and state arrays)
+    // phases: the live lists of a round live in the env's scratch, grown on demand (their counts, then each
+    // list's index, step-count (drawn durations only), control and state arrays)
     Env& e = env->env;
     auto align = [](size_t b) { return (b + 255) / 256 * 256; };
     const size_t m = std::min(n, kPhaseChunk);
-    const size_t l_idx = 256, l_steps = l_idx + align(4ull * m), l_ctl = l_steps + (p.fixed_steps ? 0 : align(4ull * m)),
-                 l_state = l_ctl + align(4ull * p.cd * m), bytes = l_state + align(4ull * p.sd * m);
+    const size_t l_steps = align(4ull * m), l_ctl = l_steps + (p.fixed_steps ? 0 : align(4ull * m)),
+                 l_state = l_ctl + align(4ull * p.cd * m), l_bytes = l_state + align(4ull * p.sd * m);
+    const size_t bytes = kCountBytes + (group == 1 && kMiddle<1> ? 2 : 1) * l_bytes;
     if(bytes > e.live_cap) {
         if(e.d_live) cudaFree(e.d_live), e.d_live = nullptr, e.live_cap = 0;
         KPAX_CUDA(cudaMalloc(&e.d_live, bytes));
         e.live_cap = bytes;
     }
-    char* l = static_cast<char*>(e.d_live);
-    const LiveList live{reinterpret_cast<uint32_t*>(l), reinterpret_cast<uint32_t*>(l + l_idx),
+    auto list = [&](int k) {
+        char *count = static_cast<char*>(e.d_live) + 128 * k, *l = static_cast<char*>(e.d_live) + kCountBytes + k * l_bytes;
+        return LiveList{reinterpret_cast<uint32_t*>(count), reinterpret_cast<uint32_t*>(l),
                         p.fixed_steps ? nullptr : reinterpret_cast<int32_t*>(l + l_steps), reinterpret_cast<float*>(l + l_ctl),
                         reinterpret_cast<float*>(l + l_state)};
+    };
     cudaStream_t s = (cudaStream_t)stream;
     const Grid g = e.view();
-    switch(p.model) {
-        case KPAX_MODEL_DOUBLE_INTEGRATOR:
-            launch_phases<KPAX_MODEL_DOUBLE_INTEGRATOR>(p, g, d_parents, d_draws, draw_stream, n, d_rows, d_valid, d_steps, live, s);
-            break;
-        case KPAX_MODEL_DUBINS_AIRPLANE:
-            launch_phases<KPAX_MODEL_DUBINS_AIRPLANE>(p, g, d_parents, d_draws, draw_stream, n, d_rows, d_valid, d_steps, live, s);
-            break;
-        default:
-            launch_phases<KPAX_MODEL_QUADROTOR>(p, g, d_parents, d_draws, draw_stream, n, d_rows, d_valid, d_steps, live, s);
-            break;
-    }
+    by_model(p.model, group, [&](auto m, auto k) {
+        launch_phases<decltype(m)::value, decltype(k)::value>(p, g, d_parents, d_draws, draw_stream, n, d_rows, d_valid, d_steps, list(0), list(1), s);
+    });
     KPAX_CHECK_LAUNCH();
     return KPAX_OK;
 }

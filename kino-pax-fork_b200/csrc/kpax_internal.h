@@ -7,6 +7,7 @@
 #include <atomic>
 #include <exception>
 #include <new>
+#include <type_traits>
 
 #include "kpax_device.cuh"
 #include "kpax_params.h"
@@ -52,6 +53,20 @@ kpax_status no_throw(const char* what, F&& f)
 }  // namespace kpax
 
 namespace kpax {
+
+// f(model, steps per query) with both as compile-time constants (run_steps): model a KPAX_MODEL_*, group
+// kGroup or 1.
+template <class F>
+auto by_model(int model, int group, F&& f)
+{
+    using std::integral_constant;
+    auto of = [&](auto m) {
+        return group > 1 ? f(m, integral_constant<int, kGroup>{}) : f(m, integral_constant<int, 1>{});
+    };
+    return model == KPAX_MODEL_DOUBLE_INTEGRATOR ? of(integral_constant<int, KPAX_MODEL_DOUBLE_INTEGRATOR>{})
+           : model == KPAX_MODEL_DUBINS_AIRPLANE ? of(integral_constant<int, KPAX_MODEL_DUBINS_AIRPLANE>{})
+                                                 : of(integral_constant<int, KPAX_MODEL_QUADROTOR>{});
+}
 
 extern std::atomic<uint64_t> g_launches;
 inline void count_launch(uint64_t n = 1) { g_launches.fetch_add(n, std::memory_order_relaxed); }

@@ -250,7 +250,7 @@ __device__ __forceinline__ float goal_distance(const float* s, const float* g)
 // ---------------------------------------------------------------- kernels
 
 // Root node and control block of each query (KPAX.cu:59-91).
-__global__ void k_begin(const QueryDev* __restrict__ qs, uint32_t plan_base, uint32_t max_iters, uint32_t stop_at_goal)
+static __global__ void k_begin(const QueryDev* __restrict__ qs, uint32_t plan_base, uint32_t max_iters, uint32_t stop_at_goal)
 {
     __shared__ QueryDev sq;
     load_query(qs, nullptr, sq);
@@ -408,7 +408,7 @@ __device__ __forceinline__ void set_budget(const KParams& p, Ctl* ctl, uint64_t 
     ctl->k = k, ctl->E = E, ctl->n = n;
 }
 
-__global__ void __launch_bounds__(kFrontierBS, kFrontierMinBlocks) k_frontier_count(const QueryDev* __restrict__ qs, uint32_t* __restrict__ active)
+static __global__ void __launch_bounds__(kFrontierBS, kFrontierMinBlocks) k_frontier_count(const QueryDev* __restrict__ qs, uint32_t* __restrict__ active)
 {
     __shared__ QueryDev sq;
     __shared__ uint32_t s_last, s_carry;
@@ -492,7 +492,7 @@ __device__ __forceinline__ void write_tile(const QueryDev& sq, uint32_t b, uint3
 // Node i owns virtual entries [a, a + rep) with a from the tile scan.  Entry j of the E taken is
 // virtual entry floor(j*R/E): node i writes entries ceil(a*E/R) .. ceil((a+rep)*E/R) - 1 (all of
 // its entries when E == R).  Nodes with an entry taken leave the frontier.
-__global__ void __launch_bounds__(kFrontierBS) k_frontier_write(const QueryDev* __restrict__ qs)
+static __global__ void __launch_bounds__(kFrontierBS) k_frontier_write(const QueryDev* __restrict__ qs)
 {
     __shared__ QueryDev sq;
     __shared__ uint32_t s_warp[kFrontierBS / 32];
@@ -605,12 +605,9 @@ struct ExpandSmem {
     GatherSmem<NW> gs;
 };
 
-// Steps per collision query (run_steps) of the single-query expansions: 5 divides the presets' 10, 20
-// and 25 steps, and the kept states (120 KB of shared memory at 512 quadrotor children per SM) leave
-// the grid over 100 KB of L1.
-constexpr int kGroup = 5;
-template <int M, int BS, int K = kGroup>
-constexpr size_t kSaveBytes = sizeof(float) * K * ModelDims<M>::SD * BS;
+// Shared memory of the kept states of a block of BS children (run_steps with groups of K).
+template <int M, int BS, int K>
+constexpr size_t kSaveBytes = K > 1 ? sizeof(float) * K * ModelDims<M>::SD * BS : 0;
 
 // The control-block values an expansion reads, and what a block's tiles add up to (thread 0).
 struct ExpandState {
@@ -637,7 +634,7 @@ struct ExpandTotals {
 // receives the children appended by all CTAs.
 // kOne: the caller takes exactly one tile per call.  Returns false when a wait gave up.  save:
 // kSaveBytes<M, BS, K> bytes of shared memory.
-template <int M, int BS, int K = kGroup, bool kOne = false>
+template <int M, int BS, int K, bool kOne = false>
 __device__ __forceinline__ bool expand_tiles(QueryDev& sq, const ExpandState st, uint32_t n, uint32_t k, uint32_t first,
                                              uint32_t stride, ExpandSmem<BS / 32>& sm, float* save, ExpandTotals& tot,
                                              const unsigned long long* entry_words = nullptr,
@@ -767,7 +764,7 @@ __device__ __forceinline__ bool expand_tiles(QueryDev& sq, const ExpandState st,
 
 // The per-stage and batch expansions: state from the control block, counters added to it, a wait
 // that gave up finishes the query with an error.
-template <int M, int BS, int K = kGroup, bool kOne = false>
+template <int M, int BS, int K, bool kOne = false>
 __device__ __forceinline__ bool expand_query_tiles(QueryDev& sq, uint32_t n, uint32_t k, uint32_t first, uint32_t stride,
                                                    uint32_t* __restrict__ active, ExpandSmem<BS / 32>& sm, float* save,
                                                    bool defer_finish = false)
@@ -790,7 +787,7 @@ __device__ __forceinline__ bool expand_query_tiles(QueryDev& sq, uint32_t n, uin
 
 // Expansion kernel of a batch: the children of query blockIdx.y (through qidx), tiles in grid-stride
 // rounds over blockIdx.x.
-template <int M, int BS>
+template <int M, int BS, int K>
 __global__ void __launch_bounds__(BS, (512 / BS > 0 ? 512 / BS : 1)) k_expand(const QueryDev* __restrict__ qs, const uint32_t* __restrict__ qidx,
                                                uint32_t* __restrict__ active)
 {
@@ -801,7 +798,7 @@ __global__ void __launch_bounds__(BS, (512 / BS > 0 ? 512 / BS : 1)) k_expand(co
     wait_predecessor();
     release_successor();
     if(__syncthreads_or(sq.ctl->done != 0u)) return;  // one decision for the whole block: barriers follow
-    expand_query_tiles<M, BS>(sq, sq.ctl->n, sq.ctl->k, blockIdx.x, gridDim.x, active, sm, s_save);
+    expand_query_tiles<M, BS, K>(sq, sq.ctl->n, sq.ctl->k, blockIdx.x, gridDim.x, active, sm, s_save);
 }
 
 // Region scores (Graph.cu:233-358): one warp per partial sum j; the warp scores groups of 32
@@ -925,7 +922,7 @@ __device__ __forceinline__ void score_finish(const QueryDev& sq, uint32_t* __res
 }
 
 // The score pass of a batch: query blockIdx.y; the last CTA of a query adds its partials.
-__global__ void __launch_bounds__(kScoreBS) k_scores(const QueryDev* __restrict__ qs, uint32_t* __restrict__ active)
+static __global__ void __launch_bounds__(kScoreBS) k_scores(const QueryDev* __restrict__ qs, uint32_t* __restrict__ active)
 {
     __shared__ QueryDev sq;
     __shared__ uint32_t s_last;
@@ -983,7 +980,7 @@ struct IterState {
     unsigned long long n_exp;
 };
 
-template <int M, int BS, int PART = kIterWhole>
+template <int M, int BS, int PART, int K>
 __global__ void __launch_bounds__(BS, (512 / BS > 0 ? 512 / BS : 1)) k_iterate(const QueryDev* __restrict__ qs,
                                                                              const Ctl* ctl_line,
                                                                              uint32_t* __restrict__ active,
@@ -1142,10 +1139,10 @@ __global__ void __launch_bounds__(BS, (512 / BS > 0 ? 512 / BS : 1)) k_iterate(c
         uint32_t appended = 0;
         bool ok;
         if((uint64_t)n <= (uint64_t)G * BS) {
-            ok = expand_tiles<M, BS>(sq, st, n, k, cb, G, sm, s_save, tot, w_entries, w_children, &appended);
+            ok = expand_tiles<M, BS, K>(sq, st, n, k, cb, G, sm, s_save, tot, w_entries, w_children, &appended);
         } else {
             const uint32_t before = tot.accepted;
-            ok = expand_tiles<M, BS>(sq, st, n, k, cb, G, sm, s_save, tot, w_entries);
+            ok = expand_tiles<M, BS, K>(sq, st, n, k, cb, G, sm, s_save, tot, w_entries);
             uint32_t below = 0;
             if(ok) ok = gather_sum<NW>(w_children, it.epoch, G, cb, tot.accepted - before, true, sm.gs, below, appended);
         }
@@ -1260,7 +1257,7 @@ struct EntrySrc {
 // Learned proposal of the quadrotor queries in qidx: one mixture record per frontier entry,
 // from the BF16 tensor-core forward pass of the entry's node.  Runs between k_frontier_write
 // and k_expand, which samples each child's draws from its entry's record.
-__global__ void __launch_bounds__(mlp::tc::kThreads, 1) k_propose(const QueryDev* __restrict__ qs, const uint32_t* __restrict__ qidx)
+static __global__ void __launch_bounds__(mlp::tc::kThreads, 1) k_propose(const QueryDev* __restrict__ qs, const uint32_t* __restrict__ qidx)
 {
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ QueryDev sq;
@@ -1272,7 +1269,7 @@ __global__ void __launch_bounds__(mlp::tc::kThreads, 1) k_propose(const QueryDev
     mlp::tc::forward(src, sq.mlp_img, smem, &sq.ctl->error);
 }
 
-__global__ void k_reactivate(const QueryDev* __restrict__ qs)
+static __global__ void k_reactivate(const QueryDev* __restrict__ qs)
 {
     __shared__ QueryDev sq;
     load_query(qs, nullptr, sq);
@@ -1288,7 +1285,7 @@ __global__ void k_reactivate(const QueryDev* __restrict__ qs)
 }
 
 // Goal-to-root walk (KPAX.cu:482-501), goal row first, root row last.
-__global__ void k_path(const QueryDev* __restrict__ qs)
+static __global__ void k_path(const QueryDev* __restrict__ qs)
 {
     __shared__ QueryDev sq;
     load_query(qs, nullptr, sq);

@@ -15,6 +15,7 @@
 #include "kpax_batch_kernels.cuh"
 #include "kpax_internal.h"
 #include "kpax_plan_kernels.cuh"
+#include "kpax_plan_steps.h"
 
 using namespace kpax;
 using namespace kpax::plan;
@@ -60,36 +61,6 @@ void launch_chained(void (*kernel)(P...), dim3 grid, unsigned block, size_t smem
     cudaLaunchKernelEx(&lc, kernel, static_cast<P>(args)...);
 }
 
-// The expansion kernel at one of its block sizes (validated by kpax_config_validate).
-template <int M>
-void launch_expand(int bs, dim3 grid, cudaStream_t s, const QueryDev* dq, const uint32_t* qidx, uint32_t* active)
-{
-    switch(bs) {
-        case 128: launch_chained(k_expand<M, 128>, grid, 128, kSaveBytes<M, 128>, s, dq, qidx, active); break;
-        case 256: launch_chained(k_expand<M, 256>, grid, 256, kSaveBytes<M, 256>, s, dq, qidx, active); break;
-        case 512: launch_chained(k_expand<M, 512>, grid, 512, kSaveBytes<M, 512>, s, dq, qidx, active); break;
-        default: launch_chained(k_expand<M, kExpandBS>, grid, kExpandBS, kSaveBytes<M, kExpandBS>, s, dq, qidx, active); break;
-    }
-}
-
-template <int M>
-void* expand_kernel(int bs)
-{
-    switch(bs) {
-        case 128: return (void*)k_expand<M, 128>;
-        case 256: return (void*)k_expand<M, 256>;
-        case 512: return (void*)k_expand<M, 512>;
-        default: return (void*)k_expand<M, kExpandBS>;
-    }
-}
-
-// Shared memory of the kept states of a block of bs children (run_steps), by model 1..3.
-size_t save_bytes(int model, int bs)
-{
-    const size_t sd = model == KPAX_MODEL_QUADROTOR ? 12 : 6;
-    return sizeof(float) * (size_t)kGroup * sd * (size_t)bs;
-}
-
 // Allows a kernel up to `most` bytes of dynamic shared memory (the default limit is 48 KB).  The limit
 // belongs to the kernel, not to the planner or batch that sets it, and a launch above it is refused, so
 // every caller passes the same number for a kernel: the most that any planner or batch can need.
@@ -102,77 +73,22 @@ kpax_status allow_smem(const void* fn, size_t most)
 // Shared memory of the per-query offsets of a persistent batch stage over n queries.
 constexpr size_t offset_bytes(size_t n) { return sizeof(uint32_t) * (n + 1); }
 
-// The fused iteration kernel (or one of its two parts around the proposal pass) at one of its
-// block sizes.
-template <int M, int PART = kIterWhole>
-void* iterate_kernel(int bs)
+// The kernels of kpax_plan_steps.h for `group` steps per collision query.
+ExpandFn expand_kernel(int model, int group, int bs)
 {
-    switch(bs) {
-        case 128: return (void*)k_iterate<M, 128, PART>;
-        case 256: return (void*)k_iterate<M, 256, PART>;
-        case 512: return (void*)k_iterate<M, 512, PART>;
-        default: return (void*)k_iterate<M, kExpandBS, PART>;
-    }
+    return group > 1 ? StepKernels<kGroup>::expand(model, bs) : StepKernels<1>::expand(model, bs);
 }
-
-template <int M, int PART = kIterWhole>
-void launch_iterate(int bs, uint32_t gx, cudaStream_t s, const QueryDev* dq, const Ctl* ctl, uint32_t* active, uint32_t inner)
+ExpandAllFn expand_all_kernel(int model, int group, int bs)
 {
-    const size_t smem = PART == kIterFront ? 0 : save_bytes(M, bs);
-    // not a cooperative launch: its residency check costs 70-100 us per launch, and a grid sized by the
-    // kernel's occupancy becomes resident as a whole once the SMs are free (the waits are bounded)
-    auto go = [&](auto kernel, unsigned block) { launch_chained(kernel, dim3(gx), block, smem, s, dq, ctl, active, inner); };
-    switch(bs) {
-        case 128: go(k_iterate<M, 128, PART>, 128); break;
-        case 256: go(k_iterate<M, 256, PART>, 256); break;
-        case 512: go(k_iterate<M, 512, PART>, 512); break;
-        default: go(k_iterate<M, kExpandBS, PART>, kExpandBS); break;
-    }
+    return group > 1 ? StepKernels<kGroup>::expand_all(model, bs) : StepKernels<1>::expand_all(model, bs);
 }
-
-// The persistent expansion of a batch's model group at one of its block sizes.
-template <int M>
-void* expand_all_kernel(int bs)
+IterateFn iterate_kernel(int model, int group, int bs)
 {
-    switch(bs) {
-        case 128: return (void*)k_expand_all<M, 128>;
-        case 256: return (void*)k_expand_all<M, 256>;
-        case 512: return (void*)k_expand_all<M, 512>;
-        default: return (void*)k_expand_all<M, kExpandBS>;
-    }
+    return group > 1 ? StepKernels<kGroup>::iterate(model, bs) : StepKernels<1>::iterate(model, bs);
 }
-
-template <int M>
-void launch_expand_all(int bs, uint32_t gx, size_t smem, cudaStream_t s, const QueryDev* dq, const Ctl* ctls,
-                       const uint32_t* qidx, uint32_t nq, uint32_t* active)
+IterateFn iterate_back_kernel(int group, int bs)
 {
-    switch(bs) {
-        case 128: launch_chained(k_expand_all<M, 128>, dim3(gx), 128, smem, s, dq, ctls, qidx, nq, active); break;
-        case 256: launch_chained(k_expand_all<M, 256>, dim3(gx), 256, smem, s, dq, ctls, qidx, nq, active); break;
-        case 512: launch_chained(k_expand_all<M, 512>, dim3(gx), 512, smem, s, dq, ctls, qidx, nq, active); break;
-        default: launch_chained(k_expand_all<M, kExpandBS>, dim3(gx), kExpandBS, smem, s, dq, ctls, qidx, nq, active); break;
-    }
-}
-
-void* expand_mixed_kernel(int bs)
-{
-    switch(bs) {
-        case 128: return (void*)k_expand_mixed<128>;
-        case 256: return (void*)k_expand_mixed<256>;
-        case 512: return (void*)k_expand_mixed<512>;
-        default: return (void*)k_expand_mixed<kExpandBS>;
-    }
-}
-
-void launch_expand_mixed(int bs, uint32_t gx, size_t smem, cudaStream_t s, const QueryDev* dq, const Ctl* ctls,
-                         const uint32_t* qidx, uint32_t nq, uint32_t* active)
-{
-    switch(bs) {
-        case 128: launch_chained(k_expand_mixed<128>, dim3(gx), 128, smem, s, dq, ctls, qidx, nq, active); break;
-        case 256: launch_chained(k_expand_mixed<256>, dim3(gx), 256, smem, s, dq, ctls, qidx, nq, active); break;
-        case 512: launch_chained(k_expand_mixed<512>, dim3(gx), 512, smem, s, dq, ctls, qidx, nq, active); break;
-        default: launch_chained(k_expand_mixed<kExpandBS>, dim3(gx), kExpandBS, smem, s, dq, ctls, qidx, nq, active); break;
-    }
+    return group > 1 ? StepKernels<kGroup>::iterate_back(bs) : StepKernels<1>::iterate_back(bs);
 }
 
 struct PlanBatch {
@@ -189,6 +105,7 @@ struct PlanBatch {
     uint32_t* d_groups[3] = {nullptr, nullptr, nullptr};
     uint32_t expand_gx[3] = {0, 0, 0};
     int expand_bs[3] = {kExpandBS, kExpandBS, kExpandBS};  // block size per model group (its first query's)
+    int step_group[3] = {kGroup, kGroup, kGroup};  // steps per collision query: 1 if a query's steps are long
     uint32_t gx_front = 1, gx_score = 1;
     bool persistent = false;  // batch: persistent stage launches over all queries (per-query offsets)
     uint32_t gx_count_all = 0, gx_write_all = 0, gx_scores_all = 0, gx_expand_all[3] = {0, 0, 0};
@@ -327,6 +244,7 @@ struct PlanBatch {
         for(uint32_t q = 0; q < n; ++q) {
             const int m = prm[q].model - 1;
             if(groups[m].empty()) expand_bs[m] = cfg[q].block_size > 0 ? cfg[q].block_size : kExpandBS;
+            if(!grouped(prm[q])) step_group[m] = 1;
             groups[m].push_back(q);
             const uint32_t bs = (uint32_t)expand_bs[m], spt = cfg[q].samples_per_thread > 0 ? cfg[q].samples_per_thread : 1;
             const uint32_t tiles = (prm[q].budget + bs - 1) / bs;
@@ -351,22 +269,21 @@ struct PlanBatch {
             KPAX_CUDA(cudaGetDevice(&dev));
             KPAX_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
             const int m = prm[0].model - 1, bs = expand_bs[m];
-            void* fn = m == 0 ? iterate_kernel<KPAX_MODEL_DOUBLE_INTEGRATOR>(bs)
-                              : m == 1 ? iterate_kernel<KPAX_MODEL_DUBINS_AIRPLANE>(bs) : iterate_kernel<KPAX_MODEL_QUADROTOR>(bs);
-            kpax_status st = allow_smem(fn, save_bytes(m + 1, bs));
+            const void* fn = (const void*)iterate_kernel(m + 1, step_group[m], bs);
+            const size_t save = save_bytes(m + 1, step_group[m], bs);
+            kpax_status st = allow_smem(fn, save);
             if(st != KPAX_OK) return st;
-            KPAX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, bs, save_bytes(m + 1, bs)));
+            KPAX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, bs, save));
             const uint32_t resident = (uint32_t)std::max(per_sm, 0) * (uint32_t)sms;
             // every resident CTA: the frontier and score phases use them all, the expansion as many as
             // it has tiles (a small budget's iteration leaves the rest idle in that phase)
             gx_iter = std::min<uint32_t>(resident, (uint32_t)kIterMaxCTAs);
             if(m == 2) {  // the two parts around the proposal pass: the smaller occupancy of the two
                 int front = 0, back = 0;
-                KPAX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-                    &front, iterate_kernel<KPAX_MODEL_QUADROTOR, kIterFront>(bs), bs, 0));
-                if((st = allow_smem(iterate_kernel<KPAX_MODEL_QUADROTOR, kIterBack>(bs), save_bytes(m + 1, bs))) != KPAX_OK) return st;
-                KPAX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-                    &back, iterate_kernel<KPAX_MODEL_QUADROTOR, kIterBack>(bs), bs, save_bytes(m + 1, bs)));
+                KPAX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&front, (const void*)iterate_front_kernel(bs), bs, 0));
+                const void* fn_back = (const void*)iterate_back_kernel(step_group[m], bs);
+                if((st = allow_smem(fn_back, save)) != KPAX_OK) return st;
+                KPAX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&back, fn_back, bs, save));
                 gx_split = std::min<uint32_t>((uint32_t)std::max(std::min(front, back), 0) * (uint32_t)sms,
                                               (uint32_t)kIterMaxCTAs);
             }
@@ -389,10 +306,8 @@ struct PlanBatch {
             if(st == KPAX_OK) st = resident((const void*)k_scores_all, kScoreBS, 0, n, gx_scores_all);
             for(int m = 0; m < 3 && st == KPAX_OK; ++m) {
                 if(groups[m].empty()) continue;
-                const void* fn = m == 0 ? expand_all_kernel<KPAX_MODEL_DOUBLE_INTEGRATOR>(expand_bs[m])
-                                        : m == 1 ? expand_all_kernel<KPAX_MODEL_DUBINS_AIRPLANE>(expand_bs[m])
-                                                 : expand_all_kernel<KPAX_MODEL_QUADROTOR>(expand_bs[m]);
-                st = resident(fn, expand_bs[m], save_bytes(m + 1, expand_bs[m]), groups[m].size(), gx_expand_all[m]);
+                st = resident((const void*)expand_all_kernel(m + 1, step_group[m], expand_bs[m]), expand_bs[m],
+                              save_bytes(m + 1, step_group[m], expand_bs[m]), groups[m].size(), gx_expand_all[m]);
             }
             if(st != KPAX_OK) return st;
             persistent = gx_count_all && gx_write_all && gx_scores_all && (groups[0].empty() || gx_expand_all[0]) &&
@@ -403,7 +318,7 @@ struct PlanBatch {
                 if(groups[m].empty()) continue;
                 ++ngroups;
                 if(!bs0) bs0 = expand_bs[m];
-                same_bs = same_bs && expand_bs[m] == bs0;
+                same_bs = same_bs && expand_bs[m] == bs0 && step_group[m] == kGroup;  // k_expand_mixed queries groups of steps
             }
             if(persistent && ngroups > 1 && same_bs) {
                 std::vector<uint32_t> order;
@@ -412,7 +327,7 @@ struct PlanBatch {
                 KPAX_CUDA(cudaMemcpyAsync(d_mixed, order.data(), sizeof(uint32_t) * order.size(), cudaMemcpyHostToDevice,
                                           stream));
                 uint32_t gx = 0;
-                if((st = resident(expand_mixed_kernel(bs0), bs0, save_bytes(KPAX_MODEL_QUADROTOR, bs0), n, gx)) != KPAX_OK) return st;
+                if((st = resident((const void*)expand_mixed_kernel(bs0), bs0, save_bytes(KPAX_MODEL_QUADROTOR, kGroup, bs0), n, gx)) != KPAX_OK) return st;
                 if(gx) mixed_bs = bs0, gx_mixed = gx;
             }
         }
@@ -422,10 +337,7 @@ struct PlanBatch {
                                    : !persistent || expand_mode == 0;
         for(int m = 0; m < 3 && staged; ++m) {
             if(groups[m].empty()) continue;
-            const void* fn = m == 0 ? expand_kernel<KPAX_MODEL_DOUBLE_INTEGRATOR>(expand_bs[m])
-                                    : m == 1 ? expand_kernel<KPAX_MODEL_DUBINS_AIRPLANE>(expand_bs[m])
-                                             : expand_kernel<KPAX_MODEL_QUADROTOR>(expand_bs[m]);
-            kpax_status st = allow_smem(fn, save_bytes(m + 1, expand_bs[m]));
+            kpax_status st = allow_smem((const void*)expand_kernel(m + 1, step_group[m], expand_bs[m]), save_bytes(m + 1, step_group[m], expand_bs[m]));
             if(st != KPAX_OK) return st;
         }
         update_fused();
@@ -439,7 +351,7 @@ struct PlanBatch {
     // Dynamic shared memory of the persistent expansion of model group m with g queries.
     size_t expand_all_smem(int m, size_t g) const
     {
-        return save_bytes(m + 1, expand_bs[m]) + offset_bytes(g);
+        return save_bytes(m + 1, step_group[m], expand_bs[m]) + offset_bytes(g);
     }
 
     void update_fused()
@@ -516,18 +428,20 @@ struct PlanBatch {
     {
         if(ev) cudaEventRecord(ev[0], stream);
         if(fused_split) {  // front launch, proposal pass, back launch; phase times from the device clock
-            launch_iterate<KPAX_MODEL_QUADROTOR, kIterFront>(expand_bs[2], gx_split, stream, dq, d_ctl, d_active, 1);
+            const int bs = expand_bs[2], group = step_group[2];
+            launch_chained(iterate_front_kernel(bs), dim3(gx_split), bs, 0, stream, dq, d_ctl, d_active, 1u);
             launch_proposal(stream);
-            launch_iterate<KPAX_MODEL_QUADROTOR, kIterBack>(expand_bs[2], gx_split, stream, dq, d_ctl, d_active, 1);
+            launch_chained(iterate_back_kernel(group, bs), dim3(gx_split), bs, save_bytes(KPAX_MODEL_QUADROTOR, group, bs), stream, dq,
+                           d_ctl, d_active, 1u);
             if(ev) cudaEventRecord(ev[3], stream);
             return;
         }
         if(fused) {  // one launch of up to `inner` iterations: phase times from the device clock (Ctl::t_*_ns)
             const int m = prm[0].model - 1;
-            const Ctl* c0 = d_ctl;  // the single query's control block
-            if(m == 0) launch_iterate<KPAX_MODEL_DOUBLE_INTEGRATOR>(expand_bs[m], gx_iter, stream, dq, c0, d_active, inner);
-            else if(m == 1) launch_iterate<KPAX_MODEL_DUBINS_AIRPLANE>(expand_bs[m], gx_iter, stream, dq, c0, d_active, inner);
-            else launch_iterate<KPAX_MODEL_QUADROTOR>(expand_bs[m], gx_iter, stream, dq, c0, d_active, inner);
+            // not a cooperative launch: its residency check costs 70-100 us per launch, and a grid sized by the
+            // kernel's occupancy becomes resident as a whole once the SMs are free (the waits are bounded)
+            launch_chained(iterate_kernel(m + 1, step_group[m], expand_bs[m]), dim3(gx_iter), expand_bs[m],
+                           save_bytes(m + 1, step_group[m], expand_bs[m]), stream, dq, d_ctl, d_active, inner);
             if(ev) cudaEventRecord(ev[3], stream);
             return;
         }
@@ -552,28 +466,20 @@ struct PlanBatch {
                         cudaStreamWaitEvent(s, ev_fork, 0);
                     }
                     const dim3 grid(expand_gx[m], (uint32_t)groups[m].size());
-                    if(m == 0) launch_expand<KPAX_MODEL_DOUBLE_INTEGRATOR>(expand_bs[m], grid, s, dq, d_groups[m], d_active);
-                    else if(m == 1) launch_expand<KPAX_MODEL_DUBINS_AIRPLANE>(expand_bs[m], grid, s, dq, d_groups[m], d_active);
-                    else launch_expand<KPAX_MODEL_QUADROTOR>(expand_bs[m], grid, s, dq, d_groups[m], d_active);
+                    launch_chained(expand_kernel(m + 1, step_group[m], expand_bs[m]), grid, expand_bs[m],
+                                   save_bytes(m + 1, step_group[m], expand_bs[m]), s, dq, d_groups[m], d_active);
                     if(u < nused - 1) cudaEventRecord(ev_join[u], s);
                 }
                 for(int u = 0; u + 1 < nused; ++u) cudaStreamWaitEvent(stream, ev_join[u], 0);
             } else if(expand_mode == 2 && mixed_bs) {
-                launch_expand_mixed(mixed_bs, gx_mixed, save_bytes(KPAX_MODEL_QUADROTOR, mixed_bs) + sq, stream, dq, d_ctl, d_mixed, nq, d_active);
+                launch_chained(expand_mixed_kernel(mixed_bs), dim3(gx_mixed), mixed_bs,
+                               save_bytes(KPAX_MODEL_QUADROTOR, kGroup, mixed_bs) + sq, stream, dq, d_ctl, d_mixed, nq, d_active);
             } else {
                 for(int m = 0; m < 3; ++m) {
                     if(groups[m].empty()) continue;
                     const uint32_t g = (uint32_t)groups[m].size();
-                    const size_t sg = expand_all_smem(m, g);
-                    if(m == 0)
-                        launch_expand_all<KPAX_MODEL_DOUBLE_INTEGRATOR>(expand_bs[m], gx_expand_all[m], sg, stream, dq, d_ctl,
-                                                                        d_groups[m], g, d_active);
-                    else if(m == 1)
-                        launch_expand_all<KPAX_MODEL_DUBINS_AIRPLANE>(expand_bs[m], gx_expand_all[m], sg, stream, dq, d_ctl,
-                                                                      d_groups[m], g, d_active);
-                    else
-                        launch_expand_all<KPAX_MODEL_QUADROTOR>(expand_bs[m], gx_expand_all[m], sg, stream, dq, d_ctl,
-                                                                d_groups[m], g, d_active);
+                    launch_chained(expand_all_kernel(m + 1, step_group[m], expand_bs[m]), dim3(gx_expand_all[m]), expand_bs[m],
+                                   expand_all_smem(m, g), stream, dq, d_ctl, d_groups[m], g, d_active);
                 }
             }
             if(ev && split) cudaEventRecord(ev[2], stream);
@@ -597,9 +503,8 @@ struct PlanBatch {
             }
             const dim3 grid(expand_gx[m], (uint32_t)groups[m].size());
             if(m == 2 && n_learned) launch_proposal(s);
-            if(m == 0) launch_expand<KPAX_MODEL_DOUBLE_INTEGRATOR>(expand_bs[m], grid, s, dq, d_groups[m], d_active);
-            else if(m == 1) launch_expand<KPAX_MODEL_DUBINS_AIRPLANE>(expand_bs[m], grid, s, dq, d_groups[m], d_active);
-            else launch_expand<KPAX_MODEL_QUADROTOR>(expand_bs[m], grid, s, dq, d_groups[m], d_active);
+            launch_chained(expand_kernel(m + 1, step_group[m], expand_bs[m]), grid, expand_bs[m],
+                           save_bytes(m + 1, step_group[m], expand_bs[m]), s, dq, d_groups[m], d_active);
             if(u < nused - 1) cudaEventRecord(ev_join[u], s);
         }
         for(int u = 0; u + 1 < nused; ++u) cudaStreamWaitEvent(stream, ev_join[u], 0);

@@ -62,12 +62,11 @@ __device__ __forceinline__ float goal_distance3(const float* s, const float* g)
     return __fsqrt_rn(__fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz)));
 }
 
-template <int M>
+template <int M, int K>
 __global__ void __launch_bounds__(32) k_rekino(const RekinoDev d)
 {
     constexpr int SD = ModelDims<M>::SD, CD = ModelDims<M>::CD, S = SD + CD + 1;
-    constexpr int kGroup = 5;  // steps per collision query (run_steps)
-    __shared__ __align__(16) float s_save[kGroup * SD * 32];
+    __shared__ __align__(16) float s_save[K > 1 ? K * SD * 32 : 4];
     extern __shared__ float s_cand[];  // [spt * 32][S] candidate rows, then [spt * 32] distances
     const KParams& p = d.p;
     const uint32_t w = blockIdx.x, lane = threadIdx.x, spt = d.spt, nsamp = 32u * spt;
@@ -100,7 +99,7 @@ __global__ void __launch_bounds__(32) k_rekino(const RekinoDev d)
 #pragma unroll
             for(int q = 0; q < SD; ++q) s[q] = cur[q];
             int done = 0;
-            const bool valid = propagate<M, kGroup>(p, d.g, s, cc, steps, done, s_save + lane * SD, 32);
+            const bool valid = propagate<M, K>(p, d.g, s, cc, steps, done, s_save + lane * SD, 32);
             row_controls<M>(cc, rc);
             float* row = s_cand + (size_t)j * S;
 #pragma unroll
@@ -304,9 +303,8 @@ static kpax_status rekino_plan_body(kpax_rekino* r, const float* h_init, const f
     RekinoDev d{p, r->env.view(), r->d_ig, r->d_ig + S, r->d_paths, r->d_lens, r->d_best, r->d_best + 1,
                 r->rp.max_iterations, spt, r->plans, r->rp.epsilon_greedy, (unsigned long long)(r->rp.timeout_ms * 1e6)};
     const size_t smem = sizeof(float) * 32u * spt * (S + 1);
-    if(p.model == KPAX_MODEL_DOUBLE_INTEGRATOR) k_rekino<KPAX_MODEL_DOUBLE_INTEGRATOR><<<W, 32, smem, r->stream>>>(d);
-    else if(p.model == KPAX_MODEL_DUBINS_AIRPLANE) k_rekino<KPAX_MODEL_DUBINS_AIRPLANE><<<W, 32, smem, r->stream>>>(d);
-    else k_rekino<KPAX_MODEL_QUADROTOR><<<W, 32, smem, r->stream>>>(d);
+    by_model(p.model, grouped(p) ? kGroup : 1,
+             [&](auto m, auto k) { k_rekino<decltype(m)::value, decltype(k)::value><<<W, 32, smem, r->stream>>>(d); });
     KPAX_CHECK_LAUNCH();
     count_launch();
     r->plans += 1;
