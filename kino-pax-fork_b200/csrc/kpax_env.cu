@@ -135,14 +135,21 @@ __global__ void k_env_fill(Grid g, const float4* __restrict__ packed, uint32_t n
 }
 
 // The three passes in one CTA with the counts in shared memory, for grids and obstacle counts that one
-// SM gets through sooner than the launches of three kernels and a memset take; its latency is a chain of
-// atomics and scattered stores per obstacle, eight lanes each.  Entries are filled in when they fit `cap`;
-// otherwise `cursor` holds the offsets for k_env_fill.  B200, the allocation-free batch with 1021
-// segments on an 8000-cell grid, host us, three kernels / one: 1 obstacle 54 / 41, 20 54 / 46, 300 56 / 52,
-// 1000 58 / 88.
+// SM gets through sooner than the launches of three kernels and a memset take.  Rows of x-neighbouring cells
+// are dealt out to the threads, so that a box over the whole grid keeps them as busy as many small ones.
+// Entries are filled in when they fit `cap`; otherwise `cursor` holds the offsets for k_env_fill.  More
+// than env_build_pairs(n) (cell, obstacle) pairs are left to the other kernels: `off` then holds zeros and
+// the number of pairs, which is known before any is counted.
+// The three kernels give each obstacle a warp on one of many SMs, so their time is the largest box's; this
+// one's is the pairs'.  B200, the allocation-free batch with 1021 segments on a 9261-cell grid, host us,
+// three kernels / one: 20 boxes of 5 m (160 pairs) 41 / 33, 45 m (15477) 62 / 45, 90 m (69232) 119 / 71; one
+// over the whole grid 155 / 37; 60 boxes of 30 m (17550) 50 / 45, 45 m (46597) 65 / 59, 60 m (89860) 78 / 85;
+// 256 of 10 m (6420) 44 / 36, 20 m (27667) 53 / 56, 45 m (184267) 61 / 154.  More than 256 of 1 to 5 m: 300
+// 56 / 52, 1000 58 / 88 with eight threads an obstacle.
 constexpr int kEnvBuildBS = 1024;
-constexpr uint32_t kEnvBuildCells = 12000;  // 48 KB of shared memory with the scan's
+constexpr uint32_t kEnvBuildCells = 12000;  // 48 KB of shared memory with the rest (22^3 cells: 46 KB)
 constexpr uint32_t kEnvBuildObstacles = 256;
+__host__ __device__ constexpr uint32_t env_build_pairs(uint32_t n) { return n <= 40u ? 0xFFFFFFFFu : n <= 80u ? 1u << 15 : 1u << 14; }
 inline bool env_build_once(uint32_t cells, uint32_t n) { return cells <= kEnvBuildCells && n <= kEnvBuildObstacles; }
 
 __global__ void __launch_bounds__(kEnvBuildBS) k_env_build(Grid g, const float* __restrict__ obs, uint32_t n, uint32_t cells,
@@ -151,45 +158,72 @@ __global__ void __launch_bounds__(kEnvBuildBS) k_env_build(Grid g, const float* 
 {
     extern __shared__ uint32_t s_cell[];  // counts, then offsets, then the next free entry
     __shared__ uint32_t s_warp[32];
+    // of each obstacle: the rows before its own, its first cell, its extents in x and y
+    __shared__ uint32_t s_row[kEnvBuildObstacles], s_cell0[kEnvBuildObstacles], s_ext[kEnvBuildObstacles];
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    // exclusive prefix of the block's values, and their sum
+    auto block_scan = [&](uint32_t v, uint32_t& total) {
+        auto warp_scan = [&](uint32_t a) {
+#pragma unroll
+            for(int d = 1; d < 32; d <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, a, d);
+                if(lane >= (uint32_t)d) a += y;
+            }
+            return a;
+        };
+        const uint32_t x = warp_scan(v);
+        if(lane == 31u) s_warp[warp] = x;
+        __syncthreads();
+        if(warp == 0) s_warp[lane] = warp_scan(s_warp[lane]);
+        __syncthreads();
+        const uint32_t below = (warp ? s_warp[warp - 1] : 0u) + x - v;
+        total = s_warp[31];
+        __syncthreads();
+        return below;
+    };
     for(uint32_t i = tid; i < cells; i += kEnvBuildBS) s_cell[i] = 0u;
-    __syncthreads();
-    auto each_cell = [&](bool pack, auto f) {
-        for(uint32_t o = tid >> 3; o < n; o += kEnvBuildBS / 8) {
-            const float* b = obs + (size_t)6 * o;
-            const float4 lo = make_float4(b[0], b[1], b[2], 0.0f), hi = make_float4(b[3], b[4], b[5], 0.0f);
-            if(pack && (tid & 7u) == 0) packed[2 * o] = lo, packed[2 * o + 1] = hi;
-            int c0[3], c1[3];
-            obstacle_cells(g, lo, hi, c0, c1);
-            const int total = box_cells(c0, c1);
-            for(int k = (int)(tid & 7u); k < total; k += 8) f(o, box_cell(g, c0, c1, k));
+    uint32_t own_rows = 0, own_pairs = 0;
+    if(tid < n) {
+        const float* b = obs + (size_t)6 * tid;
+        const float4 lo = make_float4(b[0], b[1], b[2], 0.0f), hi = make_float4(b[3], b[4], b[5], 0.0f);
+        packed[2 * tid] = lo, packed[2 * tid + 1] = hi;
+        int c0[3], c1[3];
+        obstacle_cells(g, lo, hi, c0, c1);
+        own_pairs = (uint32_t)box_cells(c0, c1);
+        if(own_pairs) own_rows = (uint32_t)((c1[1] - c0[1] + 1) * (c1[2] - c0[2] + 1));
+        s_cell0[tid] = (uint32_t)(c0[0] + g.dim * (c0[1] + g.dim * c0[2]));
+        s_ext[tid] = (uint32_t)(c1[0] - c0[0] + 1) | ((uint32_t)(c1[1] - c0[1] + 1) << 16);
+    }
+    uint32_t rows, pairs;
+    const uint32_t row0 = block_scan(own_rows, rows);
+    if(tid < n) s_row[tid] = row0;
+    block_scan(own_pairs, pairs);  // its barriers cover s_row and s_cell as well
+    if(pairs > env_build_pairs(n)) {
+        for(uint32_t i = tid; i <= cells; i += kEnvBuildBS) off[i] = i < cells ? 0u : pairs;
+        return;
+    }
+    auto each_cell = [&](auto f) {
+        for(uint32_t r = tid; r < rows; r += kEnvBuildBS) {
+            uint32_t o = 0;  // the last obstacle whose rows start at or before r
+#pragma unroll
+            for(uint32_t d = kEnvBuildObstacles / 2; d > 0; d >>= 1)
+                if(o + d < n && s_row[o + d] <= r) o += d;
+            const uint32_t q = r - s_row[o], nx = s_ext[o] & 0xFFFFu, ny = s_ext[o] >> 16, z = q / ny, y = q - z * ny;
+            const uint32_t c = s_cell0[o] + g.dim * (y + g.dim * z);
+            for(uint32_t x = 0; x < nx; ++x) f(o, c + x);
         }
     };
-    each_cell(true, [&](uint32_t, int c) { atomicAdd(s_cell + c, 1u); });
+    each_cell([&](uint32_t, uint32_t c) { atomicAdd(s_cell + c, 1u); });
     __syncthreads();
     const uint32_t per = (cells + kEnvBuildBS - 1) / kEnvBuildBS | 1u;  // odd: no bank conflicts
     const uint32_t i0 = min(tid * per, cells), i1 = min(i0 + per, cells);
-    uint32_t sum = 0;
+    uint32_t sum = 0, total;
     for(uint32_t i = i0; i < i1; ++i) sum += s_cell[i];
-    auto warp_scan = [&](uint32_t v) {
-#pragma unroll
-        for(int d = 1; d < 32; d <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, v, d);
-            if(lane >= (uint32_t)d) v += y;
-        }
-        return v;
-    };
-    const uint32_t x = warp_scan(sum);
-    if(lane == 31u) s_warp[warp] = x;
-    __syncthreads();
-    if(warp == 0) s_warp[lane] = warp_scan(s_warp[lane]);
-    __syncthreads();
-    uint32_t acc = (warp ? s_warp[warp - 1] : 0u) + x - sum;
+    uint32_t acc = block_scan(sum, total);
     for(uint32_t i = i0; i < i1; ++i) {
         const uint32_t v = s_cell[i];
         s_cell[i] = acc, acc += v;
     }
-    const uint32_t total = s_warp[31];
     __syncthreads();
     for(uint32_t i = tid; i < cells; i += kEnvBuildBS) {
         off[i] = s_cell[i];
@@ -198,7 +232,7 @@ __global__ void __launch_bounds__(kEnvBuildBS) k_env_build(Grid g, const float* 
     if(tid == 0) off[cells] = total;
     if(total > cap) return;
     __syncthreads();
-    each_cell(false, [&](uint32_t o, int c) { ent[atomicAdd(s_cell + c, 1u)] = o; });
+    each_cell([&](uint32_t o, uint32_t c) { ent[atomicAdd(s_cell + c, 1u)] = o; });
 }
 
 inline uint32_t warp_blocks(uint32_t n) { return (uint32_t)(((uint64_t)n * 32 + 255) / 256); }
@@ -525,6 +559,18 @@ __global__ void k_sincos_pair(const float* __restrict__ x, uint32_t n, float* __
 
 }  // namespace
 
+// The grid's offsets by two kernels, from counts at zero.
+static kpax_status env_count(const Grid& g, const float* d_obstacles, uint32_t n, uint32_t cells, float4* packed, uint32_t* off,
+                             uint32_t* cursor, cudaStream_t stream)
+{
+    k_env_count<<<warp_blocks(n), 256, 0, stream>>>(g, d_obstacles, n, packed, off);
+    KPAX_CHECK_LAUNCH();
+    k_env_scan<<<1, 1024, 0, stream>>>(off, cells, cursor);
+    KPAX_CHECK_LAUNCH();
+    count_launch(2);
+    return KPAX_OK;
+}
+
 kpax_status Env::build_start(const KParams& p, const float* d_obstacles, uint32_t n, cudaStream_t stream)
 {
     cell = p.cell;
@@ -562,11 +608,8 @@ kpax_status Env::build_start(const KParams& p, const float* d_obstacles, uint32_
     } else {
         KPAX_CUDA(cudaMemsetAsync(d_off, 0, sizeof(uint32_t) * (cells + 1), stream));
         if(n) {
-            k_env_count<<<warp_blocks(n), 256, 0, stream>>>(view(), d_obstacles, n, d_obs, d_off);
-            KPAX_CHECK_LAUNCH();
-            k_env_scan<<<1, 1024, 0, stream>>>(d_off, cells, d_cursor);
-            KPAX_CHECK_LAUNCH();
-            count_launch(2);
+            kpax_status st = env_count(view(), d_obstacles, n, cells, d_obs, d_off, d_cursor, stream);
+            if(st != KPAX_OK) return st;
         }
     }
     *h_total = 0;
@@ -574,9 +617,14 @@ kpax_status Env::build_start(const KParams& p, const float* d_obstacles, uint32_
     return KPAX_OK;
 }
 
-kpax_status Env::build_finish(cudaStream_t stream)
+kpax_status Env::build_finish(const float* d_obstacles, cudaStream_t stream)
 {
     n_ent = *h_total;
+    if(filled && n_ent > env_build_pairs(n_obs)) {
+        filled = false;
+        kpax_status st = env_count(view(), d_obstacles, n_obs, n_cells, d_obs, d_off, d_cursor, stream);
+        if(st != KPAX_OK) return st;
+    }
     if(n_ent > ent_cap) {
         filled = false;
         if(d_ent) cudaFree(d_ent), d_ent = nullptr, ent_cap = 0;
@@ -597,7 +645,7 @@ kpax_status Env::build(const KParams& p, const float* d_obstacles, uint32_t n, c
     kpax_status st = build_start(p, d_obstacles, n, stream);
     if(st != KPAX_OK) return st;
     if(n) KPAX_CUDA(cudaStreamSynchronize(stream));
-    return build_finish(stream);
+    return build_finish(d_obstacles, stream);
 }
 
 void Env::release()
@@ -896,11 +944,7 @@ extern "C" kpax_status kpax_propagate_batch_noalloc(const kpax_config* cfg, cons
         // the array keeps the previous call's grid: the counts must start from zero
         KPAX_CUDA(cudaMemsetAsync(s->off, 0, sizeof(uint32_t) * (cells + 1), cs));
         if(n_obs) {
-            k_env_count<<<warp_blocks(n_obs), 256, 0, cs>>>(g, d_obstacles, n_obs, s->obs, s->off);
-            KPAX_CHECK_LAUNCH();
-            k_env_scan<<<1, 1024, 0, cs>>>(s->off, cells, s->cursor);
-            KPAX_CHECK_LAUNCH();
-            count_launch(2);
+            if((st = env_count(g, d_obstacles, n_obs, cells, s->obs, s->off, s->cursor, cs)) != KPAX_OK) return st;
         }
     }
     if(n_obs) {
@@ -911,7 +955,10 @@ extern "C" kpax_status kpax_propagate_batch_noalloc(const kpax_config* cfg, cons
             return set_error("kpax_propagate_batch_noalloc: %u (cell, obstacle) pairs exceed the limit of %u", total,
                              kNoAllocMaxEntries),
                    KPAX_ECAPACITY;
-        if(!once) {
+        if(once && total > env_build_pairs(n_obs) &&
+           (st = env_count(g, d_obstacles, n_obs, cells, s->obs, s->off, s->cursor, cs)) != KPAX_OK)
+            return st;
+        if(!once || total > env_build_pairs(n_obs)) {
             k_env_fill<<<warp_blocks(n_obs), 256, 0, cs>>>(g, s->obs, n_obs, s->cursor, s->ent);
             KPAX_CHECK_LAUNCH();
             count_launch(1);

@@ -91,9 +91,9 @@ struct Env {
     // Build from n x 6 device floats on `stream` (synchronises once to size the entry list).
     kpax_status build(const KParams& p, const float* d_obstacles, uint32_t n, cudaStream_t stream);
     // The same in two halves, so that several environments can share one synchronisation of `stream`
-    // between them; view() is final after the second.
+    // between them; view() is final after the second, which takes the same obstacles.
     kpax_status build_start(const KParams& p, const float* d_obstacles, uint32_t n, cudaStream_t stream);
-    kpax_status build_finish(cudaStream_t stream);
+    kpax_status build_finish(const float* d_obstacles, cudaStream_t stream);
     void release();
 };
 

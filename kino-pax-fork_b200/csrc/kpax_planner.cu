@@ -664,7 +664,7 @@ struct PlanBatch {
         KPAX_CUDA(cudaMemcpyAsync(d_active, h_active, sizeof(uint32_t), cudaMemcpyHostToDevice, stream));
         if(counted) KPAX_CUDA(cudaStreamSynchronize(stream));
         for(uint32_t q = 0; q < nq; ++q) {
-            kpax_status st = env[q].build_finish(stream);
+            kpax_status st = env[q].build_finish(d_obstacles[q], stream);
             if(st != KPAX_OK) return st;
             hq[q].g = env[q].view();
             if(hq[q].occ) {
