@@ -219,10 +219,10 @@ struct PlanBatch {
             if(pass == 0) KPAX_CUDA(cudaMalloc(&pool, cv.used));
         }
         KPAX_CUDA(cudaMalloc(&dq, sizeof(QueryDev) * n));
-        KPAX_CUDA(cudaMalloc(&d_ctl, sizeof(Ctl) * n));
-        KPAX_CUDA(cudaMallocHost(&h_ctl, sizeof(Ctl) * n));
-        KPAX_CUDA(cudaMalloc(&d_active, sizeof(uint32_t)));
-        KPAX_CUDA(cudaMallocHost(&h_active, sizeof(uint32_t)));
+        // the count of active queries lies behind the control blocks: one copy reads both
+        KPAX_CUDA(cudaMalloc(&d_ctl, sizeof(Ctl) * n + sizeof(uint32_t)));
+        KPAX_CUDA(cudaMallocHost(&h_ctl, sizeof(Ctl) * n + sizeof(uint32_t)));
+        d_active = reinterpret_cast<uint32_t*>(d_ctl + n), h_active = reinterpret_cast<uint32_t*>(h_ctl + n);
         KPAX_CUDA(cudaMalloc(&d_ig, sizeof(float) * n * 2 * s_max));
         KPAX_CUDA(cudaMallocHost(&h_ig, sizeof(float) * n * 2 * s_max));
         KPAX_CUDA(cudaMalloc(&d_path, sizeof(float) * (size_t)path_total * s_max));
@@ -370,10 +370,10 @@ struct PlanBatch {
         for(Env& e : env) e.release();
         for(int m = 0; m < 3; ++m)
             if(d_groups[m]) cudaFree(d_groups[m]);
-        void* dev[] = {pool, dq, d_ctl, d_active, d_ig, d_path, d_flush, d_img, d_learn, d_learned, d_mixed, d_prop_off};
+        void* dev[] = {pool, dq, d_ctl, d_ig, d_path, d_flush, d_img, d_learn, d_learned, d_mixed, d_prop_off};
         for(void* p : dev)
             if(p) cudaFree(p);
-        void* host[] = {h_ctl, h_active, h_ig, h_path};
+        void* host[] = {h_ctl, h_ig, h_path};
         for(void* p : host)
             if(p) cudaFreeHost(p);
         release_capture();
@@ -698,8 +698,7 @@ struct PlanBatch {
                 count_launch(kernels_per_iteration() * (uint64_t)unroll);
             }
             if(!poll) continue;
-            KPAX_CUDA(cudaMemcpyAsync(h_active, d_active, sizeof(uint32_t), cudaMemcpyDeviceToHost, stream));
-            KPAX_CUDA(cudaMemcpyAsync(h_ctl, d_ctl, sizeof(Ctl) * nq, cudaMemcpyDeviceToHost, stream));
+            KPAX_CUDA(cudaMemcpyAsync(h_ctl, d_ctl, sizeof(Ctl) * nq + sizeof(uint32_t), cudaMemcpyDeviceToHost, stream));
             KPAX_CUDA(cudaStreamSynchronize(stream));
             if(*h_active == 0u) return check_ctl();
         }
