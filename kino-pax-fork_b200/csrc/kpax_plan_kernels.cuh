@@ -681,9 +681,11 @@ __device__ __forceinline__ bool expand_tiles(QueryDev& sq, const ExpandState st,
             if(valid) {
                 atomicAdd(rg.valid + r1v, 1);
                 const uint32_t word = (uint32_t)r2v >> 5, bit = 1u << (r2v & 31);
-                // snapshot and scores change between the iterations of one launch: through L2
-                const bool seen = (__ldcg(rg.cur + word) & bit) != 0u;
-                next = (u[5] < region_score(__ldcg(rg.score + r1v), st.total, st.ready, p.eps)) || !seen;
+                // plain loads, through L1: snapshot and scores change between the iterations of one launch, but
+                // behind a gather (as for the frontier count).  All children read the same few lines, which as
+                // L2 reads alone took 5 us of a double integrator iteration of 2^16 children.
+                const bool seen = (rg.cur[word] & bit) != 0u;
+                next = (u[5] < region_score(rg.score[r1v], st.total, st.ready, p.eps)) || !seen;
                 atomicOr(rg.nxt + word, bit);
                 if(next && p.prune) next = prune_keep(p, d_parent, goal_distance(s, ctl->goal), st.plan, st.iter, c);
             }
