@@ -476,10 +476,12 @@ __global__ void k_collide_batch(Grid g, const float* __restrict__ bbmin, const f
 // Large batches of queries with the whole grid in shared memory: a cell's record is its first entry and
 // the one past its last (16 bits each), entries are 16-bit obstacle indices, obstacles (lo, hi) pairs per
 // dimension.  The queries' cells are scattered, and a gather of 32 scattered words takes 32 wavefronts
-// from L1 but about four from shared memory; what bounds it is the issue of divergent lookups (13 of
-// 32 lanes active, 78 % issue).  Copying the grid costs every CTA 3-5 us, so it pays from 2^21 boxes on.
-// B200 (global / shared, boxes of up to 0.2 m, with ~10 us of launch and events): 2^22 boxes among 20
-// obstacles 42 / 41 us, 300 60 / 54, 1000 85 / 68, 2000 109 / 89; 2^20 boxes 18 / 20, 23 / 24, 30 / 30, 38 / 34.
+// from L1 but about four from shared memory; what bounds it is the issue of divergent lookups (a walk cell by
+// cell: 13 of 32 lanes active, 78 % issue).  Cells of a row lie behind one another in the entries, so a lane
+// walks rows.  Copying the grid costs every CTA 3-5 us, so it pays from 2^21 boxes on.
+// B200, 2^22 boxes, us (global / shared by cells / by rows): boxes of up to 0.2 m, 300 obstacles 52 / 45 / 41,
+// 1000 80 / 62 / 58, 2000 103 / 82 / 78; of up to 3 m 84 / 86 / 70, 115 / 100 / 87, 121 / 109 / 102; of up to
+// 20 m 263 / 238 / 147, 150 / 129 / 99, 105 / 94 / 84.
 constexpr int kCollideBS = 1024;
 constexpr uint32_t kCollideSharedMin = 1u << 21, kCollideSharedEnt = 4096;  // with few entries most cells are empty: 2^21 boxes among 20 obstacles 29 / 30 us
 constexpr size_t kCollideMaxSmem = 224 * 1024;
@@ -506,32 +508,34 @@ __global__ void __launch_bounds__(kCollideBS, 2) k_collide_shared(Grid g, uint32
     auto query = [&](const float* lo, const float* hi) -> bool {
         const int x0 = grid_coord(g, lo[0]), y0 = grid_coord(g, lo[1]), z0 = grid_coord(g, lo[2]);
         const int x1 = grid_coord(g, hi[0]), y1 = grid_coord(g, hi[1]), z1 = grid_coord(g, hi[2]);
-        // the walk over the box's cells as one loop: a lane whose cell is done steps to its next one
         const int row = x1 - x0, plane = y1 - y0;
-        int gx = row, gy = plane, gz = z1 - z0;
-        uint32_t c = x0 + g.dim * (y0 + g.dim * z0), r = s_cell[c], k = r & 0xFFFFu, e = r >> 16;
+        int gy = plane, gz = z1 - z0;
         if((row | plane | gz) < 0) return true;  // an inverted box has no cells
+        // the walk over the box's rows of cells, whose entries lie behind one another, as one loop: a lane
+        // whose row is done steps to its next one
+        uint32_t c = x0 + g.dim * (y0 + g.dim * z0), k = s_cell[c] & 0xFFFFu, e = s_cell[c + row] >> 16;
         for(;;) {
             if(k < e) {
                 const uint32_t o = s_ent[k++];
                 const float2 a = s_obs[o], b = s_obs[n_obs + o], d = s_obs[2 * n_obs + o];
                 if(hi[0] > a.x && a.y > lo[0] && hi[1] > b.x && b.y > lo[1] && hi[2] > d.x && d.y > lo[2]) return false;
             } else {
-                if(gx-- > 0) c += 1;
-                else if(gx = row, gy-- > 0) c += g.dim - row;
-                else if(gy = plane, gz-- > 0) c += g.dim * g.dim - g.dim * plane - row;
+                if(gy-- > 0) c += g.dim;
+                else if(gy = plane, gz-- > 0) c += g.dim * g.dim - g.dim * plane;
                 else break;
-                r = s_cell[c], k = r & 0xFFFFu, e = r >> 16;
+                k = s_cell[c] & 0xFFFFu, e = s_cell[c + row] >> 16;
             }
         }
         return true;
     };
-    // a warp takes 32 consecutive boxes at a time, so that its lanes' corners share cache lines; 64 bits,
-    // since the last stride may pass 2^32
-    for(size_t i = (size_t)blockIdx.x * kCollideBS + threadIdx.x; i < n; i += (size_t)gridDim.x * kCollideBS) {
-        const float lo[3] = {__ldcs(bbmin + 3 * i), __ldcs(bbmin + 3 * i + 1), __ldcs(bbmin + 3 * i + 2)};
-        const float hi[3] = {__ldcs(bbmax + 3 * i), __ldcs(bbmax + 3 * i + 1), __ldcs(bbmax + 3 * i + 2)};
+    // a warp takes 32 consecutive boxes at a time, so that its lanes' corners share cache lines; the last stride
+    // would pass 2^32 where n is near it
+    const uint32_t stride = gridDim.x * kCollideBS;
+    for(uint32_t i = blockIdx.x * kCollideBS + threadIdx.x; i < n; i += stride) {
+        const float lo[3] = {__ldcs(bbmin + 3 * (size_t)i), __ldcs(bbmin + 3 * (size_t)i + 1), __ldcs(bbmin + 3 * (size_t)i + 2)};
+        const float hi[3] = {__ldcs(bbmax + 3 * (size_t)i), __ldcs(bbmax + 3 * (size_t)i + 1), __ldcs(bbmax + 3 * (size_t)i + 2)};
         free_out[i] = query(lo, hi) ? 1 : 0;
+        if(n - i <= stride) break;
     }
 }
 
