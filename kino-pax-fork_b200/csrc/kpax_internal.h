@@ -12,11 +12,13 @@
 #include "kpax_device.cuh"
 #include "kpax_params.h"
 
-// Error helpers: record the failing call's text and return a status, never exit.
+// Error helpers: record the failing call's text and return a status, never exit.  The runtime's own record
+// of the error is cleared, or the next launch check would report it once more.
 #define KPAX_CUDA(call)                                                                             \
     do {                                                                                            \
         cudaError_t e_ = (call);                                                                    \
         if(e_ != cudaSuccess) {                                                                     \
+            cudaGetLastError();                                                                     \
             kpax::set_error("%s:%d %s: %s", __FILE__, __LINE__, #call, cudaGetErrorString(e_));     \
             return e_ == cudaErrorMemoryAllocation ? KPAX_ENOMEM : KPAX_ECUDA;                      \
         }                                                                                           \

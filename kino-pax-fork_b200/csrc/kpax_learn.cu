@@ -614,6 +614,7 @@ kpax_status kpax_mlp_create(uint32_t max_batch, kpax_mlp** out)
     n->max_batch = max_batch;
     const size_t P = kNumParams, B = max_batch;
     auto fail = [&](kpax_status st) {
+        cudaGetLastError();  // reported here, not by the next launch check
         kpax_mlp_destroy(n);
         return st;
     };

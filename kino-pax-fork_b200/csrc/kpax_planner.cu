@@ -622,11 +622,11 @@ struct PlanBatch {
         if(graph && key == graph_key) return KPAX_OK;
         if(graph) cudaGraphExecDestroy(graph), graph = nullptr;
         cudaGraph_t g = nullptr;
-        cudaGetLastError();  // an older call's error is not this capture's
         KPAX_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
         for(int i = 0; i < unroll; ++i) launch_iteration();
         const cudaError_t launched = cudaGetLastError();
         cudaError_t e = cudaStreamEndCapture(stream, &g);
+        if(e != cudaSuccess) cudaGetLastError();
         if(launched != cudaSuccess) {  // a refused launch ends the capture too: report the launch's reason
             if(g) cudaGraphDestroy(g);
             return set_error("launch of an iteration kernel failed: %s", cudaGetErrorString(launched)), KPAX_ECUDA;

@@ -241,6 +241,7 @@ kpax_status kpax_rekino_create(const kpax_config* cfg, const kpax_rekino_params*
     r->rp = *rp;
     kpax_status st = derive_params(*cfg, &r->p);
     auto fail = [&](kpax_status s) {
+        cudaGetLastError();  // reported here, not by the next launch check
         rekino_release(r);
         delete r;
         return s;
