@@ -292,6 +292,11 @@ kpax_status kpax_frontier_compact(const kpax_config* cfg, uint8_t* d_repeat, uin
  * (1 .. 2^22); it gives up, the kernel stores a timeout status and returns, and the call returns
  * KPAX_ETIMEOUT with *h_status = 1.  The context stays usable. */
 kpax_status kpax_test_wait_timeout(uint32_t spin_limit, uint32_t* h_status, void* stream);
+/* Test hook: CTA 0's part of a gather of the fused iteration over two CTAs of 64 threads, whose other
+ * CTA's word carries peer_tag and the value 7 (0: no word was written).  It waits until that word carries
+ * `tag`; after spin_limit polls every thread gives up and the call returns KPAX_ETIMEOUT.
+ * h_out[3]: threads that gave up, the sum of both CTAs' values (CTA 0's is 5), the sum below CTA 0. */
+kpax_status kpax_test_gather_timeout(uint32_t spin_limit, uint32_t tag, uint32_t peer_tag, uint32_t* h_out, void* stream);
 /* Test hook: for each x, writes (sin, cos) of the propagation kernels' sine/cosine and
  * (sin, cos) of CUDA's sincosf, 4 floats per input, so tests can bound their difference. */
 kpax_status kpax_test_sincos(const float* d_x, uint32_t n, float* d_out, void* stream);

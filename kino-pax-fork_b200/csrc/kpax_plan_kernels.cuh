@@ -573,7 +573,8 @@ struct GatherSmem {
 // visible afterwards.  Returns the same answer in every thread: false when a wait gave up.
 template <int NW>
 __device__ __forceinline__ bool gather_sum(unsigned long long* words, uint32_t tag, uint32_t G, uint32_t cb, uint32_t value,
-                                           bool release, GatherSmem<NW>& gs, uint32_t& below, uint32_t& total)
+                                           bool release, GatherSmem<NW>& gs, uint32_t& below, uint32_t& total,
+                                           uint32_t spin_limit = kSpinLimit)
 {
     const uint32_t tid = threadIdx.x;
     if(tid < kReplicas) gather_publish(words, G, cb, tag, value, false, release);
@@ -583,7 +584,7 @@ __device__ __forceinline__ bool gather_sum(unsigned long long* words, uint32_t t
     for(uint32_t j = tid; j < G && ok; j += 32 * NW) {
         uint32_t v = 0;
         bool f = false;
-        ok = gather_poll(words + j, tag, v, f);
+        ok = gather_poll(words + j, tag, v, f, spin_limit);
         t += v;
         b += j < cb ? v : 0u;
     }

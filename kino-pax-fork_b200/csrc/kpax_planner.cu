@@ -1342,6 +1342,16 @@ __global__ void k_test_lookback_timeout(unsigned long long* lb, uint32_t spin_li
     const bool ok = lb_exclusive(lb, 1u, 1u, excl, spin_limit);
     if(threadIdx.x == 0) *status = ok ? 0u : kErrTimeout;
 }
+
+// CTA 0's part of a gather over two CTAs, the other's word being what the host put there.
+// out: threads that saw the wait give up, the sum of the values, the sum of those below CTA 0.
+__global__ void __launch_bounds__(64) k_test_gather(unsigned long long* words, uint32_t tag, uint32_t spin_limit, uint32_t* out)
+{
+    __shared__ GatherSmem<2> gs;
+    uint32_t below = 0, total = 0;
+    if(!gather_sum<2>(words, tag, 2u, 0u, 5u, true, gs, below, total, spin_limit)) atomicAdd(out, 1u);
+    if(threadIdx.x == 0) out[1] = total, out[2] = below;
+}
 }  // namespace
 
 extern "C" {
@@ -1368,6 +1378,34 @@ kpax_status kpax_test_wait_timeout(uint32_t spin_limit, uint32_t* h_status, void
         KPAX_CUDA(cudaStreamSynchronize(s));
         if(*h_status & kErrTimeout)
             return set_error("kpax_test_wait_timeout: the look-back wait gave up after %u polls", spin_limit), KPAX_ETIMEOUT;
+        return KPAX_OK;
+    });
+}
+
+kpax_status kpax_test_gather_timeout(uint32_t spin_limit, uint32_t tag, uint32_t peer_tag, uint32_t* h_out, void* stream)
+{
+    return no_throw("kpax_test_gather_timeout", [&]() -> kpax_status {
+        if(!h_out || tag == 0 || spin_limit == 0 || spin_limit > kSpinLimit)
+            return set_error("kpax_test_gather_timeout: need an output, a tag and 1 <= spin_limit <= %u", kSpinLimit), KPAX_EINVAL;
+        constexpr size_t kWords = gather_words(2);
+        unsigned long long* mem = nullptr;
+        KPAX_CUDA(cudaMalloc(&mem, sizeof(unsigned long long) * (kWords + 2)));
+        struct Free {
+            void* m;
+            ~Free() { cudaFree(m); }
+        } free_mem{mem};
+        cudaStream_t s = (cudaStream_t)stream;
+        const unsigned long long peer = ((unsigned long long)(peer_tag & kTagMask) << 32) | 7u;
+        KPAX_CUDA(cudaMemsetAsync(mem, 0, sizeof(unsigned long long) * (kWords + 2), s));
+        if(peer_tag) KPAX_CUDA(cudaMemcpyAsync(mem + 1, &peer, sizeof(peer), cudaMemcpyHostToDevice, s));
+        uint32_t* d_out = reinterpret_cast<uint32_t*>(mem + kWords);
+        k_test_gather<<<1, 64, 0, s>>>(mem, tag, spin_limit, d_out);
+        KPAX_CHECK_LAUNCH();
+        count_launch(1);
+        KPAX_CUDA(cudaMemcpyAsync(h_out, d_out, 3 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+        KPAX_CUDA(cudaStreamSynchronize(s));
+        if(h_out[0])
+            return set_error("kpax_test_gather_timeout: the gather gave up after %u polls", spin_limit), KPAX_ETIMEOUT;
         return KPAX_OK;
     });
 }
