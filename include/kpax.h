@@ -235,8 +235,8 @@ kpax_status kpax_env_stats(kpax_env* env, uint32_t* n_cells, uint32_t* n_entries
  * 2^24 segments, two phases each, whose survivor list uses scratch held by `env` (about
  * 4 x (1 + control_dim + state_dim) bytes per segment of a round, plus 4 per segment for drawn
  * durations; kept for later calls and freed by kpax_env_destroy), so calls that share an env must be
- * issued in order on one stream.  Where five steps at the speed bound go further than a grid cell, it is
- * three phases, with twice the scratch, from 2^18 segments on (quadrotor: of any length). */
+ * issued in order on one stream.  Where five steps at the speed bound go further than about a grid cell, it
+ * is three phases, with twice the scratch, from 2^18 segments on (quadrotor: of any length). */
 kpax_status kpax_propagate_batch(const kpax_config* cfg, kpax_env* env, const float* d_parents,
                                  const float* d_draws, uint32_t draw_stream, uint32_t n,
                                  float* d_rows, uint8_t* d_valid, int32_t* d_steps, void* stream);

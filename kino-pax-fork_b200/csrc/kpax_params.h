@@ -51,15 +51,18 @@ constexpr int kGroup = 5;
 
 // Whether steps share collision queries in groups (run_steps).  A group's hull is walked over all its cells,
 // and the steps behind a colliding one are wasted, so groups pay while they stay about as small as a grid
-// cell: when kGroup steps at the speed bound go at most one cell far.  Longer steps get a query each.
-// B200, groups / query per step: the presets (0.5 to 3 m in 5 m cells) gain, see run_steps; quad-ref (15 m),
-// 100 iterations of 2^16 children 8.3 / 6.2 ms, with steps three times as long 7.5 / 2.3 ms; Dubins
-// segments of 10 m a group among 2000 obstacles, 2^19 139 / 106 us, of 4 m 122 / 119; 30011 quadrotor
-// segments of 6 m 43 / 57 us, of 60 m 304 / 68.
+// cell: when kGroup steps at the speed bound go at most a cell far, or 5/4 of one where speeds spread around
+// zero (the Dubins airplane flies near its bound).  Longer steps get a query each.
+// B200, groups / query per step: the presets (0.5 to 3 m in 5 m cells) gain, see run_steps; the quadrotor's
+// 3 m in 2.5 m cells, 300 iterations of 2^16 children, 22.3 / 23.4 ms; quad-ref (15 m in 5 m cells), 100
+// iterations 8.3 / 6.2 ms, with steps three times as long 7.5 / 2.3 ms.  Segments, 5 m cells, 2000 obstacles:
+// 30011 of the quadrotor, 6 m a group 58 / 70 us, 60 m 243 / 31; 2^19 of Dubins, 5 m 120 / 116, 6 m 145 / 119,
+// 10 m 139 / 106; 2^19 of the double integrator, 6 m 91 / 86 (30011: 27 / 29), 12.5 m 156 / 92.
 inline bool grouped(const KParams& p)
 {
     const float v = p.vmax > -p.vmin ? p.vmax : -p.vmin;
-    return (float)kGroup * p.h * v <= p.cell;
+    const float reach = p.model == KPAX_MODEL_DUBINS_AIRPLANE ? 1.0f : 1.25f;
+    return (float)kGroup * p.h * v <= reach * p.cell;
 }
 
 // Derive parameters; returns KPAX_OK or KPAX_EINVAL with a message in kpax_last_error().

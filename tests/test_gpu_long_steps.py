@@ -20,7 +20,7 @@ def _config(model):
     if model == 2:
         cfg.step_size = 0.25
     out = []
-    for cell in (5.0, 2.4):
+    for cell in (5.0, 1.9):
         c = cfg.copy()
         c.hash_cell_size = cell
         out.append(c)

@@ -9,7 +9,7 @@ import kpax_envs as E
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("preset,n,cell", [(kpax.PRESET_QUAD, (1 << 18) + 3, 5.0), (kpax.PRESET_QUAD, (1 << 18) + 3, 2.5),
+@pytest.mark.parametrize("preset,n,cell", [(kpax.PRESET_QUAD, (1 << 18) + 3, 5.0), (kpax.PRESET_QUAD, (1 << 18) + 3, 2.1),
                                            (kpax.PRESET_QUAD_REF, (1 << 18) + 1, 5.0), (kpax.PRESET_DUBINS, (1 << 19) + 5, 5.0)])
 def test_phased_batches(cuda, preset, n, cell):
     import torch
