@@ -92,7 +92,10 @@ typedef struct kpax_config {
     uint64_t seed;                  /* Philox4x32-10 key (the reference seeds cuRAND from the clock) */
     int32_t block_size;             /* threads per CTA of the expansion kernel: 0 (= 448), 128, 256, 448, 512 */
     int32_t unroll_iters;           /* planner iterations between two looks at the done flag: of a captured
-                                       CUDA graph, or of one fused launch (0 = default) */
+                                       CUDA graph (0 = 8), or of one fused launch (0 = 64).  A fused launch
+                                       holds every SM until it ends (4.8 ms for 64 iterations of the
+                                       quadrotor preset), and kernels of other streams wait that long:
+                                       1 lets them in after each iteration, for ~20 us more per iteration */
     int32_t samples_per_thread;     /* children per expansion thread, 0 (= 1) .. 8 (grid-stride rounds) */
     /* PruneKPAX goal-progress pruning (PruneKPAX.cu:466-498): an accepted child is kept with
      * probability clamp(exploration_bias + goal_bias * clamp(progress / progress_scale + 1/2, 0, 1),
@@ -101,9 +104,9 @@ typedef struct kpax_config {
     float prune_goal_bias;          /* h_goalBias_ (0.7, PruneKPAX.cu:36) */
     float prune_exploration_bias;   /* h_explorationBias_ (0.3, PruneKPAX.cu:35) */
     float prune_progress_scale;     /* h_progressScale_ (10, PruneKPAX.cu:34) */
-    /* 0: a single plan runs each iteration as one persistent launch (frontier passes, expansion
-     * and scores separated by bounded grid-wide barriers), or with the learned proposal as two such
-     * launches around the tensor-core pass; 1: one launch per stage.  Batches always run their own
+    /* 0: a single plan runs up to unroll_iters iterations as one persistent launch (frontier passes,
+     * expansion and scores joined by bounded gathers over its CTAs), or with the learned proposal each
+     * iteration as two such launches around the tensor-core pass; 1: one launch per stage.  Batches always run their own
      * persistent stages.  Plans are identical either way. */
     int32_t iteration_kernels;
     int32_t reserved[2];
@@ -292,11 +295,6 @@ kpax_status kpax_frontier_compact(const kpax_config* cfg, uint8_t* d_repeat, uin
  * (1 .. 2^22); it gives up, the kernel stores a timeout status and returns, and the call returns
  * KPAX_ETIMEOUT with *h_status = 1.  The context stays usable. */
 kpax_status kpax_test_wait_timeout(uint32_t spin_limit, uint32_t* h_status, void* stream);
-/* Test hook: CTA 0's part of a gather of the fused iteration over two CTAs of 64 threads, whose other
- * CTA's word carries peer_tag and the value 7 (0: no word was written).  It waits until that word carries
- * `tag`; after spin_limit polls every thread gives up and the call returns KPAX_ETIMEOUT.
- * h_out[3]: threads that gave up, the sum of both CTAs' values (CTA 0's is 5), the sum below CTA 0. */
-kpax_status kpax_test_gather_timeout(uint32_t spin_limit, uint32_t tag, uint32_t peer_tag, uint32_t* h_out, void* stream);
 /* Test hook: for each x, writes (sin, cos) of the propagation kernels' sine/cosine and
  * (sin, cos) of CUDA's sincosf, 4 floats per input, so tests can bound their difference. */
 kpax_status kpax_test_sincos(const float* d_x, uint32_t n, float* d_out, void* stream);

@@ -119,7 +119,7 @@ struct PlanBatch {
     // query, model groups on concurrent streams.  KPAX_BATCH_EXPAND=0|2 selects the alternatives
     // for measurements; the plans are the same.
     int expand_mode = 1;
-    bool fused = false;      // single query without the proposal: one k_iterate launch per iteration
+    bool fused = false;      // single query without the proposal: up to `unroll` iterations per k_iterate launch
     bool fused_split = false;  // single quadrotor query with the proposal: front, proposal pass, back
     uint32_t gx_split = 0;     // CTAs of the front and back launches (all resident), 0 if unusable
     uint32_t gx_iter = 0;    // its CTAs (all resident), 0 when the kernel cannot be used
@@ -1382,6 +1382,10 @@ kpax_status kpax_test_wait_timeout(uint32_t spin_limit, uint32_t* h_status, void
     });
 }
 
+// Test hook, not part of the ABI's header: CTA 0's part of a gather of the fused iteration over two CTAs of 64
+// threads, whose other CTA's word carries peer_tag and the value 7 (0: no word was written).  After spin_limit
+// polls without `tag` every thread gives up and the call returns KPAX_ETIMEOUT.  h_out[3]: threads that gave
+// up, the sum of both CTAs' values (CTA 0's is 5), the sum below CTA 0.
 kpax_status kpax_test_gather_timeout(uint32_t spin_limit, uint32_t tag, uint32_t peer_tag, uint32_t* h_out, void* stream)
 {
     return no_throw("kpax_test_gather_timeout", [&]() -> kpax_status {

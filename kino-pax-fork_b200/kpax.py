@@ -153,7 +153,6 @@ _SIGNATURES = {
     "kpax_region_batch": (_I32, [ctypes.POINTER(Config), _VP, _U32, _VP, _VP, _VP]),
     "kpax_frontier_compact": (_I32, [ctypes.POINTER(Config), _VP, _U32, _U32, _VP, ctypes.POINTER(FrontierStats), _VP]),
     "kpax_test_wait_timeout": (_I32, [_U32, ctypes.POINTER(_U32), _VP]),
-    "kpax_test_gather_timeout": (_I32, [_U32, _U32, _U32, ctypes.POINTER(_U32), _VP]),
     "kpax_kernel_launches": (ctypes.c_uint64, []),
     "kpax_batch_create": (_I32, [_VP, _U32, ctypes.POINTER(_VP)]),
     "kpax_batch_destroy": (_I32, [_VP]),
@@ -310,16 +309,6 @@ def test_wait_timeout(spin_limit: int, stream: int = 0) -> None:
     raises KpaxError with status ETIMEOUT once the wait gives up."""
     st = ctypes.c_uint32(0)
     check(load().kpax_test_wait_timeout(spin_limit, ctypes.byref(st), stream), "kpax_test_wait_timeout")
-
-
-def test_gather_timeout(spin_limit: int, tag: int, peer_tag: int, stream: int = 0) -> tuple[int, list[int]]:
-    """One CTA's gather over two CTAs, the other's word tagged peer_tag (kpax_test_gather_timeout): the call's
-    status and (threads that gave up, sum of the values, sum below)."""
-    out = (ctypes.c_uint32 * 3)()
-    status = load().kpax_test_gather_timeout(spin_limit, tag, peer_tag, out, stream)
-    if status not in (OK, ETIMEOUT):
-        check(status, "kpax_test_gather_timeout")
-    return status, list(out)
 
 
 def fp32_peak(iters: int = 1 << 16, stream: int = 0) -> tuple[float, float]:

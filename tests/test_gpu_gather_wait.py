@@ -10,26 +10,38 @@ import kpax
 import kpax_envs as E
 
 
-def test_arguments_are_checked_without_a_gpu():
-    lib = kpax.load()
+def _hook():
+    fn = kpax.load().kpax_test_gather_timeout
+    u32 = ctypes.c_uint32
+    fn.restype, fn.argtypes = ctypes.c_int32, [u32, u32, u32, ctypes.POINTER(u32), ctypes.c_void_p]
+    return fn
+
+
+def _gather(spin_limit, tag, peer):
+    """Status and (threads that gave up, sum of the values, sum below) of one CTA's gather over two."""
     out = (ctypes.c_uint32 * 3)()
-    assert lib.kpax_test_gather_timeout(0, 1, 0, out, None) == kpax.EINVAL
-    assert lib.kpax_test_gather_timeout(16, 0, 0, out, None) == kpax.EINVAL
-    assert lib.kpax_test_gather_timeout((1 << 22) + 1, 1, 0, out, None) == kpax.EINVAL
-    assert lib.kpax_test_gather_timeout(16, 1, 0, None, None) == kpax.EINVAL
+    return _hook()(spin_limit, tag, peer, out, None), list(out)
+
+
+def test_arguments_are_checked_without_a_gpu():
+    fn, out = _hook(), (ctypes.c_uint32 * 3)()
+    assert fn(0, 1, 0, out, None) == kpax.EINVAL
+    assert fn(16, 0, 0, out, None) == kpax.EINVAL
+    assert fn((1 << 22) + 1, 1, 0, out, None) == kpax.EINVAL
+    assert fn(16, 1, 0, None, None) == kpax.EINVAL
 
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("tag,peer", [(1, 0), (7, 6), (7, 8), ((1 << 30) - 1, (1 << 30) - 2), (1 << 30, (1 << 30) - 1)])
 def test_a_missing_or_stale_word_ends_the_wait(cuda, tag, peer):
-    status, (gave_up, _, _) = kpax.test_gather_timeout(1 << 10, tag, peer)
+    status, (gave_up, _, _) = _gather(1 << 10, tag, peer)
     assert status == kpax.ETIMEOUT and gave_up == 64
 
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("tag", [1, 7, (1 << 30) - 1, (1 << 30) + 5])
 def test_the_tagged_word_is_summed(cuda, tag):
-    assert kpax.test_gather_timeout(1 << 10, tag, tag) == (kpax.OK, [0, 12, 0])
+    assert _gather(1 << 10, tag, tag) == (kpax.OK, [0, 12, 0])
 
 
 @pytest.mark.gpu
@@ -46,5 +58,5 @@ def test_plans_run_after_a_wait_that_ended(cuda):
         r = pl.plan(s, g, d.data_ptr(), len(obs))
         out.append((r.tree_size, r.valid_expansions))
         pl.close()
-        assert kpax.test_gather_timeout(1 << 10, 3, 2)[0] == kpax.ETIMEOUT
+        assert _gather(1 << 10, 3, 2)[0] == kpax.ETIMEOUT
     assert out[0] == out[1]
