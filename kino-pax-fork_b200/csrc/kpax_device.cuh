@@ -203,12 +203,6 @@ __device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c)
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
     return r;
 }
-__device__ __forceinline__ F2 mul2(F2 a, F2 b)
-{
-    F2 r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
 
 // float -> int with the reference's device semantics (saturating, NaN -> 0).
 __device__ __forceinline__ int f2i(float x) { return __float2int_rz(x); }

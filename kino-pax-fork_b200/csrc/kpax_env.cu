@@ -286,7 +286,7 @@ __global__ void __launch_bounds__((kBatchBS<M, K>), kBatchBlocks) k_propagate_ba
     if(steps_out) steps_out[i] = done;
 }
 
-// Large batches run in two phases so that lanes do not idle behind their warp's longest segment: the
+// Large batches run in phases so that lanes do not idle behind their warp's longest segment: the
 // head runs every segment for its first kHeadSteps steps and finishes the segments that end there; the
 // others are appended, state and controls, to a compact list, which the tail carries to the end with
 // full warps.  Both run the same per-step code in the same order, so rows, verdicts and step counts

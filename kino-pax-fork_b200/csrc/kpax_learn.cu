@@ -34,11 +34,11 @@ namespace {
 //   k_mlp_dw    dW = dZ^T A of all layers, 64 x 64 tiles, the rows split over up to kSplits partial sums
 //   k_mlp_grad  partial sums added in split order (and Adam)
 // Products accumulate in pairs of FP32 values (fma.rn.f32x2), each output in a fixed order.
-// B200, loss and gradient of 4096 rows: 1766 us with one 64 x 64-tile SGEMM per product (8-16 CTAs
+// B200, loss and gradient of 4096 rows: 1770-1840 us with one 64 x 64-tile SGEMM per product (8-16 CTAs
 // summing all rows for a weight gradient, 645-695 us each) and one thread per column for the bias
 // gradients (230 us each); now 120 us: rows 75, weight gradients 34 (46 with 4 x 8 outputs per thread),
 // sums 5.5.  Both products are bound by shared memory's return bandwidth, 21-26 of 72.6 TFLOP/s.
-// Error of the gradient against 64 bits: 2.5e-6 before, 2.2e-6 now.
+// Error of the gradient against 64 bits, by seed: 2.3-2.9e-6 before, 2.1-2.7e-6 now.
 
 constexpr int kRowThreads = 256;
 constexpr int kChunkK = 32, kWStride = kChunkK + 4;  // weights chunk: [columns][32], rows 36 floats apart (conflict-free)
