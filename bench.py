@@ -51,14 +51,15 @@ FLOP_PER_STEP = {kpax.MODEL_DOUBLE_INTEGRATOR: 18, kpax.MODEL_DUBINS_AIRPLANE: 5
 # dram__bytes_read.sum + dram__bytes_write.sum of one steady-state k_iterate launch (the fused
 # iteration, 2^16 children, L2 flushed before it) in an ncu capture of the default workload; none
 # for the others
-ITERATE_DRAM_BYTES = {kpax.MODEL_QUADROTOR: 2093824 + 0}
+ITERATE_DRAM_BYTES = {kpax.MODEL_QUADROTOR: 2509312 + 768}
 # the same sum for the one-pass kernel (kpax_propagate_batch_noalloc) on 2^20 Dubins segments, L2
 # flushed before the step, per segment
-ONE_PASS_DRAM_BYTES_PER_SEGMENT = (25186304 + 48397824) / (1 << 20)
-# the same sum over the three phase kernels of one 2^20-segment Dubins batch (L2 flushed before the
+ONE_PASS_DRAM_BYTES_PER_SEGMENT = (25239808 + 45287424) / (1 << 20)
+# the same sum over the two phase kernels of one 2^20-segment Dubins batch (L2 flushed before the
 # step, no cache flush between the kernels), per segment: scaled by the segment count, as the
 # traffic grows with it
-PHASED_DRAM_BYTES_PER_SEGMENT = (30508800 + 103499264) / (1 << 20)
+PHASED_DRAM_BYTES_PER_SEGMENT = (34460160 + 60135680 + 2912512 + 25795584) / (1 << 20)
+PHASED_MIN_SEGMENTS = 1 << 19  # kPhasedMin of the Dubins kernels (kpax_env.cu)
 WORKLOADS = {
     "quad": (kpax.PRESET_QUAD, E.quad_scene, "12D quadrotor, building scene (1000 AABBs incl. windowed wall), "
              "2^16 expansions/iteration, 25 RK4 steps of 0.02 s"),
@@ -933,20 +934,20 @@ def run_segments(args) -> None:
 
     peaks = load_peaks()
     sm_mhz = peaks.get("sm_max_mhz", 1965.0)
-    phased = n >= 1 << 18 and not args.one_pass
+    phased = n >= PHASED_MIN_SEGMENTS and not args.one_pass
     achieved = n_steps * FLOP_PER_STEP[cfg.model] / t_s / 1e12
     roofline = {"bound": "fp32", "achieved": achieved, "peak": fp32_peak, "unit": "TFLOP/s", "frac": achieved / fp32_peak,
                 "traffic": int(PHASED_DRAM_BYTES_PER_SEGMENT * n) if phased
                            else int(ONE_PASS_DRAM_BYTES_PER_SEGMENT * n) if args.one_pass else None,
-                "traffic_note": ("DRAM bytes read + written per step by the three phase kernels, from an ncu capture of "
+                "traffic_note": ("DRAM bytes read + written per step by the two phase kernels, from an ncu capture of "
                                  "2^20 segments scaled to the segment count (summary under profiles/); "
                                  "the algorithmic bytes are 69 per segment (parent 24, row 40, verdict 1, steps 4), the "
                                  "rest is the survivors' round trips and partial-sector fills of rows written out of order")
                                 if phased else
                                 ("DRAM bytes read + written per step by the one-pass kernel, from an ncu capture of 2^20 "
-                                 "segments scaled to the segment count (summary under profiles/): 70.2 B per segment "
-                                 "against 69 algorithmic"),
-                "kernel": "k_propagate_head + 2 x k_propagate_tail<Dubins> (phased batch)" if phased
+                                 "segments scaled to the segment count (summary under profiles/): 67.3 B per segment "
+                                 "against 69 algorithmic (the last rows are still dirty in L2 when it ends)"),
+                "kernel": "k_propagate_head + k_propagate_tail<Dubins> (phased batch)" if phased
                           else "k_propagate_batch<Dubins>",
                 "peak_note": "measured: kpax_fp32_peak (FMA chains, CUDA events) on this GPU inside the clock-sampling "
                              "window; MEASURED_PEAKS.json has no FP32 figure; plus 12 transcendental per step on the MUFU "
